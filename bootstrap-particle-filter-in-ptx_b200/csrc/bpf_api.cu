@@ -104,6 +104,7 @@ struct Impl {
   // fused launch (gpu_bpf_set_fused_small)
   bool fused_small = true;
   int small_tiles = 4;                  // largest fused cluster on the filter's device (tiles)
+  int res_tiles = 0;                    // largest filter of a resident run on it (tiles)
 
   // profiling
   bool profiling = false;
@@ -133,6 +134,19 @@ int ensure_device(Impl* m) {
 // profiling); the two give bit-identical results.
 bool use_small(const Impl* m, const TickArgs& a) {
   return m->fused_small && !m->profiling && m->plan.G <= m->small_tiles && small_eligible(m->plan, a);
+}
+
+// A run of consecutive ticks of a larger filter stays on the chip as one resident launch (same
+// conditions, same results).
+bool use_resident(const Impl* m, const TickArgs& a) {
+  return m->fused_small && !m->profiling && !use_small(m, a) && m->plan.G <= m->res_tiles && !a.learn && a.apf == 0 &&
+         !(a.silverman > 0.0f);
+}
+// Whether a run of ticks is one launch, and that launch (a.y_ptr, a.rec: the run's first tick).
+bool one_launch(const Impl* m, const TickArgs& a) { return use_small(m, a) || use_resident(m, a); }
+cudaError_t launch_run(Impl* m, const TickArgs& a, int n_ticks) {
+  if (use_small(m, a)) return launch_small(m->plan, a, n_ticks, m->stream, m->pdl);
+  return launch_resident(m->plan, a, ResidentTape{}, false, n_ticks, m->res_tiles, m->stream);
 }
 
 // Filters of at most kTailTiles tiles run the plan in pass 1's last CTA instead of a plan
@@ -337,8 +351,8 @@ int build_graph(GpuBpfState* s, Impl* m) {
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaMemcpyAsync(m->y_dev, m->y_pin, kGraphChunk * sizeof(float), cudaMemcpyHostToDevice, m->stream);
   const TickArgs a0 = make_args(s, m, 0.0f, m->y_dev, m->rec_dev + 1);
-  if (err == cudaSuccess && use_small(m, a0)) {
-    err = launch_small(m->plan, a0, kGraphChunk, m->stream, m->pdl);     // the chunk as one launch
+  if (err == cudaSuccess && one_launch(m, a0)) {
+    err = launch_run(m, a0, kGraphChunk);                                // the chunk as one launch
   } else {
     for (int k = 0; k < kGraphChunk && err == cudaSuccess; ++k) {
       TickArgs a = make_args(s, m, 0.0f, m->y_dev + k, m->rec_dev + 1 + k);
@@ -366,8 +380,8 @@ int build_device_graph(GpuBpfState* s, Impl* m, const float* y_dev, int n, BpfTi
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
   const TickArgs a0 = make_args(s, m, 0.0f, y_dev, rec_dev);
-  if (use_small(m, a0)) {
-    err = launch_small(m->plan, a0, n, m->stream, m->pdl);              // the whole run as one launch
+  if (one_launch(m, a0)) {
+    err = launch_run(m, a0, n);                                         // the whole run as one launch
   } else {
     for (int k = 0; k < n && err == cudaSuccess; ++k) {
       TickArgs a = make_args(s, m, 0.0f, y_dev + k, rec_dev + k);
@@ -489,6 +503,7 @@ static int create_impl(GpuBpfState* s, Impl* m, int n, float rho, float sigma_z,
   CK(cudaMemsetAsync(m->rec_dev, 0, (1 + kGraphChunk) * sizeof(BpfTickRecord), m->stream));
   m->pass2_grid = pass2_grid_size(m->device);
   m->small_tiles = small_max_tiles(m->device);
+  m->res_tiles = resident_max_tiles(m->device);
   if (const char* v = std::getenv("BPF_DISABLE_PDL")) m->pdl = (v[0] == '0');
 
   // observation model (gpu_bpf_ptx_full.cu:406-412)
@@ -716,7 +731,7 @@ int gpu_bpf_step_many(GpuBpfState* s, const float* y, int n_ticks, BpfResult* ou
       std::memcpy(m->y_pin, y + t, kGraphChunk * sizeof(float));
       CK(cudaGraphLaunch(m->graph, m->stream));
       CK(cudaStreamSynchronize(m->stream));
-      g_launches += use_small(m, make_args(s, m, 0.0f, nullptr, nullptr))
+      g_launches += one_launch(m, make_args(s, m, 0.0f, nullptr, nullptr))
                         ? 1 : (long long)tick_launches(m, make_args(s, m, 0.0f, nullptr, nullptr)) * kGraphChunk;
       m->ticks_enqueued += kGraphChunk;
       for (int k = 0; k < kGraphChunk; ++k) {
@@ -773,7 +788,7 @@ int gpu_bpf_step_many_device(GpuBpfState* s, const float* y_dev, int n_ticks, Bp
                        m->dg_silv != s->silverman_shrink || m->dg_anc != m->record_anc;
     if (stale) { rc = build_device_graph(s, m, y_dev, n_ticks, rec_dev); if (rc) return rc; }
     CK(cudaGraphLaunch(m->dgraph, m->stream));
-    g_launches += use_small(m, make_args(s, m, 0.0f, nullptr, nullptr))
+    g_launches += one_launch(m, make_args(s, m, 0.0f, nullptr, nullptr))
                       ? 1 : (long long)tick_launches(m, make_args(s, m, 0.0f, nullptr, nullptr)) * n_ticks;
     m->ticks_enqueued += n_ticks;
   } else {

@@ -35,6 +35,7 @@
 // ptx_assembly/bpf_kernels_full.ptx:231-842.
 #include "bpf_plain.cuh"
 #include "bpf_block.cuh"
+#include "bpf_tick.cuh"
 #include <cooperative_groups.h>
 #include <cmath>
 #include <mutex>
@@ -682,24 +683,6 @@ constexpr size_t kPass2Smem = kMarkOffset + kMarkBytes;         // one staged ti
 static_assert(kMarkOffset % 16 == 0 && kMarkBytes % 16 == 0, "marks are cleared with 16-byte stores");
 static_assert((size_t)kOutChunk % kGatherStep == 0, "the gather reads marks in steps of 256 slots");
 
-// Tile-frame thresholds of the child count are kept relative to the thread's first
-// element and capped here: a thread's 16 fixed-point weights sum to at most 16 * 2^50
-// < kThCap, so a capped threshold is never reached, and threshold + c * spacing stays
-// below 2^57 for every count c the loop forms.
-constexpr unsigned long long kThCap = 1ull << 55;
-
-// Exact count of targets up to element `upto` of a thread's 16 staged log2-weights d:
-// #{m >= 0 : R0 + m D <= sum_{i <= upto} floor(2^d_i 2^50)}, at most cap. The rare path of
-// the FP32 estimate in pass 2's child count.
-__device__ __noinline__ int exact_count(const float* d, int upto, unsigned long long R0, unsigned long long D,
-                                        int cap) {
-  unsigned long long l = 0ull;
-  for (int i = 0; i <= upto; ++i) l += fix_weight(tile_weight(d[i]));
-  if (l < R0) return 0;
-  const unsigned long long c = udiv_fp64(l - R0, D) + 1ull;
-  return c >= (unsigned long long)cap ? cap : (int)c;
-}
-
 __device__ __forceinline__ void pass2_fetch(const Plan& p, const float* hsrc, int it, unsigned char* buf,
                                             uint64_t* bar) {
   const int k = p.items[it].x;
@@ -1098,12 +1081,6 @@ constexpr int kChunks = kTile / 4;                      // four-slot chunks of a
 constexpr int kYStage = kSmallThreads;                  // observations staged per refill
 static_assert(kChunks == kSmallThreads, "one four-slot chunk per thread");
 
-// What the finish of a tick's plan needs from its decision (plan_fused_decide -> plan_fused_finish).
-struct FusedTail {
-  double tS, tH, ess, logS_prev_old;
-  int nM, degenerate, resample, resampled_prev_old, tick_old;
-};
-
 struct FusedPlan {
   unsigned long long base, delta, magic, total;
   int nM, Fg, items, zero_spacing;
@@ -1408,7 +1385,7 @@ __device__ __forceinline__ void plan_fused(const TickArgs& a, int N, FusedShared
 // The same plan in two parts, for ticks whose next tick should not wait for the record: the
 // decision (plan_fused_decide, warp 0) computes the statistics as plan_fused and writes the
 // device-state fields that the next tick's pass 1 and the resampling read: plan_decide's
-// operations on them, in its order; the finish (plan_fused_finish, lane 0 of warp 0, later in
+// operations on them, in its order; the finish (fused_finish, one thread, later in
 // the tick) computes the log-likelihood increment and the filtered mean and writes the record, the
 // running sums and, when the tick keeps its particles, the log of its weight sum, from the values
 // the decision left in sh.tail. The two parts together write what plan_decide writes, with the
@@ -1435,68 +1412,7 @@ __device__ __forceinline__ void plan_fused_decide(const TickArgs& a, int N, Fuse
     }
     tS = warp_sum_d(S); tQ = warp_sum_d(Q); tH = warp_sum_d(H);
   }
-  if (lane != 0) return;
-  DevState* st = &sh.st;
-  FusedTail& tl = sh.tail;
-  const bool degenerate = (nM == kNkEmpty) || !(tS > 0.0);
-  double ess = 0.0;
-  int resample = 0;
-  if (!degenerate) {
-    ess = tS * tS / tQ;
-    resample = (a.ess_threshold <= 0.0f) || (ess / (double)N < (double)a.ess_threshold);
-  }
-  tl.tS = tS; tl.tH = tH; tl.ess = ess; tl.nM = nM;
-  tl.degenerate = degenerate ? 1 : 0; tl.resample = resample;
-  tl.logS_prev_old = st->logS_prev; tl.resampled_prev_old = st->resampled_prev; tl.tick_old = st->tick;
-  const int cur = st->cur;
-  if (degenerate) st->error = BPF_ERR_DEGENERATE;
-  {
-    const int d1 = st->dirs & 1;
-    st->dirs = (resample ? d1 : (d1 ^ 1)) | ((d1 ^ 1) << 1);
-  }
-  st->k1 = st->k1 * kPcgMult;
-  st->k2 = st->k2 * kPcgMult + 1ull;
-  st->tick = tl.tick_old + 1;
-  st->do_resample = resample;
-  st->nM = nM;
-  if (resample) {
-    const uint64_t old = st->u_state;
-    st->u_state = old * kPcgMult + kHostInc;
-    st->u23 = pcg_output(old) >> 9;
-    st->logS_prev = a.log_n;
-    st->resampled_prev = 1;
-    st->resample_count += 1;
-    st->src = cur;
-    st->cur = cur ^ 1;
-  } else if (degenerate) {
-    st->logS_prev = a.log_n;
-    st->resampled_prev = 1;
-  } else {
-    st->resampled_prev = 0;
-    st->nM_prev = nM;
-  }
-}
-
-__device__ __forceinline__ void plan_fused_finish(const FusedShared& sh_in, DevState* st, BpfTickRecord* rec_out) {
-  const FusedTail& tl = sh_in.tail;
-  constexpr double kLn2d = 0.693147180559945309417232121458;
-  double dll = -INFINITY, hm = __longlong_as_double(0x7FF8000000000000LL), L = 0.0;
-  if (!tl.degenerate) {
-    L = log(tl.tS);
-    dll = __fma_rn((double)tl.nM, kLn2d, L) - tl.logS_prev_old;
-    hm = tl.tH / tl.tS;
-  }
-  const double ll_ref = (tl.resampled_prev_old ? 0.0 : st->ll_ref) + dll;
-  st->ll_ref = ll_ref;
-  st->hm = tl.degenerate ? 0.0 : hm;
-  st->ll_total += dll;
-  if (rec_out) {
-    BpfTickRecord r;
-    r.dloglik = dll; r.loglik_ref = ll_ref; r.loglik_total = st->ll_total;
-    r.h_mean = (float)hm; r.ess = (float)tl.ess; r.resampled = tl.resample; r.tick = tl.tick_old;
-    *rec_out = r;
-  }
-  if (!tl.resample && !tl.degenerate) st->logS_prev = L;
+  if (lane == 0) fused_decide(a, N, nM, tS, tQ, tH, &sh.st, sh.tail);
 }
 
 // The resampling plan into the device state (on a resampling tick).
@@ -1564,17 +1480,6 @@ __device__ __forceinline__ bool plan_fused_targets(int N, double rcpN, FusedShar
   return live;
 }
 
-// A chunk of CH consecutive slots of the tile (slots CH c .. CH c + CH - 1) against the tick's
-// targets: its weights, their FP32 sum in order, its first target and tile-frame thresholds
-// (th = kThCap: no target is reachable from the chunk).
-template <int CH>
-struct ChunkTargets {
-  float wf[CH];
-  float lfT;
-  unsigned long long th, D;
-  int q, c;
-};
-
 template <int NCTA, int CH>
 __device__ __forceinline__ ChunkTargets<CH> chunk_targets(int N, int k, int par, int c, const FusedShared& sh) {
   static_assert(CH % 4 == 0, "whole four-slot chunks");
@@ -1596,13 +1501,7 @@ __device__ __forceinline__ ChunkTargets<CH> chunk_targets(int N, int k, int par,
   for (int e = 0; e < CH; ++e) ct.lfT += ct.wf[e];
   const unsigned long long loc = sh.chunkP[l0 / 4];   // exclusive prefix of its first four-slot chunk
   // child counts against tile-frame thresholds, as pass 2
-  ct.q = targets_below(Pk + shr64(loc, r), base, delta, pl.magic, N);
-  ct.th = kThCap; ct.D = kThCap;
-  if (r < 64 && ct.q < N && j0 < N) {
-    const unsigned long long m = base + (unsigned long long)ct.q * delta - Pk + 1ull;
-    if (m <= (~0ull >> r)) ct.th = min((m << r) - loc, kThCap);
-    if (delta <= (kThCap >> r)) ct.D = delta << r;
-  }
+  chunk_thresholds<CH>(N, loc, Pk, r, j0 < N, base, delta, pl.magic, ct);
   return ct;
 }
 
@@ -1620,43 +1519,10 @@ template <int NCTA, int CH>
 __device__ __forceinline__ void count_write(const TickArgs& a, int N, int k, const ChunkTargets<CH>& ct, int src,
                                             int dst, FusedShared& sh) {
   const int j0 = k * kTile + CH * ct.c;
-  const float* d = sh.w + CH * ct.c;               // its log2-weights, for the exact recount
   const float* hs = sh.h[src] + CH * ct.c;         // its particles
-  const unsigned long long R0 = ct.th, D = ct.D;
-  const bool none = R0 >= kThCap;
-  const float R0w = (float)R0 * 0x1p-50f;
-  const float invDw = 1.0f / ((float)D * 0x1p-50f);
-  const float R0x = R0w * invDw;
-  const float eL = 0x1p-18f * invDw, e0 = fmaf(R0w, eL, 0x1p-44f * invDw);
-  const float xT = fmaf(ct.lfT, invDw, -R0x);
-  float err = fmaf(ct.lfT, eL, fmaf(fmaxf(fabsf(xT), R0x), 0x1p-21f, e0));
-  if (!(xT < 0x1p22f)) err = 1.0f;
-  const float err_hi = 1.0f - err;
-  const int q0 = ct.q, Kq = 0x4AFFFFFF - q0;
-  float lf = 0.0f;
+  const int q0 = ct.q;
   int qe[CH];                                      // q_j: the end of element j's children
-#pragma unroll
-  for (int g = 0; g < CH / 4; ++g) {
-    int qq[4];
-    bool rc[4], any = false;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      lf += ct.wf[4 * g + e];
-      const float x = fmaf(lf, invDw, -R0x);
-      const float fl = floorf(x);
-      const float fr = x - fl;                       // exact
-      rc[e] = !none && !(fr > err && fr < err_hi);
-      any |= rc[e];
-      qq[e] = none ? q0 : min(max(__float_as_int(fl + 0x1p23f) - Kq, q0), N);
-    }
-    if (__any_sync(0xffffffffu, any)) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (rc[e]) qq[e] = min(q0 + exact_count(d, 4 * g + e, R0, D, N), N);
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) qe[4 * g + e] = qq[e];
-  }
+  chunk_child_ends<CH>(N, ct, sh.w + CH * ct.c, qe);
   // The chunk's children fill the slots [q0, q_last): slot o belongs to element #{j : q_j <= o}.
   // Each lane writes its run in one loop, starting at an offset rotated by lane / 4: the runs of
   // a warp's lanes start about eight slots apart, so without the rotation eight lanes would store
@@ -1792,7 +1658,7 @@ small_kernel(Plan p, TickArgs a, int n_ticks) {
       }
       // the tick's record and running sums, on a warp outside pass 1, while the others start the
       // next tick
-      if (tid == kSmallThreads - 32) plan_fused_finish(sh, &sh.st, (a.rec && k == 0) ? a.rec + t : nullptr);
+      if (tid == kSmallThreads - 32) fused_finish(sh.tail, &sh.st, (a.rec && k == 0) ? a.rec + t : nullptr);
     }
   }
   if (tid == 0 && a.mirror) sh.st.seq = a.seq;
@@ -1880,9 +1746,11 @@ cudaError_t plan_alloc(Plan& p, int N) {
   al(&p.jticket, sizeof(unsigned));
   al(&p.pticket, sizeof(unsigned));
   al(&p.st, sizeof(DevState));
+  al(&p.xbuf, resident_xbuf_bytes(p.G));
   if (e == cudaSuccess) e = cudaMemset(p.nexp, 0, p.G * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(p.jticket, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(p.pticket, 0, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(p.xbuf, 0, resident_xbuf_bytes(p.G));
   if (e == cudaSuccess) e = cudaDeviceSynchronize();   // visible to every stream before first use
   return e;
 }
@@ -1891,7 +1759,7 @@ void plan_free(Plan& p) {
   bpf_free(p.h0); bpf_free(p.h1); bpf_free(p.w);
   bpf_free(p.nexp); bpf_free(p.E); bpf_free(p.rec); bpf_free(p.rec2);
   bpf_free(p.P); bpf_free(p.ofirst); bpf_free(p.items); bpf_free(p.st);
-  bpf_free(p.jpart); bpf_free(p.jticket); bpf_free(p.pticket);
+  bpf_free(p.jpart); bpf_free(p.jticket); bpf_free(p.pticket); bpf_free(p.xbuf);
   p = Plan{};
 }
 

@@ -64,6 +64,7 @@ struct Plan {
   unsigned* jticket;         // CTAs of the jitter-variance kernel done this tick (the last one resets it)
   unsigned* pticket;         // pass-1 CTAs done this tick when the last one runs the plan (it resets it)
   DevState* st;
+  unsigned char* xbuf;       // exchange buffer of resident runs (zeroed once), or null: none
 };
 
 // Host-mapped mirror of the state a synchronous tick reads back (zero-copy): written by the
@@ -126,6 +127,21 @@ cudaError_t launch_jitter(const Plan& p, const TickArgs& a, cudaStream_t s, bool
 // n_ticks is 1). Not for learning, auxiliary-filter, Silverman or taped ticks.
 bool small_eligible(const Plan& p, const TickArgs& a);
 cudaError_t launch_small(const Plan& p, const TickArgs& a, int n_ticks, cudaStream_t s, bool pdl);
+// Resident runs (bpf_resident.cu): n_ticks consecutive ticks of a filter of at most
+// resident_max_tiles(device) tiles in one cooperative launch, bit-identical to the tick-per-launch
+// path. a.y_ptr and a.rec point at the run's first tick; apf: auxiliary-filter ticks (threshold 0).
+// Not for learning, Silverman or mirrored ticks.
+struct ResidentTape {        // gradient tape of a taped run from tick 0 (all null otherwise)
+  int32_t* csr; size_t csr_stride;     // first child slots, tick t's at csr + t * csr_stride
+  float* ckpt; size_t ckpt_stride;     // particles entering every K-th tick
+  int K;
+  float2* aux;                         // {1/S, nM} per tick
+};
+constexpr int kResMaxTilesPerCta = 4;
+size_t resident_xbuf_bytes(int G);
+int resident_max_tiles(int device);    // 0: the device takes no resident runs
+cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
+                            int max_tiles, cudaStream_t s);
 int pass2_grid_size(int device);
 // Tiles the fused tick takes on this device (16, else 8; 4 before pass2_grid_size configured it).
 int small_max_tiles(int device);

@@ -1,0 +1,753 @@
+// bpf_resident.cu — a run of consecutive ticks of a medium filter in one launch, its particles
+// resident in shared memory across the GPU (one CTA per SM, up to kResMaxTilesPerCta tiles a CTA).
+//
+// The tick-per-launch path of such a filter (pass 1, the plan in its last CTA, pass 2) is bound by
+// latency, not by work: two dependent launches, a ticket and a one-CTA plan per tick. Here every CTA
+// keeps its tiles' particles, log2-weights and the next tick's noise in shared memory from the first
+// tick to the last, and the CTAs meet once per tick (twice when the tick resamples):
+//   pass 1    the tile arithmetic of pass 1 (kThreads * SPLIT threads a tile, the FP32 partial sums
+//             handed along in pass 1's element order), so every tile record is bit for bit pass 1's;
+//   exchange  each tile's record {S, Q, H, n_k, E} is published as two 16-byte words that carry the
+//             exchange's number, and thread k of every CTA polls tile k's record until the numbers
+//             match: barrier and data in one trip through L2. The next tick's noise is formed before
+//             the poll, while the records travel;
+//   plan      every CTA forms the plan's FP64 sums in the plan kernel's order (one tile a thread, warp
+//             butterfly, warps in sequence) and takes the same decision; one CTA (the keeper) also
+//             writes the record, whose FP64 log is left to the next tick's exchange;
+//   resample  the plan kernel's exact fixed-point rule: the u64 scan over the tile masses in every
+//             CTA, then each parent writes its particle to its children's slots: in its own tile's
+//             shared memory where they fall there (nearly all do: a tile's outputs drift from its
+//             slots by about sqrt(N)), else to the other particle buffer (L2), from which the owner
+//             takes them once the CTAs that write there have raised their flags.
+// What bounds it: latency, three grid-wide dependencies deep at most, and the issue of about 60
+// thread-instructions per particle (16 particles a thread keep the per-thread overhead small: with
+// 1024 threads of 4 the same tick issued 144 per particle). Measured per tick: N = 300000 at
+// ESS < 0.5 N 4.4 us (16.4 with a launch per kernel), always resampling 10.4 us (20.8); N = 1000003 at
+// ESS < 0.5 N 6.1 us (12.5).
+// Results equal the tick-per-launch path's bit for bit.
+//
+// The CTAs wait on one another, so the launch is cooperative (all resident or none start), and every
+// wait gives up after kResWaitNs: the run then ends with BPF_ERR_STATE.
+#include "bpf_tick.cuh"
+#include <mutex>
+#include <type_traits>
+
+namespace bpf {
+
+constexpr int kResThreads = 512;
+constexpr int kResWarps = kResThreads / 32;
+constexpr unsigned long long kResWaitNs = 2000000000ull;
+constexpr int kResMaxTiles = 1024;        // records an exchange holds at most (32 sums of 32 tiles)
+constexpr int kResHeavy = 16;             // children above which a parent's run is shared by its warp
+static_assert(kResMaxTilesPerCta == 4, "four tiles of two groups of threads");
+
+// ---------------------------------------------------------------------------
+// Exchange buffer (Plan::xbuf): word 0 the epoch (exchange numbers used so far, advanced by every
+// launch's keeper), word 1 the abort mark; then kMail mailboxes, each with a flag per CTA and two
+// parities of two 16-byte record words per tile. A record word is read and written as one 128-bit
+// access, so its number vouches for its data. Every record and flag is written to all mailboxes and
+// CTA b polls mailbox b % kMail: with one mailbox polled by all, the polls of a few hot lines held
+// up the records themselves.
+// ---------------------------------------------------------------------------
+constexpr int kMail = 16;
+constexpr size_t kXHeader = 256;
+__host__ __device__ inline size_t mail_flag_bytes(int G) { return ((size_t)G * 4 + 127) & ~(size_t)127; }
+__host__ __device__ inline size_t mail_bytes(int G) { return mail_flag_bytes(G) + (((size_t)G * 64 + 127) & ~(size_t)127); }
+size_t resident_xbuf_bytes(int G) { return kXHeader + kMail * mail_bytes(G); }
+
+__device__ __forceinline__ void st_relaxed_b128(void* p, unsigned long long lo, unsigned long long hi) {
+  asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p), "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ void ld_relaxed_b128(const void* p, unsigned long long& lo, unsigned long long& hi) {
+  asm volatile("{ .reg .b128 v; ld.relaxed.gpu.global.b128 v, [%2]; mov.b128 {%0, %1}, v; }"
+               : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Whether a warp's wait goes on (the same answer in every lane): every 256 polls it looks at the time
+// and at the abort mark of this launch.
+struct Patience {
+  unsigned long long t0 = 0ull;
+  unsigned spins = 0u;
+  __device__ __forceinline__ bool more(const unsigned* abort_word, unsigned mark) {
+    if ((++spins & 255u) != 0u) return true;
+    const unsigned long long t = global_timer_ns();
+    if (t0 == 0ull) t0 = t;
+    return __all_sync(0xffffffffu, t - t0 < kResWaitNs && ld_relaxed_u32(abort_word) != mark);
+  }
+};
+
+template <int NT>
+struct ResidentShared {
+  float h[NT][kTile];                     // particles
+  float w[NT][kTile];                     // tile-relative log2-weights
+  float z[NT][kTile];                     // state noise of the next propagation
+  float part[NT][3][kThreads];            // pass 1's per-thread FP32 partials S, Q, H
+  unsigned long long partE[NT][kThreads];
+  float ys[kResThreads];                  // observations of the next ticks
+  double wS[32], wQ[32], wH[32];          // record sums of 32 tiles, in their own frame
+  unsigned long long wE[32];              // their fixed-point mass, global frame
+  unsigned long long wscan[NT][kResWarps];// chunk masses of each warp, by tile
+  unsigned long long pre[NT], P[NT];      // own tiles' prefix: within their 32 tiles, global
+  unsigned long long base, delta, magic;  // the tick's targets
+  double ess_bound;                       // the smallest ESS that keeps the particles
+  int wn[32];                             // frame of each 32 tiles
+  float smax[2][kResWarps];
+  int nexp[NT];
+  __align__(16) DevState st;
+  FusedTail tail;
+};
+
+// The smallest double x with x / n >= thr as the plan rounds it (the quotient is monotone in x), so
+// that the decision is one comparison of the ESS.
+__device__ __noinline__ double ess_keep_bound(float thr, int n) {
+  const double t = (double)thr, d = (double)n;
+  double x = t * d;
+  if (!(x > 0.0) || isinf(x)) return x;
+  while (x / d >= t) x = __longlong_as_double(__double_as_longlong(x) - 1ll);
+  while (x / d < t) x = __longlong_as_double(__double_as_longlong(x) + 1ll);
+  return x;
+}
+
+// SPLIT threads share a pass-1 thread's sixteen particles; Q tiles per group of kThreads * SPLIT
+// threads: (2, 1) for one tile a CTA, (1, 1) for two, (1, 2) for three and four.
+template <bool TSTATE, bool GAUSS, bool APF, int SPLIT, int Q>
+__global__ void __launch_bounds__(kResThreads, 1)
+resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
+  constexpr int NG = kResThreads / (kThreads * SPLIT);   // groups
+  constexpr int NT = NG * Q;                    // tiles a CTA can hold
+  constexpr int GW = 8 * SPLIT;                 // warps of a group
+  constexpr int R = 4 / SPLIT;                  // float4 groups of a thread (a tile)
+  constexpr int LW = 32 / SPLIT;
+  constexpr int CH = 4 * R;                     // consecutive slots of a thread when children are counted
+  extern __shared__ __align__(16) unsigned char res_smem[];
+  ResidentShared<NT>& sh = *reinterpret_cast<ResidentShared<NT>*>(res_smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int N = p.N, G = p.G;
+  const int first = (int)blockIdx.x * nt;       // this CTA's tiles
+  const int nth = min(nt, G - first);
+  const bool keeper = blockIdx.x == gridDim.x - 1;
+  // this thread's group: tiles grp + NG q; in each, pass-1 thread v's float4 groups s R .. s R + R - 1
+  const int grp = warp / GW, gw = warp % GW, gt = tid % (kThreads * SPLIT);
+  const int s = lane / LW, v = LW * gw + (lane % LW);
+  const int l_first = 4 * (v + kThreads * s * R);        // slot of its first float4; the next is kThreads * 4 on
+  const int nwp = (G + 31) >> 5;                // groups of 32 records
+  unsigned* xw = reinterpret_cast<unsigned*>(p.xbuf);
+  const size_t mail_size = mail_bytes(G);
+  const unsigned char* mail = p.xbuf + kXHeader + (blockIdx.x % kMail) * mail_size;   // the one this CTA polls
+  const unsigned epoch = ld_relaxed_u32(xw);
+  const int Fg = min(kFixF, 62 - ceil_log2_u((unsigned)N));
+  const double rcpN = 1.0 / (double)N;
+
+  if (tid < (int)(sizeof(DevState) / 8))
+    reinterpret_cast<unsigned long long*>(&sh.st)[tid] = __ldcg(reinterpret_cast<const unsigned long long*>(p.st) + tid);
+  if (tid == kResThreads - 32) sh.ess_bound = ess_keep_bound(a.ess_threshold, N);
+  __syncthreads();
+  int nk[Q];                                    // the tiles' exponents (previous tick's until pass 1 sets them)
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int j = grp + NG * q;
+    nk[q] = kNkEmpty;
+    if (j >= nth) continue;
+    const size_t off = (size_t)(first + j) * kTile;
+    const float* hg = (sh.st.cur ? p.h1 : p.h0) + off;
+    nk[q] = __ldcg(p.nexp + first + j);
+#pragma unroll
+    for (int rr = 0; rr < R; ++rr) {
+      const int l0 = l_first + 4 * kThreads * rr;
+      *reinterpret_cast<float4*>(sh.h[j] + l0) = __ldcg(reinterpret_cast<const float4*>(hg + l0));
+      *reinterpret_cast<float4*>(sh.w[j] + l0) = __ldcg(reinterpret_cast<const float4*>(p.w + off + l0));
+    }
+  }
+  // state noise of this thread's particles for the tick with stream constants (k1, k2): read again
+  // only by this thread
+  auto noise = [&](uint64_t k1, uint64_t k2) {
+    const uint64_t k33 = k2 << 33, step2 = 2ull * k2, step_r = (uint64_t)(2 * 4 * kThreads - 8) * k2;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int j = grp + NG * q;
+      if (j >= nth) continue;
+      uint64_t sx = k1 + k2 * pcg_inc((uint32_t)((first + j) * kTile + l_first));
+#pragma unroll
+      for (int rr = 0; rr < R; ++rr) {
+        float zz[4];
+        if (rr > 0) sx += step_r;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float z = icdf_normal_warp(pcg_uniform(pcg_output(sx)));
+          if (TSTATE) z *= tstate_scale_warp(sx, k33, a.nu_int, a.nu_state);
+          zz[e] = z;
+          sx += step2;
+        }
+        *reinterpret_cast<float4*>(sh.z[j] + l_first + 4 * kThreads * rr) = make_float4(zz[0], zz[1], zz[2], zz[3]);
+      }
+    }
+  };
+  uint64_t k1 = sh.st.k1, k2 = sh.st.k2;        // stream constants of the next tick (all threads)
+  if (!APF && sh.st.tick > 0) noise(k1, k2);
+
+  unsigned xn = 0u;                             // exchanges so far
+  bool failed = false;                          // a wait gave up (the same in every thread of the CTA)
+  bool pending = false;                         // the keeper's finish of the last decision is due
+  int pending_rec = 0;
+  auto finish = [&](int apf_stage, int t) {
+    BpfTickRecord* rec = (a.rec && apf_stage != 1) ? a.rec + t : nullptr;
+    if (!APF || apf_stage == 0) {
+      fused_finish<0>(sh.tail, &sh.st, rec);
+    } else if (apf_stage == 1) {
+      fused_finish<1>(sh.tail, &sh.st, nullptr);
+    } else {
+      fused_finish<2>(sh.tail, &sh.st, rec);
+    }
+  };
+  const bool ahead = a.ess_threshold <= 0.0f;   // every tick that can resample does
+  int stage = 0, prev_stage = 0;                // APF: 0 the first tick of all, else stages 1 and 2 of a tick
+  int t = 0;
+  while (t < n_ticks) {
+    if ((!APF || stage != 2) && (t & (kResThreads - 1)) == 0) {
+      __syncthreads();
+      if (t + tid < n_ticks) sh.ys[tid] = __ldg(a.y_ptr + t + tid);
+      __syncthreads();
+    }
+    const float y = sh.ys[t & (kResThreads - 1)];
+    const int tick = sh.st.tick;
+    if (APF && stage != 2) stage = tick > 0 ? 1 : 0;
+    const int cur0 = sh.st.cur;
+    ++xn;
+    const unsigned xno = epoch + xn;
+
+    // ---- pass 1 ----
+    if (grp < nth) {
+      const bool carry = sh.st.resampled_prev == 0;
+      const int nM_prev = sh.st.nM_prev;
+      ObsModel obs = a.obs;
+      obs.y = y;
+      const float y2 = y * y;
+      const float y2nu = __fmul_rn(y2, obs.inv_nu);
+      float x[Q][4 * R];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int j = grp + NG * q;
+        if (j >= nth) continue;
+        const int tile0 = (first + j) * kTile;
+        float carry_off = 0.0f;
+        if (carry) carry_off = (nk[q] == kNkEmpty) ? -INFINITY : (float)(nk[q] - nM_prev);
+        const float gauss_c = kGaussLog2C + carry_off;
+        const float t_c = __fmul_rn(obs.c_obs, kLog2e) + carry_off;
+        auto density = [&](float h) { return GAUSS ? obs_log2pdf_gauss_plus(y2, h, gauss_c) : obs_log2pdf_t_plus(obs, y2nu, h, t_c); };
+        float* ck = (tape.ckpt && tick % tape.K == 0) ? tape.ckpt + (size_t)(tick / tape.K) * tape.ckpt_stride + tile0 : nullptr;
+#pragma unroll
+        for (int rr = 0; rr < R; ++rr) {
+          const int l0 = l_first + 4 * kThreads * rr;
+          const float4 h4 = *reinterpret_cast<const float4*>(sh.h[j] + l0);
+          if (ck) *reinterpret_cast<float4*>(ck + l0) = h4;
+          float hh[4] = {h4.x, h4.y, h4.z, h4.w};
+          float wp[4] = {0.f, 0.f, 0.f, 0.f}, zz[4] = {0.f, 0.f, 0.f, 0.f};
+          if (carry) {
+            const float4 w4 = *reinterpret_cast<const float4*>(sh.w[j] + l0);
+            wp[0] = w4.x; wp[1] = w4.y; wp[2] = w4.z; wp[3] = w4.w;
+          }
+          if (APF ? stage == 2 : tick > 0) {
+            const float4 z4 = *reinterpret_cast<const float4*>(sh.z[j] + l0);
+            zz[0] = z4.x; zz[1] = z4.y; zz[2] = z4.z; zz[3] = z4.w;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float h = hh[e], xx;
+            if (!APF || stage == 0) {
+              if (!APF && tick > 0) h = propagate(h, a.mu, a.rho, a.sigma, zz[e]);
+              xx = density(h);
+            } else {
+              const float m = propagate_mean(h, a.mu, a.rho);
+              xx = density(m);
+              if (stage == 2) {
+                h = fmaf(a.sigma, zz[e], m);
+                xx = density(h) - xx;
+              }
+            }
+            if (carry) xx += wp[e];
+            hh[e] = h;
+            x[q][4 * rr + e] = xx;
+          }
+          if (!APF || stage != 1) *reinterpret_cast<float4*>(sh.h[j] + l0) = make_float4(hh[0], hh[1], hh[2], hh[3]);
+        }
+        if (tile0 + kTile > N) {                     // padding slots carry no weight
+#pragma unroll
+          for (int i = 0; i < 4 * R; ++i)
+            if (tile0 + l_first + 4 * kThreads * (i >> 2) + (i & 3) >= N) x[q][i] = -INFINITY;
+        }
+        float mx = x[q][0];
+#pragma unroll
+        for (int e = 1; e < 4 * R; ++e) mx = fmaxf(mx, x[q][e]);
+        mx = warp_max_f(mx);
+        if (lane == 0) sh.smax[q][warp] = mx;
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int j = grp + NG * q;
+        if (j >= nth) continue;
+        const float mx = warp_max_f(sh.smax[q][grp * GW + lane % GW]);
+        nk[q] = (mx == -INFINITY) ? kNkEmpty : (int)ceilf(fmaxf(mx, -1.0e9f));
+        const float fnk = (nk[q] == kNkEmpty) ? INFINITY : (float)nk[q];
+        unsigned long long E = 0ull;
+#pragma unroll
+        for (int rr = 0; rr < R; ++rr) {
+          float dv[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            dv[e] = x[q][4 * rr + e] - fnk;
+            x[q][4 * rr + e] = tile_weight(dv[e]);       // the weight from here on
+            E += fix_weight(x[q][4 * rr + e]);
+          }
+          *reinterpret_cast<float4*>(sh.w[j] + l_first + 4 * kThreads * rr) = make_float4(dv[0], dv[1], dv[2], dv[3]);
+        }
+        // pass 1's per-thread FP32 sums, in its element order, handed along the SPLIT threads
+        float aS = 0.f, aQ = 0.f, aH = 0.f;
+#pragma unroll
+        for (int step = 0; step < SPLIT; ++step) {
+          if (SPLIT == 1 || s == step) {
+#pragma unroll
+            for (int rr = 0; rr < R; ++rr) {
+              const float4 h4 = *reinterpret_cast<const float4*>(sh.h[j] + l_first + 4 * kThreads * rr);
+              const float hv[4] = {h4.x, h4.y, h4.z, h4.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float w = x[q][4 * rr + e];
+                aS += w;
+                aQ = fmaf(w, w, aQ);
+                aH = fmaf(w, hv[e], aH);
+              }
+            }
+          }
+          if (step + 1 < SPLIT) {
+            const float nS = __shfl_up_sync(0xffffffffu, aS, LW);
+            const float nQ = __shfl_up_sync(0xffffffffu, aQ, LW);
+            const float nH = __shfl_up_sync(0xffffffffu, aH, LW);
+            if (s == step + 1) { aS = nS; aQ = nQ; aH = nH; }
+          }
+        }
+#pragma unroll
+        for (int o = LW; o < 32; o <<= 1) E += __shfl_xor_sync(0xffffffffu, E, o);
+        if (s == SPLIT - 1) { sh.part[j][0][v] = aS; sh.part[j][1][v] = aQ; sh.part[j][2][v] = aH; }
+        if (s == 0) sh.partE[j][v] = E;
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int j = grp + NG * q;
+        if (gw == q && j < nth) {                      // pass 1's FP64 tile record, published by warp q
+          double tS = 0.0, tQ = 0.0, tH = 0.0;
+          unsigned long long tE = 0ull;
+#pragma unroll
+          for (int w = 0; w < kThreads / 32; ++w) {
+            tS += (double)sh.part[j][0][lane + 32 * w];
+            tQ += (double)sh.part[j][1][lane + 32 * w];
+            tH += (double)sh.part[j][2][lane + 32 * w];
+            tE += sh.partE[j][lane + 32 * w];
+          }
+          tS = warp_sum_d(tS); tQ = warp_sum_d(tQ); tH = warp_sum_d(tH);
+          tE = warp_sum_u64(tE);
+          if (lane < kMail) {                          // (every lane holds the same sums)
+            unsigned char* slot = p.xbuf + kXHeader + lane * mail_size + mail_flag_bytes(G) +
+                                  ((size_t)(xn & 1u) * G + first + j) * 32;
+            st_relaxed_b128(slot, (unsigned long long)__float_as_uint((float)tS) | ((unsigned long long)__float_as_uint((float)tQ) << 32),
+                            (unsigned long long)(unsigned)nk[q] | ((unsigned long long)xno << 32));
+            st_relaxed_b128(slot + 16, (unsigned long long)__float_as_uint((float)tH) | (tE << 32),
+                            (tE >> 32) | ((unsigned long long)xno << 32));
+          }
+          if (lane == 0) sh.nexp[j] = nk[q];
+        }
+      }
+    }
+
+    // ---- while the records travel: the next noise, and the keeper's record of the last decision ----
+    if (!APF || stage != 1) { k1 = k1 * kPcgMult; k2 = k2 * kPcgMult + 1ull; }
+    if (APF ? stage == 1 : t + 1 < n_ticks) noise(k1, k2);
+    if (keeper && pending && tid == kResThreads - 32) finish(prev_stage, pending_rec);
+
+    // ---- exchange: lane l of the warp of 32 tiles takes its tile's record ----
+    constexpr int MAXP = (kResMaxTiles + kResThreads - 1) / kResThreads;   // records a thread may take
+    int rn[MAXP];
+    unsigned long long rE[MAXP];
+    bool bad = false;
+#pragma unroll
+    for (int u = 0; u < MAXP; ++u) {
+      rn[u] = kNkEmpty;
+      rE[u] = 0ull;
+      const int pw = warp + u * kResWarps;
+      if (pw >= nwp) continue;
+      const int k = 32 * pw + lane;
+      // The loop leaves by a warp vote: a lane that left alone would keep the warp split through the
+      // shuffles below (measured 3.5 us for the sums after a spin, 0.13 us together).
+      const unsigned char* slot = mail + mail_flag_bytes(G) + ((size_t)(xn & 1u) * G + min(k, G - 1)) * 32;
+      unsigned long long a0 = 0ull, a1 = 0ull, b0 = 0ull, b1 = 0ull;
+      Patience pt;
+      for (;;) {
+        ld_relaxed_b128(slot, a0, a1);
+        ld_relaxed_b128(slot + 16, b0, b1);
+        const bool ok = (unsigned)(a1 >> 32) == xno && (unsigned)(b1 >> 32) == xno;
+        if (__all_sync(0xffffffffu, ok)) break;
+        if (!pt.more(xw + 1, epoch + 1u)) { bad = true; break; }     // the same in every lane
+      }
+      float rS = 0.f, rQ = 0.f, rH = 0.f;
+      if (k < G && !bad) {
+        rS = __uint_as_float((unsigned)a0); rQ = __uint_as_float((unsigned)(a0 >> 32));
+        rn[u] = (int)(unsigned)a1;
+        rH = __uint_as_float((unsigned)b0);
+        rE[u] = (b0 >> 32) | (b1 << 32);
+      }
+      // the plan's sums of 32 tiles, in their own frame: scaling by a power of two is exact, so moving
+      // them to the global frame afterwards gives the plan's values
+      const int nW = __reduce_max_sync(0xffffffffu, rn[u]);
+      double S = 0.0, Qs = 0.0, H = 0.0;
+      if (rn[u] != kNkEmpty) {
+        const double sc = pow2d(rn[u] - nW);
+        S = (double)rS * sc; Qs = (double)rQ * (sc * sc); H = (double)rH * sc;
+      }
+      S = warp_sum_d(S); Qs = warp_sum_d(Qs); H = warp_sum_d(H);
+      if (lane == 0) { sh.wn[pw] = nW; sh.wS[pw] = S; sh.wQ[pw] = Qs; sh.wH[pw] = H; }
+    }
+    if (__syncthreads_or(bad)) { failed = true; break; }
+
+    // ---- decision (the last warp), and beside it, when every tick resamples, the masses ----
+    const int nM = __reduce_max_sync(0xffffffffu, lane < nwp ? sh.wn[lane] : kNkEmpty);
+    if (warp == kResWarps - 1) {
+      double S = 0.0, Qs = 0.0, H = 0.0;
+      if (lane < nwp && sh.wn[lane] != kNkEmpty) {
+        const double sc = pow2d(sh.wn[lane] - nM);
+        S = sh.wS[lane] * sc; Qs = sh.wQ[lane] * sc * sc; H = sh.wH[lane] * sc;
+      }
+      double tS = 0.0, tQ = 0.0, tH = 0.0;
+      for (int w = 0; w < nwp; ++w) {
+        tS += __shfl_sync(0xffffffffu, S, w);
+        tQ += __shfl_sync(0xffffffffu, Qs, w);
+        tH += __shfl_sync(0xffffffffu, H, w);
+      }
+      if (lane == 0) {
+        if (APF && stage == 1) fused_decide<1>(a, N, nM, tS, tQ, tH, &sh.st, sh.tail, sh.ess_bound);
+        else fused_decide<0>(a, N, nM, tS, tQ, tH, &sh.st, sh.tail, sh.ess_bound);
+        if (tape.aux && keeper)
+          tape.aux[tick] = sh.tail.degenerate ? make_float2(0.0f, __int_as_float(0))
+                                              : make_float2((float)(1.0 / tS), __int_as_float(nM));
+      }
+      __syncwarp();
+    }
+    pending = true;
+    pending_rec = t;
+    prev_stage = stage;
+    if (!ahead) __syncthreads();
+    if (ahead || sh.st.do_resample) {
+      // exact fixed-point masses: the tiles' in the global frame, and the own tiles' chunks of CH slots
+#pragma unroll
+      for (int u = 0; u < MAXP; ++u) {
+        const int pw = warp + u * kResWarps;
+        if (pw >= nwp) continue;
+        const int k = 32 * pw + lane;
+        rE[u] = (rn[u] != kNkEmpty) ? shr64(rE[u], nM - rn[u] + kFixF - Fg) : 0ull;
+        const unsigned long long incl = warp_incl_scan_add(rE[u], lane);
+        if (lane == 31) sh.wE[pw] = incl;
+        if (k >= first && k < first + nth) sh.pre[k - first] = incl - rE[u];
+        rE[u] = incl;                              // the prefix through tile k from here on
+      }
+      unsigned long long loc[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int j = grp + NG * q;
+        loc[q] = 0ull;
+        if (j >= nth) continue;
+        unsigned long long e = 0ull;
+#pragma unroll
+        for (int g = 0; g < CH / 4; ++g) {
+          const float4 d4 = *reinterpret_cast<const float4*>(sh.w[j] + CH * gt + 4 * g);
+          e += fix_weight(tile_weight(d4.x)) + fix_weight(tile_weight(d4.y));
+          e += fix_weight(tile_weight(d4.z)) + fix_weight(tile_weight(d4.w));
+        }
+        const unsigned long long incl = warp_incl_scan_add(e, lane);
+        if (lane == 31) sh.wscan[j][gw] = incl;
+        loc[q] = incl - e;
+      }
+      __syncthreads();
+      if (sh.st.do_resample) {
+        // the targets, and the own tiles' prefixes (every warp forms the totals; warp 0 the rest)
+        const unsigned long long we = lane < nwp ? sh.wE[lane] : 0ull;
+        const unsigned long long winc = warp_incl_scan_add(we, lane);
+        if (warp == 0) {
+          const unsigned long long total = __shfl_sync(0xffffffffu, winc, 31);
+          const int mine = first + min(lane, nth - 1);
+          const unsigned long long before = __shfl_sync(0xffffffffu, winc - we, mine >> 5);
+          if (lane < nth) sh.P[lane] = sh.pre[lane] + before;
+          unsigned long long delta = udiv_fp64_rcp(total, (unsigned long long)N, rcpN);
+          const bool zero_spacing = delta == 0ull;
+          if (zero_spacing) delta = 1ull;
+          const unsigned long long u = sh.st.u23;
+          const unsigned long long hi = __umul64hi(u, delta), lo = u * delta;
+          if (lane == 0) {
+            DevState& st = sh.st;
+            sh.base = (hi << 41) | (lo >> 23);       // floor(u * delta / 2^23)
+            sh.delta = delta;
+            sh.magic = udiv_magic_of(delta);
+            if (zero_spacing) st.error = BPF_ERR_DEGENERATE;
+            st.base = sh.base; st.delta = delta; st.delta_magic = sh.magic; st.total = total; st.Fg = Fg;
+          }
+        }
+        __syncthreads();
+        const unsigned long long base = sh.base, delta = sh.delta, magic = sh.magic;
+        float* hdst = cur0 ? p.h0 : p.h1;
+        const int slot_lo = first * kTile, slot_hi = (first + nth) * kTile;
+        // which CTAs write children into this CTA's slots: bit u, tile 32 (warp + u kResWarps) + lane
+        unsigned need = 0u;
+#pragma unroll
+        for (int u = 0; u < MAXP; ++u) {
+          const int pw = warp + u * kResWarps;
+          if (pw >= nwp) continue;
+          const int k = 32 * pw + lane;
+          const unsigned long long before = __shfl_sync(0xffffffffu, winc - we, pw);
+          const int o1 = targets_below(before + rE[u], base, delta, magic, N);
+          int o0 = __shfl_up_sync(0xffffffffu, o1, 1);
+          if (lane == 0) o0 = targets_below(before, base, delta, magic, N);
+          if (k < G && o1 > o0 && o0 < slot_hi && o1 > slot_lo && (k < first || k >= first + nth)) need |= 1u << u;
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const int j = grp + NG * q;
+          if (j >= nth) continue;                    // whole groups
+          const unsigned long long off = warp_sum_u64(lane < gw ? sh.wscan[j][lane] : 0ull);
+          const int tk = sh.nexp[j];
+          const int r = (tk == kNkEmpty) ? 64 : nM - tk + kFixF - Fg;
+          const int j0 = (first + j) * kTile + CH * gt;
+          const float* d = sh.w[j] + CH * gt;
+          ChunkTargets<CH> ct;
+          ct.c = gt;
+          ct.lfT = 0.0f;
+          float hv[CH];
+#pragma unroll
+          for (int g = 0; g < CH / 4; ++g) {
+            const float4 d4 = *reinterpret_cast<const float4*>(d + 4 * g);
+            const float4 h4 = *reinterpret_cast<const float4*>(sh.h[j] + CH * gt + 4 * g);
+            ct.wf[4 * g] = tile_weight(d4.x); ct.wf[4 * g + 1] = tile_weight(d4.y);
+            ct.wf[4 * g + 2] = tile_weight(d4.z); ct.wf[4 * g + 3] = tile_weight(d4.w);
+            hv[4 * g] = h4.x; hv[4 * g + 1] = h4.y; hv[4 * g + 2] = h4.z; hv[4 * g + 3] = h4.w;
+          }
+#pragma unroll
+          for (int e = 0; e < CH; ++e) ct.lfT += ct.wf[e];
+          chunk_thresholds<CH>(N, off + loc[q], sh.P[j], r, j0 < N, base, delta, magic, ct);
+          int qe[CH];
+          chunk_child_ends<CH>(N, ct, d, qe);
+          if (tape.csr) {                            // first child of each parent
+            int32_t* cs = tape.csr + (size_t)tick * tape.csr_stride + j0;
+#pragma unroll
+            for (int g = 0; g < CH / 4; ++g) {
+              const int4 f4 = make_int4(g ? qe[4 * g - 1] : ct.q, qe[4 * g], qe[4 * g + 1], qe[4 * g + 2]);
+              if (j0 + 4 * g + 4 <= N) {
+                *reinterpret_cast<int4*>(cs + 4 * g) = f4;
+              } else {
+                const int f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) if (j0 + 4 * g + e < N) cs[4 * g + e] = f[e];
+              }
+            }
+          }
+          // Every thread of the group holds its particles in registers, so the tile's shared-memory
+          // copy takes the children that fall into its own slots; the others go to the other
+          // particle buffer, for the CTA that owns them.
+          asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");
+          const int own = (first + j) * kTile;
+          float* hown = sh.h[j];
+          auto put = [&](int o, float hc, int anc) {
+            if ((unsigned)(o - own) < (unsigned)kTile) hown[o - own] = hc;
+            else hdst[o] = hc;
+            if (a.anc) a.anc[o] = anc;
+          };
+          int qp = ct.q;
+#pragma unroll
+          for (int e = 0; e < CH; ++e) {
+            const int q1 = qe[e];
+            if (q1 - qp <= kResHeavy)
+              for (int o = qp; o < q1; ++o) put(o, hv[e], j0 + e);
+            qp = q1;
+          }
+          // long runs are shared by the warp
+          bool any_heavy = false;
+#pragma unroll
+          for (int e = 0; e < CH; ++e) any_heavy |= qe[e] - (e ? qe[e - 1] : ct.q) > kResHeavy;
+          if (__any_sync(0xffffffffu, any_heavy)) {
+#pragma unroll
+            for (int e = 0; e < CH; ++e) {
+              const int b0 = e ? qe[e - 1] : ct.q, b1 = qe[e];
+              unsigned heavy = __ballot_sync(0xffffffffu, b1 - b0 > kResHeavy);
+              while (heavy) {
+                const int src = __ffs(heavy) - 1;
+                heavy &= heavy - 1u;
+                const int c0 = __shfl_sync(0xffffffffu, b0, src), c1 = __shfl_sync(0xffffffffu, b1, src);
+                const float hc = __shfl_sync(0xffffffffu, hv[e], src);
+                const int an = __shfl_sync(0xffffffffu, j0 + e, src);
+                for (int o = c0 + lane; o < c1; o += 32) put(o, hc, an);
+              }
+            }
+          }
+          // slots of this tile that its own children do not fill are loaded after the flags
+        }
+        // every CTA whose children fall into this CTA's slots has written them before they are read
+        __syncthreads();
+        if (tid < kMail) {
+          __threadfence();
+          st_release_u32(reinterpret_cast<unsigned*>(p.xbuf + kXHeader + tid * mail_size) + blockIdx.x, xno);
+        }
+#pragma unroll
+        for (int u = 0; u < MAXP; ++u) {
+          const bool wait = (need & (1u << u)) != 0u;
+          if (!__any_sync(0xffffffffu, wait)) continue;
+          const unsigned* flag = reinterpret_cast<const unsigned*>(mail) + (wait ? (32 * (warp + u * kResWarps) + lane) / nt : (int)blockIdx.x);
+          Patience pt;
+          for (;;) {                              // left by a warp vote, as above
+            const bool ok = !wait || (int)(ld_relaxed_u32(flag) - xno) >= 0;
+            if (__all_sync(0xffffffffu, ok)) break;
+            if (!pt.more(xw + 1, epoch + 1u)) { bad = true; break; }
+          }
+          __threadfence();                        // acquire (a relaxed poll leaves L1 alone)
+        }
+        if (__syncthreads_or(bad)) { failed = true; break; }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const int j = grp + NG * q;
+          if (j >= nth) continue;
+          // the tile's own children fill the slots [c0, c1) of it
+          const int own = (first + j) * kTile;
+          const int tk = sh.nexp[j];
+          const int r = (tk == kNkEmpty) ? 64 : nM - tk + kFixF - Fg;
+          unsigned long long mass = 0ull;
+          for (int w = 0; w < GW; ++w) mass += sh.wscan[j][w];
+          const int c0 = targets_below(sh.P[j], base, delta, magic, N) - own;
+          const int c1 = targets_below(sh.P[j] + shr64(mass, r), base, delta, magic, N) - own;
+#pragma unroll
+          for (int rr = 0; rr < R; ++rr) {
+            const int l0 = l_first + 4 * kThreads * rr;
+            if (l0 >= c0 && l0 + 4 <= c1) continue;
+            const float4 g4 = __ldcg(reinterpret_cast<const float4*>(hdst + own + l0));
+            const float hv[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (l0 + e < c0 || l0 + e >= c1) sh.h[j][l0 + e] = hv[e];
+          }
+        }
+      }
+    }
+    if (APF && stage == 1) {
+      stage = 2;
+    } else {
+      stage = 0;
+      ++t;
+    }
+  }
+
+  if (tid == kResThreads - 32 && pending && keeper && !failed) finish(prev_stage, pending_rec);
+  __syncthreads();
+  if (failed && tid == 0) st_release_u32(xw + 1, epoch + 1u);   // the other CTAs stop waiting
+  if (!failed) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int j = grp + NG * q;
+      if (j >= nth) continue;
+      const size_t off = (size_t)(first + j) * kTile;
+      float* hg = (sh.st.cur ? p.h1 : p.h0) + off;
+#pragma unroll
+      for (int rr = 0; rr < R; ++rr) {
+        const int l0 = l_first + 4 * kThreads * rr;
+        *reinterpret_cast<float4*>(hg + l0) = *reinterpret_cast<const float4*>(sh.h[j] + l0);
+        *reinterpret_cast<float4*>(p.w + off + l0) = *reinterpret_cast<const float4*>(sh.w[j] + l0);
+      }
+      if (gt == 0) p.nexp[first + j] = nk[q];
+    }
+  }
+  if (keeper) {
+    if (tid == 0) {
+      if (failed) sh.st.error = BPF_ERR_STATE;
+      *reinterpret_cast<volatile unsigned*>(xw) = epoch + 4u * (unsigned)n_ticks + 4u;   // past every number used
+    }
+    __syncthreads();
+    if (tid < (int)(sizeof(DevState) / 8))
+      reinterpret_cast<unsigned long long*>(p.st)[tid] = reinterpret_cast<const unsigned long long*>(&sh.st)[tid];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Launcher
+// ---------------------------------------------------------------------------
+namespace {
+
+using ResidentKernel = void (*)(Plan, TickArgs, ResidentTape, int, int);
+
+template <bool APF, int SPLIT, int Q>
+ResidentKernel pick_model(bool tstate, bool gauss, size_t* smem) {
+  *smem = sizeof(ResidentShared<kResThreads / (kThreads * SPLIT) * Q>);
+  if (tstate) return gauss ? resident_kernel<true, true, APF, SPLIT, Q> : resident_kernel<true, false, APF, SPLIT, Q>;
+  return gauss ? resident_kernel<false, true, APF, SPLIT, Q> : resident_kernel<false, false, APF, SPLIT, Q>;
+}
+template <bool APF>
+ResidentKernel pick_shape(int nt, bool tstate, bool gauss, size_t* smem) {
+  if (nt <= 1) return pick_model<APF, 2, 1>(tstate, gauss, smem);
+  if (nt <= 2) return pick_model<APF, 1, 1>(tstate, gauss, smem);
+  return pick_model<APF, 1, 2>(tstate, gauss, smem);
+}
+ResidentKernel pick(int nt, bool tstate, bool gauss, bool apf, size_t* smem) {
+  return apf ? pick_shape<true>(nt, tstate, gauss, smem) : pick_shape<false>(nt, tstate, gauss, smem);
+}
+
+constexpr int kMaxConfiguredDevices = 64;
+std::mutex g_lock;
+int g_sms[kMaxConfiguredDevices] = {};       // 0: not looked at yet, -1: no resident runs on this device
+
+}  // namespace
+
+int resident_max_tiles(int device) {
+  if (device < 0 || device >= kMaxConfiguredDevices) return 0;
+  std::lock_guard<std::mutex> guard(g_lock);
+  if (g_sms[device] == 0) {
+    int sms = 0, coop = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    bool ok = coop != 0 && sms > 0 && sms * kResMaxTilesPerCta <= kResMaxTiles;
+    for (int m = 0; m < 8 && ok; ++m)
+      for (int nt : {1, 2, 4}) {
+        size_t smem = 0;
+        ResidentKernel k = pick(nt, m & 1, m & 2, m & 4, &smem);
+        int per = 0;
+        ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kResThreads, smem) == cudaSuccess && per >= 1;
+      }
+    if (!ok) cudaGetLastError();
+    g_sms[device] = ok ? sms : -1;
+  }
+  return g_sms[device] > 0 ? g_sms[device] * kResMaxTilesPerCta : 0;
+}
+
+cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
+                            int max_tiles, cudaStream_t s) {
+  if (!p.xbuf || p.G < 1 || p.G > max_tiles || n_ticks < 1 || !a.y_ptr) return cudaErrorInvalidValue;
+  const int sms = max_tiles / kResMaxTilesPerCta;
+  const int nt = (p.G + sms - 1) / sms;
+  size_t smem = 0;
+  ResidentKernel k = pick(nt, a.nu_int > 0, !(a.obs.nu > 0.0f), apf, &smem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((p.G + nt - 1) / nt);
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, p, a, tape, n_ticks, nt);
+}
+
+}  // namespace bpf

@@ -240,8 +240,10 @@ int    gpu_bpf_load(GpuBpfState* state, const void* buf, size_t len);
  * reading each other's through distributed shared memory), and a captured run of
  * ticks (gpu_bpf_step_many, gpu_bpf_step_many_device) as one launch for the whole
  * run, with results bit-identical to the three-kernel tick. Filters of more than
- * 32768 particles take it where the device schedules a cluster of 16 CTAs. On by
- * default; enable = 0 selects the three-kernel tick. Learning filters, Silverman
+ * 32768 particles take it where the device schedules a cluster of 16 CTAs. Runs of
+ * ticks of larger filters, up to four 4096-particle tiles per SM (2.4 million
+ * particles on 148 SMs), stay on the chip as one cooperative launch, bit-identical
+ * too. On by default; enable = 0 selects the three-kernel tick for both. Learning filters, Silverman
  * jitter and profiled ticks always take the three-kernel path. */
 int gpu_bpf_set_fused_small(GpuBpfState* state, int enable);
 

@@ -1,0 +1,93 @@
+"""Resident runs (csrc/bpf_resident.cu): consecutive ticks of a medium filter as one cooperative
+launch. The records, ancestors, particles and weights equal the tick-per-launch path's bit for bit
+(gpu_bpf_set_fused_small(state, 0) selects that one), so the tolerance is zero."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+RHO, SIG, MU = 0.97, 0.15, -1.0
+TILE = 4096
+
+
+def _series(T, seed, outliers=False):
+    from gpubpf import dgp
+    y = np.asarray(dgp.matched_series(T, RHO, SIG, MU, seed)[1], dtype=np.float32)
+    if outliers:                      # a few particles take nearly all of the weight
+        y[T // 3] = 40.0
+        y[T // 2] = -90.0
+    return y
+
+
+def _device_run(bpf, N, thr, nu_obs, nu_state, y, fused, seeds, anc=False):
+    import torch
+    T = len(y)
+    yd = torch.tensor(y, device="cuda")
+    rec = torch.zeros(T * 40, dtype=torch.uint8, device="cuda")
+    f = bpf.GpuBpf(N, RHO, SIG, MU, nu_state, nu_obs, 17, ess_threshold=thr)
+    f.set_fused_small(fused)
+    if anc:
+        f.record_ancestors(True)
+    out = []
+    for seed in seeds:                # the second run replays the captured launch
+        f.reset(seed)
+        f.step_many_device(yd.data_ptr(), T, rec.data_ptr())
+        torch.cuda.synchronize()
+        w, te, u23 = f.get_resample_inputs()
+        out.append((rec.cpu().numpy().tobytes(), bytes(f.get_particles()), bytes(w), bytes(te), u23,
+                    f.get_loglik_total(), f.get_resample_count(), bytes(f.get_ancestors()[1]) if anc else b""))
+    f.close()
+    return out
+
+
+# one tile more than the cluster path takes; one, two, three and four tiles a CTA at their edges
+@pytest.mark.parametrize("N,thr,nu_obs,nu_state,outliers", [
+    (65537, 0.5, 0.0, 0.0, False), (74 * TILE - 1, 0.0, 0.0, 0.0, True), (148 * TILE, 0.5, 5.0, 0.0, False),
+    (148 * TILE + 1, 0.0, 0.0, 5.0, False), (1000003, 0.5, 5.0, 5.0, True), (296 * TILE, 0.5, 0.0, 6.0, False),
+    (296 * TILE + 5, 0.0, 5.0, 0.0, True), (1500000, 0.5, 0.0, 0.0, False), (592 * TILE, 0.5, 0.0, 0.0, True),
+    (592 * TILE - 4097, 0.0, 0.0, 0.0, False)])
+def test_resident_run_matches_tick_launches(bpf, N, thr, nu_obs, nu_state, outliers):
+    y = _series(60, 9, outliers)
+    a = _device_run(bpf, N, thr, nu_obs, nu_state, y, True, (17, 5), anc=True)
+    b = _device_run(bpf, N, thr, nu_obs, nu_state, y, False, (17, 5), anc=True)
+    assert a == b
+    assert a[0] != a[1]
+
+
+def test_resident_long_run_restages_observations(bpf):
+    y = _series(2500, 42)
+    assert _device_run(bpf, 100001, 0.5, 0.0, 0.0, y, True, (3,)) == _device_run(bpf, 100001, 0.5, 0.0, 0.0, y, False, (3,))
+
+
+@pytest.mark.parametrize("N,thr", [(70000, 0.0), (700001, 0.5)])
+def test_resident_host_runs_and_single_ticks_interleave(bpf, N, thr):
+    """step_many (chunks and a remainder), single steps and a checkpoint between them."""
+    y = _series(200, 21).tolist()
+
+    def run(fused):
+        f = bpf.GpuBpf(N, RHO, SIG, MU, seed=4, ess_threshold=thr)
+        f.set_fused_small(fused)
+        recs = f.step_many(y[:70], records=True)
+        for v in y[70:73]:
+            f.step(v)
+            recs.append(f.get_record())
+        blob = f.save()
+        recs += f.step_many(y[73:], records=True)
+        f.load(blob)
+        recs += f.step_many(y[73:], records=True)
+        parts = bytes(f.get_particles())
+        f.close()
+        return [bytes(r) for r in recs], parts
+
+    assert run(True) == run(False)
+
+
+def test_resident_degenerate_tick(bpf):
+    """A tick whose every weight underflows: the same records as tick by tick."""
+    y = _series(40, 3)
+    y[20] = 3e18
+    a = _device_run(bpf, 80000, 0.5, 0.0, 0.0, y, True, (17,))
+    b = _device_run(bpf, 80000, 0.5, 0.0, 0.0, y, False, (17,))
+    assert a == b
