@@ -1522,7 +1522,8 @@ __device__ __forceinline__ void count_write(const TickArgs& a, int N, int k, con
   const float* hs = sh.h[src] + CH * ct.c;         // its particles
   const int q0 = ct.q;
   int qe[CH];                                      // q_j: the end of element j's children
-  chunk_child_ends<CH>(N, ct, sh.w + CH * ct.c, qe);
+  const float* d = sh.w + CH * ct.c;               // its log2-weights
+  chunk_child_ends<CH>(N, ct, qe, [&](int upto) { return exact_count(d, upto, ct.th, ct.D, N); });
   // The chunk's children fill the slots [q0, q_last): slot o belongs to element #{j : q_j <= o}.
   // Each lane writes its run in one loop, starting at an offset rotated by lane / 4: the runs of
   // a warp's lanes start about eight slots apart, so without the rotation eight lanes would store

@@ -85,23 +85,58 @@ struct Patience {
   }
 };
 
-template <int NT>
+// A tile's particles and log2-weights in shared memory: float4 group i4 sits at swz4(i4), so that a
+// warp reading CH consecutive slots a lane (the child counts) falls on distinct banks, as one reading
+// consecutive groups (pass 1) does.
+__device__ __forceinline__ int swz4(int i4) { return i4 ^ ((i4 >> 3) & 7); }
+__device__ __forceinline__ float4 ld4(const float* tile, int i) { return reinterpret_cast<const float4*>(tile)[swz4(i >> 2)]; }
+__device__ __forceinline__ void st4(float* tile, int i, float4 v) { reinterpret_cast<float4*>(tile)[swz4(i >> 2)] = v; }
+__device__ __forceinline__ float& el(float* tile, int i) { return tile[(swz4(i >> 2) << 2) | (i & 3)]; }
+
+// exact_count on a swizzled tile: the element's chunk starts at slot i0.
+static __device__ __noinline__ int exact_count_swz(const float* tile, int i0, int upto, unsigned long long R0,
+                                                   unsigned long long D, int cap) {
+  unsigned long long l = 0ull;
+  for (int i = i0; i <= i0 + upto; ++i) l += fix_weight(tile_weight(tile[(swz4(i >> 2) << 2) | (i & 3)]));
+  if (l < R0) return 0;
+  const unsigned long long c = udiv_fp64(l - R0, D) + 1ull;
+  return c >= (unsigned long long)cap ? cap : (int)c;
+}
+
+// Output slots a tile's children are gathered in: a window of kResSteps steps of 128 slots a warp,
+// from the tile's first output rounded down to a float4. Children past it are written one by one.
+template <int SPLIT> struct ResWindow {
+  static constexpr int kSteps = SPLIT == 1 ? 5 : 3;
+  static constexpr int kSlots = 8 * SPLIT * kSteps * 128;      // 5120, 6144
+};
+
+template <int NT, int SPLIT>
 struct ResidentShared {
+  static constexpr int NG = kResThreads / (kThreads * SPLIT);
   float h[NT][kTile];                     // particles
   float w[NT][kTile];                     // tile-relative log2-weights
   float z[NT][kTile];                     // state noise of the next propagation
-  float part[NT][3][kThreads];            // pass 1's per-thread FP32 partials S, Q, H
-  unsigned long long partE[NT][kThreads];
+  union {
+    struct {
+      float part[NT][3][kThreads];        // pass 1's per-thread FP32 partials S, Q, H
+      unsigned long long partE[NT][kThreads];
+    };
+    unsigned short marks[NG][ResWindow<SPLIT>::kSlots];   // resampling: start marks of a tile's children
+  };
   float ys[kResThreads];                  // observations of the next ticks
   double wS[32], wQ[32], wH[32];          // record sums of 32 tiles, in their own frame
   unsigned long long wE[32];              // their fixed-point mass, global frame
   unsigned long long wscan[NT][kResWarps];// chunk masses of each warp, by tile
-  unsigned long long pre[NT], P[NT];      // own tiles' prefix: within their 32 tiles, global
+  unsigned long long pre[NT], mass[NT], P[NT];   // own tiles: prefix within their 32 tiles, mass, global prefix
   unsigned long long base, delta, magic;  // the tick's targets
+  unsigned long long ustate;              // resampling-uniform PCG32
   double ess_bound;                       // the smallest ESS that keeps the particles
   int wn[32];                             // frame of each 32 tiles
+  int c0[NT], c1[NT];                     // own tiles' first output slots and their ends
   float smax[2][kResWarps];
+  unsigned wmax[kResWarps];
   int nexp[NT];
+  int resample, degenerate;               // this tick's decision
   __align__(16) DevState st;
   FusedTail tail;
 };
@@ -128,8 +163,9 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
   constexpr int R = 4 / SPLIT;                  // float4 groups of a thread (a tile)
   constexpr int LW = 32 / SPLIT;
   constexpr int CH = 4 * R;                     // consecutive slots of a thread when children are counted
+  constexpr int STEPS = ResWindow<SPLIT>::kSteps, WSLOTS = ResWindow<SPLIT>::kSlots;
   extern __shared__ __align__(16) unsigned char res_smem[];
-  ResidentShared<NT>& sh = *reinterpret_cast<ResidentShared<NT>*>(res_smem);
+  ResidentShared<NT, SPLIT>& sh = *reinterpret_cast<ResidentShared<NT, SPLIT>*>(res_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = p.N, G = p.G;
   const int first = (int)blockIdx.x * nt;       // this CTA's tiles
@@ -151,6 +187,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
     reinterpret_cast<unsigned long long*>(&sh.st)[tid] = __ldcg(reinterpret_cast<const unsigned long long*>(p.st) + tid);
   if (tid == kResThreads - 32) sh.ess_bound = ess_keep_bound(a.ess_threshold, N);
   __syncthreads();
+  if (tid == 0) sh.ustate = sh.st.u_state;
   int nk[Q];                                    // the tiles' exponents (previous tick's until pass 1 sets them)
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
@@ -163,8 +200,8 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {
       const int l0 = l_first + 4 * kThreads * rr;
-      *reinterpret_cast<float4*>(sh.h[j] + l0) = __ldcg(reinterpret_cast<const float4*>(hg + l0));
-      *reinterpret_cast<float4*>(sh.w[j] + l0) = __ldcg(reinterpret_cast<const float4*>(p.w + off + l0));
+      st4(sh.h[j], l0, __ldcg(reinterpret_cast<const float4*>(hg + l0)));
+      st4(sh.w[j], l0, __ldcg(reinterpret_cast<const float4*>(p.w + off + l0)));
     }
   }
   // state noise of this thread's particles for the tick with stream constants (k1, k2): read again
@@ -194,19 +231,31 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
   uint64_t k1 = sh.st.k1, k2 = sh.st.k2;        // stream constants of the next tick (all threads)
   if (!APF && sh.st.tick > 0) noise(k1, k2);
 
+  // what every thread follows of the device state; the keeper's copy is brought up to date (and the
+  // record written) during the next exchange, from the sums its decision left with thread kDecider
+  int tick = sh.st.tick, cur = sh.st.cur, nM_prev = sh.st.nM_prev;
+  bool carry = sh.st.resampled_prev == 0;
+  constexpr int kDecider = kResThreads - 32;
+  double dS = 0.0, dQ = 0.0, dH = 0.0;
+  int d_nM = 0;
   unsigned xn = 0u;                             // exchanges so far
   bool failed = false;                          // a wait gave up (the same in every thread of the CTA)
-  bool pending = false;                         // the keeper's finish of the last decision is due
+  bool pending = false;                         // the keeper's state is one decision behind
   int pending_rec = 0;
-  auto finish = [&](int apf_stage, int t) {
+  auto settle = [&](int apf_stage, int t) {
     BpfTickRecord* rec = (a.rec && apf_stage != 1) ? a.rec + t : nullptr;
-    if (!APF || apf_stage == 0) {
-      fused_finish<0>(sh.tail, &sh.st, rec);
-    } else if (apf_stage == 1) {
+    const int tk = sh.st.tick;
+    if (APF && apf_stage == 1) {
+      fused_decide<1>(a, N, d_nM, dS, dQ, dH, &sh.st, sh.tail);
       fused_finish<1>(sh.tail, &sh.st, nullptr);
     } else {
-      fused_finish<2>(sh.tail, &sh.st, rec);
+      fused_decide<0>(a, N, d_nM, dS, dQ, dH, &sh.st, sh.tail);
+      if (APF && apf_stage == 2) fused_finish<2>(sh.tail, &sh.st, rec);
+      else fused_finish<0>(sh.tail, &sh.st, rec);
     }
+    if (tape.aux)
+      tape.aux[tk] = sh.tail.degenerate ? make_float2(0.0f, __int_as_float(0))
+                                        : make_float2((float)(1.0 / dS), __int_as_float(d_nM));
   };
   const bool ahead = a.ess_threshold <= 0.0f;   // every tick that can resample does
   int stage = 0, prev_stage = 0;                // APF: 0 the first tick of all, else stages 1 and 2 of a tick
@@ -218,16 +267,12 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       __syncthreads();
     }
     const float y = sh.ys[t & (kResThreads - 1)];
-    const int tick = sh.st.tick;
     if (APF && stage != 2) stage = tick > 0 ? 1 : 0;
-    const int cur0 = sh.st.cur;
     ++xn;
     const unsigned xno = epoch + xn;
 
     // ---- pass 1 ----
     if (grp < nth) {
-      const bool carry = sh.st.resampled_prev == 0;
-      const int nM_prev = sh.st.nM_prev;
       ObsModel obs = a.obs;
       obs.y = y;
       const float y2 = y * y;
@@ -247,12 +292,12 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
 #pragma unroll
         for (int rr = 0; rr < R; ++rr) {
           const int l0 = l_first + 4 * kThreads * rr;
-          const float4 h4 = *reinterpret_cast<const float4*>(sh.h[j] + l0);
+          const float4 h4 = ld4(sh.h[j], l0);
           if (ck) *reinterpret_cast<float4*>(ck + l0) = h4;
           float hh[4] = {h4.x, h4.y, h4.z, h4.w};
           float wp[4] = {0.f, 0.f, 0.f, 0.f}, zz[4] = {0.f, 0.f, 0.f, 0.f};
           if (carry) {
-            const float4 w4 = *reinterpret_cast<const float4*>(sh.w[j] + l0);
+            const float4 w4 = ld4(sh.w[j], l0);
             wp[0] = w4.x; wp[1] = w4.y; wp[2] = w4.z; wp[3] = w4.w;
           }
           if (APF ? stage == 2 : tick > 0) {
@@ -277,7 +322,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
             hh[e] = h;
             x[q][4 * rr + e] = xx;
           }
-          if (!APF || stage != 1) *reinterpret_cast<float4*>(sh.h[j] + l0) = make_float4(hh[0], hh[1], hh[2], hh[3]);
+          if (!APF || stage != 1) st4(sh.h[j], l0, make_float4(hh[0], hh[1], hh[2], hh[3]));
         }
         if (tile0 + kTile > N) {                     // padding slots carry no weight
 #pragma unroll
@@ -308,7 +353,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
             x[q][4 * rr + e] = tile_weight(dv[e]);       // the weight from here on
             E += fix_weight(x[q][4 * rr + e]);
           }
-          *reinterpret_cast<float4*>(sh.w[j] + l_first + 4 * kThreads * rr) = make_float4(dv[0], dv[1], dv[2], dv[3]);
+          st4(sh.w[j], l_first + 4 * kThreads * rr, make_float4(dv[0], dv[1], dv[2], dv[3]));
         }
         // pass 1's per-thread FP32 sums, in its element order, handed along the SPLIT threads
         float aS = 0.f, aQ = 0.f, aH = 0.f;
@@ -317,7 +362,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
           if (SPLIT == 1 || s == step) {
 #pragma unroll
             for (int rr = 0; rr < R; ++rr) {
-              const float4 h4 = *reinterpret_cast<const float4*>(sh.h[j] + l_first + 4 * kThreads * rr);
+              const float4 h4 = ld4(sh.h[j], l_first + 4 * kThreads * rr);
               const float hv[4] = {h4.x, h4.y, h4.z, h4.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -369,10 +414,10 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       }
     }
 
-    // ---- while the records travel: the next noise, and the keeper's record of the last decision ----
+    // ---- while the records travel: the next noise, and the keeper's state and record of the last tick ----
     if (!APF || stage != 1) { k1 = k1 * kPcgMult; k2 = k2 * kPcgMult + 1ull; }
     if (APF ? stage == 1 : t + 1 < n_ticks) noise(k1, k2);
-    if (keeper && pending && tid == kResThreads - 32) finish(prev_stage, pending_rec);
+    if (keeper && pending && tid == kDecider) settle(prev_stage, pending_rec);
 
     // ---- exchange: lane l of the warp of 32 tiles takes its tile's record ----
     constexpr int MAXP = (kResMaxTiles + kResThreads - 1) / kResThreads;   // records a thread may take
@@ -432,12 +477,18 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
         tQ += __shfl_sync(0xffffffffu, Qs, w);
         tH += __shfl_sync(0xffffffffu, H, w);
       }
+      dS = tS; dQ = tQ; dH = tH; d_nM = nM;
       if (lane == 0) {
-        if (APF && stage == 1) fused_decide<1>(a, N, nM, tS, tQ, tH, &sh.st, sh.tail, sh.ess_bound);
-        else fused_decide<0>(a, N, nM, tS, tQ, tH, &sh.st, sh.tail, sh.ess_bound);
-        if (tape.aux && keeper)
-          tape.aux[tick] = sh.tail.degenerate ? make_float2(0.0f, __int_as_float(0))
-                                              : make_float2((float)(1.0 / tS), __int_as_float(nM));
+        // plan_decide's test, ESS = fl(fl(tS tS) / tQ) < ess_bound, without the division away from the
+        // bound (2^-48 covers the quotient's and the product's roundings)
+        const bool degenerate = (nM == kNkEmpty) || !(tS > 0.0);
+        int resample = 0;
+        if (!degenerate) {
+          const double ss = tS * tS, lim = sh.ess_bound * tQ;
+          resample = ahead || (ss < lim * (1.0 - 0x1p-48) ? true : (ss > lim * (1.0 + 0x1p-48) ? false : ss / tQ < sh.ess_bound));
+        }
+        sh.resample = resample;
+        sh.degenerate = degenerate ? 1 : 0;
       }
       __syncwarp();
     }
@@ -445,7 +496,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
     pending_rec = t;
     prev_stage = stage;
     if (!ahead) __syncthreads();
-    if (ahead || sh.st.do_resample) {
+    if (ahead || sh.resample) {
       // exact fixed-point masses: the tiles' in the global frame, and the own tiles' chunks of CH slots
 #pragma unroll
       for (int u = 0; u < MAXP; ++u) {
@@ -455,7 +506,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
         rE[u] = (rn[u] != kNkEmpty) ? shr64(rE[u], nM - rn[u] + kFixF - Fg) : 0ull;
         const unsigned long long incl = warp_incl_scan_add(rE[u], lane);
         if (lane == 31) sh.wE[pw] = incl;
-        if (k >= first && k < first + nth) sh.pre[k - first] = incl - rE[u];
+        if (k >= first && k < first + nth) { sh.pre[k - first] = incl - rE[u]; sh.mass[k - first] = rE[u]; }
         rE[u] = incl;                              // the prefix through tile k from here on
       }
       unsigned long long loc[Q];
@@ -467,7 +518,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
         unsigned long long e = 0ull;
 #pragma unroll
         for (int g = 0; g < CH / 4; ++g) {
-          const float4 d4 = *reinterpret_cast<const float4*>(sh.w[j] + CH * gt + 4 * g);
+          const float4 d4 = ld4(sh.w[j], CH * gt + 4 * g);
           e += fix_weight(tile_weight(d4.x)) + fix_weight(tile_weight(d4.y));
           e += fix_weight(tile_weight(d4.z)) + fix_weight(tile_weight(d4.w));
         }
@@ -476,32 +527,59 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
         loc[q] = incl - e;
       }
       __syncthreads();
-      if (sh.st.do_resample) {
-        // the targets, and the own tiles' prefixes (every warp forms the totals; warp 0 the rest)
+      if (sh.resample) {
+        // The targets and the own tiles' prefixes by warp 0; the others load their first chunk and clear
+        // the marks meanwhile.
         const unsigned long long we = lane < nwp ? sh.wE[lane] : 0ull;
         const unsigned long long winc = warp_incl_scan_add(we, lane);
         if (warp == 0) {
           const unsigned long long total = __shfl_sync(0xffffffffu, winc, 31);
-          const int mine = first + min(lane, nth - 1);
-          const unsigned long long before = __shfl_sync(0xffffffffu, winc - we, mine >> 5);
-          if (lane < nth) sh.P[lane] = sh.pre[lane] + before;
           unsigned long long delta = udiv_fp64_rcp(total, (unsigned long long)N, rcpN);
           const bool zero_spacing = delta == 0ull;
           if (zero_spacing) delta = 1ull;
-          const unsigned long long u = sh.st.u23;
+          const unsigned long long old = sh.ustate;
+          const unsigned long long u = pcg_output(old) >> 9;       // the tick's resampling uniform
           const unsigned long long hi = __umul64hi(u, delta), lo = u * delta;
+          const unsigned long long base = (hi << 41) | (lo >> 23);   // floor(u * delta / 2^23)
+          const unsigned long long magic = udiv_magic_of(delta);
+          const int jm = min(lane >> 1, nth - 1);      // lanes 2 j and 2 j + 1: own tile j's first output and its end
+          const unsigned long long before = __shfl_sync(0xffffffffu, winc - we, (first + jm) >> 5);
+          const unsigned long long Pj = sh.pre[jm] + before;
+          const int c = targets_below((lane & 1) ? Pj + sh.mass[jm] : Pj, base, delta, magic, N);
+          if (lane < 2 * nth) {
+            if (lane & 1) sh.c1[jm] = c;
+            else { sh.c0[jm] = c; sh.P[jm] = Pj; }
+          }
+          __syncwarp();
           if (lane == 0) {
+            sh.ustate = old * kPcgMult + kHostInc;
+            sh.base = base; sh.delta = delta; sh.magic = magic;
             DevState& st = sh.st;
-            sh.base = (hi << 41) | (lo >> 23);       // floor(u * delta / 2^23)
-            sh.delta = delta;
-            sh.magic = udiv_magic_of(delta);
             if (zero_spacing) st.error = BPF_ERR_DEGENERATE;
-            st.base = sh.base; st.delta = delta; st.delta_magic = sh.magic; st.total = total; st.Fg = Fg;
+            st.base = base; st.delta = delta; st.delta_magic = magic; st.total = total; st.Fg = Fg;
           }
         }
+        ChunkTargets<CH> ct;
+        unsigned short* mk = sh.marks[grp];
+        unsigned long long chunk_loc = 0ull;
+        auto load_chunk = [&](int j, unsigned long long lq) {
+          ct.c = gt;
+          ct.lfT = 0.0f;
+#pragma unroll
+          for (int g = 0; g < CH / 4; ++g) {
+            const float4 d4 = ld4(sh.w[j], CH * gt + 4 * g);
+            ct.wf[4 * g] = tile_weight(d4.x); ct.wf[4 * g + 1] = tile_weight(d4.y);
+            ct.wf[4 * g + 2] = tile_weight(d4.z); ct.wf[4 * g + 3] = tile_weight(d4.w);
+          }
+#pragma unroll
+          for (int e = 0; e < CH; ++e) ct.lfT += ct.wf[e];
+          chunk_loc = lq + warp_sum_u64(lane < gw ? sh.wscan[j][lane] : 0ull);   // its prefix within the tile
+          for (int i = gt; i < WSLOTS / 8; i += kThreads * SPLIT) reinterpret_cast<uint4*>(mk)[i] = make_uint4(0u, 0u, 0u, 0u);
+        };
+        if (grp < nth) load_chunk(grp, loc[0]);
         __syncthreads();
         const unsigned long long base = sh.base, delta = sh.delta, magic = sh.magic;
-        float* hdst = cur0 ? p.h0 : p.h1;
+        float* hdst = cur ? p.h0 : p.h1;
         const int slot_lo = first * kTile, slot_hi = (first + nth) * kTile;
         // which CTAs write children into this CTA's slots: bit u, tile 32 (warp + u kResWarps) + lane
         unsigned need = 0u;
@@ -520,28 +598,17 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
         for (int q = 0; q < Q; ++q) {
           const int j = grp + NG * q;
           if (j >= nth) continue;                    // whole groups
-          const unsigned long long off = warp_sum_u64(lane < gw ? sh.wscan[j][lane] : 0ull);
+          if (q > 0) {
+            load_chunk(j, loc[q]);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");   // marks cleared
+          }
           const int tk = sh.nexp[j];
           const int r = (tk == kNkEmpty) ? 64 : nM - tk + kFixF - Fg;
-          const int j0 = (first + j) * kTile + CH * gt;
-          const float* d = sh.w[j] + CH * gt;
-          ChunkTargets<CH> ct;
-          ct.c = gt;
-          ct.lfT = 0.0f;
-          float hv[CH];
-#pragma unroll
-          for (int g = 0; g < CH / 4; ++g) {
-            const float4 d4 = *reinterpret_cast<const float4*>(d + 4 * g);
-            const float4 h4 = *reinterpret_cast<const float4*>(sh.h[j] + CH * gt + 4 * g);
-            ct.wf[4 * g] = tile_weight(d4.x); ct.wf[4 * g + 1] = tile_weight(d4.y);
-            ct.wf[4 * g + 2] = tile_weight(d4.z); ct.wf[4 * g + 3] = tile_weight(d4.w);
-            hv[4 * g] = h4.x; hv[4 * g + 1] = h4.y; hv[4 * g + 2] = h4.z; hv[4 * g + 3] = h4.w;
-          }
-#pragma unroll
-          for (int e = 0; e < CH; ++e) ct.lfT += ct.wf[e];
-          chunk_thresholds<CH>(N, off + loc[q], sh.P[j], r, j0 < N, base, delta, magic, ct);
+          const int own = (first + j) * kTile;
+          const int j0 = own + CH * gt;
+          chunk_thresholds<CH>(N, chunk_loc, sh.P[j], r, j0 < N, base, delta, magic, ct);
           int qe[CH];
-          chunk_child_ends<CH>(N, ct, d, qe);
+          chunk_child_ends<CH>(N, ct, qe, [&](int upto) { return exact_count_swz(sh.w[j], CH * gt, upto, ct.th, ct.D, N); });
           if (tape.csr) {                            // first child of each parent
             int32_t* cs = tape.csr + (size_t)tick * tape.csr_stride + j0;
 #pragma unroll
@@ -556,52 +623,116 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
               }
             }
           }
-          // Every thread of the group holds its particles in registers, so the tile's shared-memory
-          // copy takes the children that fall into its own slots; the others go to the other
-          // particle buffer, for the CTA that owns them.
-          asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");
-          const int own = (first + j) * kTile;
-          float* hown = sh.h[j];
-          auto put = [&](int o, float hc, int anc) {
-            if ((unsigned)(o - own) < (unsigned)kTile) hown[o - own] = hc;
-            else hdst[o] = hc;
-            if (a.anc) a.anc[o] = anc;
-          };
-          int qp = ct.q;
+          // start marks (slot of a parent's first child: its index in the tile + 1) in the window
+          const int c0 = sh.c0[j], c1 = sh.c1[j];
+          const int wb = c0 & ~3, we1 = min(c1, wb + WSLOTS);   // window [wb, we1)
 #pragma unroll
           for (int e = 0; e < CH; ++e) {
-            const int q1 = qe[e];
-            if (q1 - qp <= kResHeavy)
-              for (int o = qp; o < q1; ++o) put(o, hv[e], j0 + e);
-            qp = q1;
+            const int b0 = e ? qe[e - 1] : ct.q;
+            if (qe[e] > b0 && b0 < we1) mk[b0 - wb] = (unsigned short)(CH * gt + e + 1);
           }
-          // long runs are shared by the warp
-          bool any_heavy = false;
+          if (c1 > we1) {                            // a tile of many children: the rest one by one
+            auto put = [&](int o, float hc, int anc) {
+              hdst[o] = hc;
+              if (a.anc) a.anc[o] = anc;
+            };
+            float hv[CH];
 #pragma unroll
-          for (int e = 0; e < CH; ++e) any_heavy |= qe[e] - (e ? qe[e - 1] : ct.q) > kResHeavy;
-          if (__any_sync(0xffffffffu, any_heavy)) {
+            for (int g = 0; g < CH / 4; ++g) {
+              const float4 h4 = ld4(sh.h[j], CH * gt + 4 * g);
+              hv[4 * g] = h4.x; hv[4 * g + 1] = h4.y; hv[4 * g + 2] = h4.z; hv[4 * g + 3] = h4.w;
+            }
 #pragma unroll
             for (int e = 0; e < CH; ++e) {
-              const int b0 = e ? qe[e - 1] : ct.q, b1 = qe[e];
+              const int b0 = max(e ? qe[e - 1] : ct.q, we1), b1 = qe[e];
+              if (b1 - b0 <= kResHeavy)
+                for (int o = b0; o < b1; ++o) put(o, hv[e], j0 + e);
               unsigned heavy = __ballot_sync(0xffffffffu, b1 - b0 > kResHeavy);
-              while (heavy) {
+              while (heavy) {                        // long runs are shared by the warp
                 const int src = __ffs(heavy) - 1;
                 heavy &= heavy - 1u;
-                const int c0 = __shfl_sync(0xffffffffu, b0, src), c1 = __shfl_sync(0xffffffffu, b1, src);
+                const int h0 = __shfl_sync(0xffffffffu, b0, src), h1 = __shfl_sync(0xffffffffu, b1, src);
                 const float hc = __shfl_sync(0xffffffffu, hv[e], src);
                 const int an = __shfl_sync(0xffffffffu, j0 + e, src);
-                for (int o = c0 + lane; o < c1; o += 32) put(o, hc, an);
+                for (int o = h0 + lane; o < h1; o += 32) put(o, hc, an);
               }
             }
           }
-          // slots of this tile that its own children do not fill are loaded after the flags
+          asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");   // marks set
+          // Gather: the ancestor of window slot o is the last mark at or before o. Each warp takes a run
+          // of slots in steps of 128 (4 per lane); the running maximum of the marks is a lane-local scan,
+          // a warp max-scan and a carry from the earlier steps and warps.
+          const int nB = we1 - wb;
+          const int run = ((nB + GW - 1) / GW + 127) & ~127;
+          const int rs = gw * run, re = min(rs + run, nB);
+          uint2 mv[STEPS];
+          unsigned wm = 0u;
+#pragma unroll
+          for (int x = 0; x < STEPS; ++x) {
+            mv[x] = make_uint2(0u, 0u);
+            if (rs + 128 * x < re) mv[x] = reinterpret_cast<const uint2*>(mk + rs + 128 * x)[lane];
+            const unsigned m2 = __vmaxu2(mv[x].x, mv[x].y);
+            wm = max(wm, max(m2 & 0xffffu, m2 >> 16));
+          }
+          wm = __reduce_max_sync(0xffffffffu, wm);
+          if (lane == 0) sh.wmax[warp] = wm;
+          asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");
+          unsigned last = __reduce_max_sync(0xffffffffu, lane < gw ? sh.wmax[grp * GW + lane] : 0u);
+          float4 out[STEPS];
+#pragma unroll
+          for (int x = 0; x < STEPS; ++x) {
+            out[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (rs + 128 * x >= re) continue;
+            unsigned am[4];
+            am[0] = mv[x].x & 0xffffu;
+            am[1] = max(am[0], mv[x].x >> 16);
+            am[2] = max(am[1], mv[x].y & 0xffffu);
+            am[3] = max(am[2], mv[x].y >> 16);
+            unsigned sc = am[3];
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+              const unsigned o = __shfl_up_sync(0xffffffffu, sc, off);
+              if (lane >= off) sc = max(sc, o);
+            }
+            unsigned pr = __shfl_up_sync(0xffffffffu, sc, 1);
+            pr = max(last, lane == 0 ? 0u : pr);
+            last = max(last, __shfl_sync(0xffffffffu, sc, 31));
+            float hv[4];
+            const int o = wb + rs + 128 * x + 4 * lane;          // first of the lane's four slots
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const unsigned jj = max(pr, am[e]);                // 0 before the tile's first child (slot < c0)
+              const int src = jj ? (int)jj - 1 : 0;
+              hv[e] = el(sh.h[j], src);
+              if (a.anc && o + e >= c0 && o + e < we1) a.anc[o + e] = own + src;
+            }
+            out[x] = make_float4(hv[0], hv[1], hv[2], hv[3]);
+            if ((unsigned)(o - own) >= (unsigned)kTile) {        // another tile's slots: to its owner
+              if (o >= c0 && o + 4 <= we1) {
+                *reinterpret_cast<float4*>(hdst + o) = out[x];
+              } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) if (o + e >= c0 && o + e < we1) hdst[o + e] = hv[e];
+              }
+            }
+          }
+          asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");   // every parent read
+#pragma unroll
+          for (int x = 0; x < STEPS; ++x) {
+            const int o = wb + rs + 128 * x + 4 * lane;
+            if (rs + 128 * x >= re || (unsigned)(o - own) >= (unsigned)kTile) continue;
+            if (o >= c0 && o + 4 <= we1) {
+              st4(sh.h[j], o - own, out[x]);
+            } else {
+              const float hv[4] = {out[x].x, out[x].y, out[x].z, out[x].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) if (o + e >= c0 && o + e < we1) el(sh.h[j], o + e - own) = hv[e];
+            }
+          }
         }
         // every CTA whose children fall into this CTA's slots has written them before they are read
         __syncthreads();
-        if (tid < kMail) {
-          __threadfence();
-          st_release_u32(reinterpret_cast<unsigned*>(p.xbuf + kXHeader + tid * mail_size) + blockIdx.x, xno);
-        }
+        if (tid < kMail) st_release_u32(reinterpret_cast<unsigned*>(p.xbuf + kXHeader + tid * mail_size) + blockIdx.x, xno);
 #pragma unroll
         for (int u = 0; u < MAXP; ++u) {
           const bool wait = (need & (1u << u)) != 0u;
@@ -613,21 +744,16 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
             if (__all_sync(0xffffffffu, ok)) break;
             if (!pt.more(xw + 1, epoch + 1u)) { bad = true; break; }
           }
-          __threadfence();                        // acquire (a relaxed poll leaves L1 alone)
+          asm volatile("fence.acq_rel.gpu;" ::: "memory");   // acquire (a relaxed poll leaves L1 alone)
         }
         if (__syncthreads_or(bad)) { failed = true; break; }
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
           const int j = grp + NG * q;
           if (j >= nth) continue;
-          // the tile's own children fill the slots [c0, c1) of it
+          // the slots that the tile's own window did not fill
           const int own = (first + j) * kTile;
-          const int tk = sh.nexp[j];
-          const int r = (tk == kNkEmpty) ? 64 : nM - tk + kFixF - Fg;
-          unsigned long long mass = 0ull;
-          for (int w = 0; w < GW; ++w) mass += sh.wscan[j][w];
-          const int c0 = targets_below(sh.P[j], base, delta, magic, N) - own;
-          const int c1 = targets_below(sh.P[j] + shr64(mass, r), base, delta, magic, N) - own;
+          const int c0 = sh.c0[j] - own, c1 = min(sh.c1[j], (sh.c0[j] & ~3) + WSLOTS) - own;
 #pragma unroll
           for (int rr = 0; rr < R; ++rr) {
             const int l0 = l_first + 4 * kThreads * rr;
@@ -636,11 +762,18 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
             const float hv[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              if (l0 + e < c0 || l0 + e >= c1) sh.h[j][l0 + e] = hv[e];
+              if (l0 + e < c0 || l0 + e >= c1) el(sh.h[j], l0 + e) = hv[e];
           }
         }
+        cur ^= 1;
+        carry = false;
       }
     }
+    if (!sh.resample) {
+      carry = sh.degenerate == 0;
+      if (carry) nM_prev = nM;
+    }
+    if (!APF || stage != 1) ++tick;
     if (APF && stage == 1) {
       stage = 2;
     } else {
@@ -649,7 +782,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
     }
   }
 
-  if (tid == kResThreads - 32 && pending && keeper && !failed) finish(prev_stage, pending_rec);
+  if (tid == kDecider && pending && keeper && !failed) settle(prev_stage, pending_rec);
   __syncthreads();
   if (failed && tid == 0) st_release_u32(xw + 1, epoch + 1u);   // the other CTAs stop waiting
   if (!failed) {
@@ -658,12 +791,12 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       const int j = grp + NG * q;
       if (j >= nth) continue;
       const size_t off = (size_t)(first + j) * kTile;
-      float* hg = (sh.st.cur ? p.h1 : p.h0) + off;
+      float* hg = (cur ? p.h1 : p.h0) + off;
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
         const int l0 = l_first + 4 * kThreads * rr;
-        *reinterpret_cast<float4*>(hg + l0) = *reinterpret_cast<const float4*>(sh.h[j] + l0);
-        *reinterpret_cast<float4*>(p.w + off + l0) = *reinterpret_cast<const float4*>(sh.w[j] + l0);
+        *reinterpret_cast<float4*>(hg + l0) = ld4(sh.h[j], l0);
+        *reinterpret_cast<float4*>(p.w + off + l0) = ld4(sh.w[j], l0);
       }
       if (gt == 0) p.nexp[first + j] = nk[q];
     }
@@ -688,7 +821,7 @@ using ResidentKernel = void (*)(Plan, TickArgs, ResidentTape, int, int);
 
 template <bool APF, int SPLIT, int Q>
 ResidentKernel pick_model(bool tstate, bool gauss, size_t* smem) {
-  *smem = sizeof(ResidentShared<kResThreads / (kThreads * SPLIT) * Q>);
+  *smem = sizeof(ResidentShared<kResThreads / (kThreads * SPLIT) * Q, SPLIT>);
   if (tstate) return gauss ? resident_kernel<true, true, APF, SPLIT, Q> : resident_kernel<true, false, APF, SPLIT, Q>;
   return gauss ? resident_kernel<false, true, APF, SPLIT, Q> : resident_kernel<false, false, APF, SPLIT, Q>;
 }

@@ -35,17 +35,15 @@ struct FusedTail {
 // The tick's decision from its statistics, by one thread: plan_decide's operations on the device-state
 // fields that the next tick and the resampling read, in its order; the rest is left to fused_finish
 // in tl. APF as TickArgs::apf (the first stage of an auxiliary-filter tick does not advance the tick).
-// keep_bound: the smallest ESS x whose quotient x / N is not below the threshold (< 0: divide).
 template <int APF = 0>
 __device__ __forceinline__ void fused_decide(const TickArgs& a, int N, int nM, double tS, double tQ, double tH,
-                                             DevState* st, FusedTail& tl, double keep_bound = -1.0) {
+                                             DevState* st, FusedTail& tl) {
   const bool degenerate = (nM == kNkEmpty) || !(tS > 0.0);
   double ess = 0.0;
   int resample = 0;
   if (!degenerate) {
     ess = tS * tS / tQ;
-    resample = (a.ess_threshold <= 0.0f) ||
-               (keep_bound >= 0.0 ? ess < keep_bound : ess / (double)N < (double)a.ess_threshold);
+    resample = (a.ess_threshold <= 0.0f) || (ess / (double)N < (double)a.ess_threshold);
   }
   tl.tS = tS; tl.tH = tH; tl.ess = ess; tl.nM = nM;
   tl.degenerate = degenerate ? 1 : 0; tl.resample = resample;
@@ -138,10 +136,10 @@ __device__ __forceinline__ void chunk_thresholds(int N, unsigned long long loc, 
 // The end of each element's children (output slots [q_{j-1}, q_j), q_{-1} = ct.q): the running count
 // c_j = #{m >= 0 : th + m D <= l_j} (l_j the exact fixed-point sum of the chunk's weights up to j)
 // estimated in FP32 with pass 2's bound on the estimate's error taken at the chunk's largest sum; near
-// a target boundary (one vote per four elements) the element recounts in exact 64-bit integers from
-// its log2-weights d. Whole warps only.
-template <int CH>
-__device__ __forceinline__ void chunk_child_ends(int N, const ChunkTargets<CH>& ct, const float* d, int qe[CH]) {
+// a target boundary (one vote per four elements) element i recounts in exact 64-bit integers,
+// recount(i) = exact_count of its log2-weights. Whole warps only.
+template <int CH, class F>
+__device__ __forceinline__ void chunk_child_ends(int N, const ChunkTargets<CH>& ct, int qe[CH], F recount) {
   const unsigned long long R0 = ct.th, D = ct.D;
   const bool none = R0 >= kThCap;
   const float R0w = (float)R0 * 0x1p-50f;
@@ -171,7 +169,7 @@ __device__ __forceinline__ void chunk_child_ends(int N, const ChunkTargets<CH>& 
     if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (rc[e]) qq[e] = min(q0 + exact_count(d, 4 * g + e, R0, D, N), N);
+        if (rc[e]) qq[e] = min(q0 + recount(4 * g + e), N);
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) qe[4 * g + e] = qq[e];
