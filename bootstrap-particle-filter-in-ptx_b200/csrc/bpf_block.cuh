@@ -145,6 +145,18 @@ __device__ int block_max_i(int v, int* sh) {
   return m;
 }
 
+// For marks that increase over the set ones (0 = none), one per lane: the last set mark of the lanes
+// before this one (else `last`), and of the whole warp (else `last`): a vote and two shuffles in place
+// of a max-scan.
+__device__ __forceinline__ void marks_before(unsigned m, int lane, unsigned last, unsigned& before, unsigned& all) {
+  const unsigned set = __ballot_sync(0xffffffffu, m != 0u);
+  const unsigned lower = set & ((1u << lane) - 1u);
+  const unsigned b = __shfl_sync(0xffffffffu, m, lower ? 31 - __clz((int)lower) : 0);
+  const unsigned e = __shfl_sync(0xffffffffu, m, set ? 31 - __clz((int)set) : 0);
+  before = lower ? b : last;
+  all = set ? e : last;
+}
+
 // 2^e as a double (exact IEEE encoding; 0 below the normal range).
 __device__ __forceinline__ double pow2d(int e) {
   if (e < -1022) return 0.0;

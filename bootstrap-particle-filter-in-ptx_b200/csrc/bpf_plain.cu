@@ -18,7 +18,7 @@
 //   pass 2  (persistent CTAs over work items: one tile, a run of outputs)
 //           systematic resampling: exact integer prefix of the tile weights,
 //           each element counts the evenly spaced targets it owns and marks
-//           the first of them, a warp max-scan over the marks gives every
+//           the first of them, a warp scan over the marks gives every
 //           output its ancestor, gather of h[ancestor] from a bulk-async
 //           (TMA) copy of the tile, 16-byte vector stores. Four CTAs per SM,
 //           each staging one item's tiles at a time (the next item's copy is
@@ -866,8 +866,8 @@ __global__ void __launch_bounds__(kThreads, 4) pass2_kernel(Plan p, TickArgs a) 
     // Gather: the ancestor of window slot o is the last start mark at or
     // before o (marks increase along the window). Each warp takes a run of
     // slots in steps of 256 (8 per lane): the running maximum of the marks
-    // is a lane-local scan, a warp max-scan and a carry from the earlier
-    // steps and warps. A lane's 8 slots are 16-byte aligned in the output,
+    // is a lane-local scan, the last marked lane before and a carry from
+    // the earlier steps and warps. A lane's 8 slots are 16-byte aligned in the output,
     // so whole groups are written with two vector stores; every slot from
     // the item's first one on has a mark at or before it, so a group that
     // lies inside the item needs no per-slot test.
@@ -897,14 +897,8 @@ __global__ void __launch_bounds__(kThreads, 4) pass2_kernel(Plan p, TickArgs a) 
         am[5] = max(am[4], m.z >> 16);
         am[6] = max(am[5], m.w & 0xffffu);
         am[7] = max(am[6], m.w >> 16);
-        unsigned x = am[7];
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const unsigned t = __shfl_up_sync(0xffffffffu, x, off);
-          if (lane >= off) x = max(x, t);
-        }
-        unsigned pre = __shfl_up_sync(0xffffffffu, x, 1);
-        pre = max(carry, lane == 0 ? 0u : pre);
+        unsigned pre, next_carry;
+        marks_before(am[7], lane, carry, pre, next_carry);
         const int o = o0 + 8 * lane;
         if (o >= olo && o + 7 < ce) {
 #pragma unroll
@@ -934,7 +928,7 @@ __global__ void __launch_bounds__(kThreads, 4) pass2_kernel(Plan p, TickArgs a) 
             }
           }
         }
-        carry = max(carry, __shfl_sync(0xffffffffu, x, 31));
+        carry = next_carry;
       }
     }
     __syncthreads();   // the staged tile is free: fetch the next item's

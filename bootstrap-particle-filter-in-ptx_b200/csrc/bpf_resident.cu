@@ -205,8 +205,8 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
     }
   }
   // state noise of this thread's particles for the tick with stream constants (k1, k2): read again
-  // only by this thread
-  auto noise = [&](uint64_t k1, uint64_t k2) {
+  // only by this thread; half 0 and 1: the first and second half of its groups, 2: all
+  auto noise = [&](uint64_t k1, uint64_t k2, int half) {
     const uint64_t k33 = k2 << 33, step2 = 2ull * k2, step_r = (uint64_t)(2 * 4 * kThreads - 8) * k2;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -215,8 +215,8 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       uint64_t sx = k1 + k2 * pcg_inc((uint32_t)((first + j) * kTile + l_first));
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
+        if (half == (rr < R / 2 ? 1 : 0)) { sx += 4ull * step2 + step_r; continue; }
         float zz[4];
-        if (rr > 0) sx += step_r;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           float z = icdf_normal_warp(pcg_uniform(pcg_output(sx)));
@@ -224,12 +224,13 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
           zz[e] = z;
           sx += step2;
         }
+        sx += step_r;
         *reinterpret_cast<float4*>(sh.z[j] + l_first + 4 * kThreads * rr) = make_float4(zz[0], zz[1], zz[2], zz[3]);
       }
     }
   };
   uint64_t k1 = sh.st.k1, k2 = sh.st.k2;        // stream constants of the next tick (all threads)
-  if (!APF && sh.st.tick > 0) noise(k1, k2);
+  if (!APF && sh.st.tick > 0) noise(k1, k2, 2);
 
   // what every thread follows of the device state; the keeper's copy is brought up to date (and the
   // record written) during the next exchange, from the sums its decision left with thread kDecider
@@ -416,11 +417,23 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
 
     // ---- while the records travel: the next noise, and the keeper's state and record of the last tick ----
     if (!APF || stage != 1) { k1 = k1 * kPcgMult; k2 = k2 * kPcgMult + 1ull; }
-    if (APF ? stage == 1 : t + 1 < n_ticks) noise(k1, k2);
+    const bool make_noise = APF ? stage == 1 : t + 1 < n_ticks;
+    if (make_noise) noise(k1, k2, Q == 1 ? 0 : 2);
     if (keeper && pending && tid == kDecider) settle(prev_stage, pending_rec);
 
     // ---- exchange: lane l of the warp of 32 tiles takes its tile's record ----
+    // (with little noise to form, the first look is issued before its second half: 3% of a tick)
     constexpr int MAXP = (kResMaxTiles + kResThreads - 1) / kResThreads;   // records a thread may take
+    auto slot_of = [&](int u) {
+      const int k = 32 * (warp + u * kResWarps) + lane;
+      return mail + mail_flag_bytes(G) + ((size_t)(xn & 1u) * G + min(k, G - 1)) * 32;
+    };
+    unsigned long long a0 = 0ull, a1 = 0ull, b0 = 0ull, b1 = 0ull;
+    if (warp < nwp) {
+      ld_relaxed_b128(slot_of(0), a0, a1);
+      ld_relaxed_b128(slot_of(0) + 16, b0, b1);
+    }
+    if (Q == 1 && make_noise) noise(k1, k2, 1);
     int rn[MAXP];
     unsigned long long rE[MAXP];
     bool bad = false;
@@ -433,15 +446,15 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       const int k = 32 * pw + lane;
       // The loop leaves by a warp vote: a lane that left alone would keep the warp split through the
       // shuffles below (measured 3.5 us for the sums after a spin, 0.13 us together).
-      const unsigned char* slot = mail + mail_flag_bytes(G) + ((size_t)(xn & 1u) * G + min(k, G - 1)) * 32;
-      unsigned long long a0 = 0ull, a1 = 0ull, b0 = 0ull, b1 = 0ull;
+      const unsigned char* slot = slot_of(u);
+      if (u > 0) { ld_relaxed_b128(slot, a0, a1); ld_relaxed_b128(slot + 16, b0, b1); }
       Patience pt;
       for (;;) {
-        ld_relaxed_b128(slot, a0, a1);
-        ld_relaxed_b128(slot + 16, b0, b1);
         const bool ok = (unsigned)(a1 >> 32) == xno && (unsigned)(b1 >> 32) == xno;
         if (__all_sync(0xffffffffu, ok)) break;
         if (!pt.more(xw + 1, epoch + 1u)) { bad = true; break; }     // the same in every lane
+        ld_relaxed_b128(slot, a0, a1);
+        ld_relaxed_b128(slot + 16, b0, b1);
       }
       float rS = 0.f, rQ = 0.f, rH = 0.f;
       if (k < G && !bad) {
@@ -580,20 +593,6 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
         __syncthreads();
         const unsigned long long base = sh.base, delta = sh.delta, magic = sh.magic;
         float* hdst = cur ? p.h0 : p.h1;
-        const int slot_lo = first * kTile, slot_hi = (first + nth) * kTile;
-        // which CTAs write children into this CTA's slots: bit u, tile 32 (warp + u kResWarps) + lane
-        unsigned need = 0u;
-#pragma unroll
-        for (int u = 0; u < MAXP; ++u) {
-          const int pw = warp + u * kResWarps;
-          if (pw >= nwp) continue;
-          const int k = 32 * pw + lane;
-          const unsigned long long before = __shfl_sync(0xffffffffu, winc - we, pw);
-          const int o1 = targets_below(before + rE[u], base, delta, magic, N);
-          int o0 = __shfl_up_sync(0xffffffffu, o1, 1);
-          if (lane == 0) o0 = targets_below(before, base, delta, magic, N);
-          if (k < G && o1 > o0 && o0 < slot_hi && o1 > slot_lo && (k < first || k >= first + nth)) need |= 1u << u;
-        }
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
           const int j = grp + NG * q;
@@ -661,7 +660,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
           asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kThreads * SPLIT) : "memory");   // marks set
           // Gather: the ancestor of window slot o is the last mark at or before o. Each warp takes a run
           // of slots in steps of 128 (4 per lane); the running maximum of the marks is a lane-local scan,
-          // a warp max-scan and a carry from the earlier steps and warps.
+          // the last marked lane before and a carry from the earlier steps and warps.
           const int nB = we1 - wb;
           const int run = ((nB + GW - 1) / GW + 127) & ~127;
           const int rs = gw * run, re = min(rs + run, nB);
@@ -688,15 +687,9 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
             am[1] = max(am[0], mv[x].x >> 16);
             am[2] = max(am[1], mv[x].y & 0xffffu);
             am[3] = max(am[2], mv[x].y >> 16);
-            unsigned sc = am[3];
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-              const unsigned o = __shfl_up_sync(0xffffffffu, sc, off);
-              if (lane >= off) sc = max(sc, o);
-            }
-            unsigned pr = __shfl_up_sync(0xffffffffu, sc, 1);
-            pr = max(last, lane == 0 ? 0u : pr);
-            last = max(last, __shfl_sync(0xffffffffu, sc, 31));
+            unsigned pr, next_last;
+            marks_before(am[3], lane, last, pr, next_last);
+            last = next_last;
             float hv[4];
             const int o = wb + rs + 128 * x + 4 * lane;          // first of the lane's four slots
 #pragma unroll
@@ -733,6 +726,20 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
         // every CTA whose children fall into this CTA's slots has written them before they are read
         __syncthreads();
         if (tid < kMail) st_release_u32(reinterpret_cast<unsigned*>(p.xbuf + kXHeader + tid * mail_size) + blockIdx.x, xno);
+        const int slot_lo = first * kTile, slot_hi = (first + nth) * kTile;
+        // which CTAs write children into this CTA's slots: bit u, tile 32 (warp + u kResWarps) + lane
+        unsigned need = 0u;
+#pragma unroll
+        for (int u = 0; u < MAXP; ++u) {
+          const int pw = warp + u * kResWarps;
+          if (pw >= nwp) continue;
+          const int k = 32 * pw + lane;
+          const unsigned long long before = __shfl_sync(0xffffffffu, winc - we, pw);
+          const int o1 = targets_below(before + rE[u], base, delta, magic, N);
+          int o0 = __shfl_up_sync(0xffffffffu, o1, 1);
+          if (lane == 0) o0 = targets_below(before, base, delta, magic, N);
+          if (k < G && o1 > o0 && o0 < slot_hi && o1 > slot_lo && (k < first || k >= first + nth)) need |= 1u << u;
+        }
 #pragma unroll
         for (int u = 0; u < MAXP; ++u) {
           const bool wait = (need & (1u << u)) != 0u;

@@ -91,3 +91,20 @@ def test_resident_degenerate_tick(bpf):
     a = _device_run(bpf, 80000, 0.5, 0.0, 0.0, y, True, (17,))
     b = _device_run(bpf, 80000, 0.5, 0.0, 0.0, y, False, (17,))
     assert a == b
+
+
+@pytest.mark.parametrize("N,nu_obs,nu_state,outliers", [
+    (1, 0.0, 0.0, False), (4097, 5.0, 0.0, True), (50000, 0.0, 0.0, False), (148 * TILE + 1, 0.0, 5.0, True),
+    (1500000, 5.0, 0.0, False)])
+def test_resident_apf_matches_kernel_launches(bpf, N, nu_obs, nu_state, outliers):
+    """Auxiliary-filter runs: a filter that records its ancestors keeps the launch per kernel."""
+    y = _series(70, 13, outliers).tolist()
+    out = []
+    for record in (False, True):
+        f = bpf.GpuApf(N, RHO, SIG, MU, nu_state, nu_obs, 19)
+        f.record_ancestors(record)
+        recs = f.step_many(y[:66], records=True)
+        recs += f.step_many(y[66:], records=True)
+        out.append(([bytes(r) for r in recs], bytes(f.get_particles()), f.get_loglik_total()))
+        f.close()
+    assert out[0] == out[1]
