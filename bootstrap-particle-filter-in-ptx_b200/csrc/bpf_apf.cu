@@ -33,6 +33,7 @@ using namespace bpf;
 namespace {
 
 constexpr int kApfChunk = 64;   // ticks per captured graph in gpu_apf_step_many
+constexpr int kApfRun = 1024;   // ticks per resident launch there
 
 inline int set_err(int code) { return bpf_record_error(code); }
 
@@ -53,10 +54,10 @@ struct ApfImpl {
   int pass2_grid = 0;
   int res_tiles = 0;                  // largest filter of a resident run on the device (tiles)
   cudaStream_t stream = nullptr;
-  BpfTickRecord* rec_dev = nullptr;   // [1 + kApfChunk]: slot 0 single step, 1.. graph ticks
+  BpfTickRecord* rec_dev = nullptr;   // [1 + kApfRun]: slot 0 single step, 1.. a chunk's ticks
   BpfTickRecord* rec_pin = nullptr;
   DevState* st_pin = nullptr;
-  float* y_dev = nullptr;             // [kApfChunk]
+  float* y_dev = nullptr;             // [kApfRun]
   float* y_pin = nullptr;
   int32_t* anc_dev = nullptr;         // when recording: first stage, then second stage at anc_stride
   bool record_anc = false;
@@ -111,9 +112,7 @@ cudaError_t launch3(ApfImpl* m, const TickArgs& a) {
 // Runs of ticks of a filter that fits on the chip are one resident launch (bpf_resident.cu: both
 // stages of every tick, the same results) instead of six dependent kernels a tick; recorded ancestors
 // are those of single ticks, so recording filters keep the kernels. N = 4096: 31 -> 12 us per tick.
-bool use_resident(const ApfImpl* m, int n_ticks) {
-  return m->plan.G <= m->res_tiles && !m->record_anc && n_ticks > 0;
-}
+bool use_resident(const ApfImpl* m) { return m->plan.G <= m->res_tiles && !m->record_anc; }
 
 // One APF tick (tick index `t` on the host): a bootstrap tick at t = 0, else
 // the two stages. Returns the kernels launched, or -1 on a launch error.
@@ -149,12 +148,12 @@ int create_impl(GpuApfState* s, ApfImpl* m, int seed) {
   ACK(cudaGetDevice(&m->device));
   ACK(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
   ACK(plan_alloc(m->plan, s->n_particles));
-  ACK(bpf_malloc(&m->rec_dev, (1 + kApfChunk) * sizeof(BpfTickRecord)));
-  ACK(bpf_malloc(&m->y_dev, kApfChunk * sizeof(float)));
-  ACK(bpf_malloc_host(&m->rec_pin, (1 + kApfChunk) * sizeof(BpfTickRecord)));
+  ACK(bpf_malloc(&m->rec_dev, (1 + kApfRun) * sizeof(BpfTickRecord)));
+  ACK(bpf_malloc(&m->y_dev, kApfRun * sizeof(float)));
+  ACK(bpf_malloc_host(&m->rec_pin, (1 + kApfRun) * sizeof(BpfTickRecord)));
   ACK(bpf_malloc_host(&m->st_pin, sizeof(DevState)));
-  ACK(bpf_malloc_host(&m->y_pin, kApfChunk * sizeof(float)));
-  ACK(cudaMemsetAsync(m->rec_dev, 0, (1 + kApfChunk) * sizeof(BpfTickRecord), m->stream));
+  ACK(bpf_malloc_host(&m->y_pin, kApfRun * sizeof(float)));
+  ACK(cudaMemsetAsync(m->rec_dev, 0, (1 + kApfRun) * sizeof(BpfTickRecord), m->stream));
   m->pass2_grid = pass2_grid_size(m->device);
   m->res_tiles = resident_max_tiles(m->device);
   if (const char* v = std::getenv("BPF_DISABLE_PDL")) m->pdl = (v[0] == '0');
@@ -262,8 +261,9 @@ int gpu_apf_step_many(GpuApfState* s, const float* y, int n_ticks, BpfResult* ou
   if (rc) return rc;
   int t = 0;
   while (t < n_ticks) {
-    const int n = std::min(kApfChunk, n_ticks - t);
-    if (use_resident(m, n)) {
+    const bool resident = use_resident(m);
+    const int n = std::min(resident ? kApfRun : kApfChunk, n_ticks - t);
+    if (resident) {
       std::memcpy(m->y_pin, y + t, n * sizeof(float));
       ACK(cudaMemcpyAsync(m->y_dev, m->y_pin, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
       TickArgs a = make_args(s, m, 0.0f, m->y_dev);

@@ -42,6 +42,9 @@ void bpf_note_launches(long long n) { g_launches += n; }
 namespace {
 
 constexpr int kGraphChunk = 64;   // ticks per captured graph
+// Ticks per launch of a host run that is one launch a chunk (fused small filters, resident runs): with
+// 64 a synchronise, two copies and the particles' way in and out of the chip cost 0.2-0.9 us per tick.
+constexpr int kRunChunk = 1024;
 
 struct Impl {
   int device = 0;
@@ -50,7 +53,7 @@ struct Impl {
   int pass2_grid = 0;
   cudaStream_t stream = nullptr;
 
-  BpfTickRecord* rec_dev = nullptr;     // [1 + kGraphChunk]: slot 0 single step, 1.. graph ticks
+  BpfTickRecord* rec_dev = nullptr;     // [1 + kRunChunk]: slot 0 single step, 1.. a chunk's ticks
   BpfTickRecord* rec_pin = nullptr;     // pinned mirror
   DevState* st_pin = nullptr;           // pinned DevState snapshot
   // single ticks (gpu_bpf_step / step_async) write their record and outcome straight into
@@ -61,8 +64,8 @@ struct Impl {
   TickMirror* mir_map_dev = nullptr;
   bool last_in_map = false;             // the last enqueued tick wrote rec_map (not rec_dev[0])
   int seq = 0;                          // request number of the last tick that writes the mirror
-  float* y_dev = nullptr;               // [kGraphChunk]
-  float* y_pin = nullptr;               // [kGraphChunk]
+  float* y_dev = nullptr;               // [kRunChunk]
+  float* y_pin = nullptr;               // [kRunChunk]
   int32_t* anc_dev = nullptr;           // [N] when recording
   bool record_anc = false;
   int ll_mode = 0;
@@ -350,15 +353,8 @@ int build_graph(GpuBpfState* s, Impl* m) {
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaMemcpyAsync(m->y_dev, m->y_pin, kGraphChunk * sizeof(float), cudaMemcpyHostToDevice, m->stream);
-  const TickArgs a0 = make_args(s, m, 0.0f, m->y_dev, m->rec_dev + 1);
-  if (err == cudaSuccess && one_launch(m, a0)) {
-    err = launch_run(m, a0, kGraphChunk);                                // the chunk as one launch
-  } else {
-    for (int k = 0; k < kGraphChunk && err == cudaSuccess; ++k) {
-      TickArgs a = make_args(s, m, 0.0f, m->y_dev + k, m->rec_dev + 1 + k);
-      err = launch_tick3(m, a);
-    }
-  }
+  for (int k = 0; k < kGraphChunk && err == cudaSuccess; ++k)
+    err = launch_tick3(m, make_args(s, m, 0.0f, m->y_dev + k, m->rec_dev + 1 + k));
   if (err == cudaSuccess)
     err = cudaMemcpyAsync(m->rec_pin + 1, m->rec_dev + 1, kGraphChunk * sizeof(BpfTickRecord), cudaMemcpyDeviceToHost, m->stream);
   cudaError_t e2 = cudaStreamEndCapture(m->stream, &g);
@@ -489,18 +485,18 @@ static int create_impl(GpuBpfState* s, Impl* m, int n, float rho, float sigma_z,
   Plan& p = m->plan;
   CK(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
   CK(plan_alloc(p, n));
-  CK(bpf_malloc(&m->rec_dev, (1 + kGraphChunk) * sizeof(BpfTickRecord)));
-  CK(bpf_malloc(&m->y_dev, kGraphChunk * sizeof(float)));
-  CK(bpf_malloc_host(&m->rec_pin, (1 + kGraphChunk) * sizeof(BpfTickRecord)));
+  CK(bpf_malloc(&m->rec_dev, (1 + kRunChunk) * sizeof(BpfTickRecord)));
+  CK(bpf_malloc(&m->y_dev, kRunChunk * sizeof(float)));
+  CK(bpf_malloc_host(&m->rec_pin, (1 + kRunChunk) * sizeof(BpfTickRecord)));
   CK(bpf_malloc_host(&m->st_pin, sizeof(DevState)));
-  CK(bpf_malloc_host(&m->y_pin, kGraphChunk * sizeof(float)));
+  CK(bpf_malloc_host(&m->y_pin, kRunChunk * sizeof(float)));
   CK(bpf_host_alloc(&m->rec_map, sizeof(BpfTickRecord), cudaHostAllocMapped));
   CK(bpf_host_alloc(&m->mir_map, sizeof(TickMirror), cudaHostAllocMapped));
   CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&m->rec_map_dev), m->rec_map, 0));
   CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&m->mir_map_dev), m->mir_map, 0));
   std::memset(m->rec_map, 0, sizeof(BpfTickRecord));
   std::memset(m->mir_map, 0, sizeof(TickMirror));
-  CK(cudaMemsetAsync(m->rec_dev, 0, (1 + kGraphChunk) * sizeof(BpfTickRecord), m->stream));
+  CK(cudaMemsetAsync(m->rec_dev, 0, (1 + kRunChunk) * sizeof(BpfTickRecord), m->stream));
   m->pass2_grid = pass2_grid_size(m->device);
   m->small_tiles = small_max_tiles(m->device);
   m->res_tiles = resident_max_tiles(m->device);
@@ -725,20 +721,38 @@ int gpu_bpf_step_many(GpuBpfState* s, const float* y, int n_ticks, BpfResult* ou
   rc = ensure_device(m);
   if (rc) return rc;
   int t = 0;
-  if (!m->profiling && !m->learn_mode) {            // learning updates need the host every K ticks
+  int last = 0;                                     // the last tick's place in its chunk
+  if (one_launch(m, make_args(s, m, 0.0f, m->y_dev, m->rec_dev + 1))) {
+    while (n_ticks - t > 1) {                       // (a single tick has less to load as kernels)
+      const int n = std::min(kRunChunk, n_ticks - t);
+      std::memcpy(m->y_pin, y + t, n * sizeof(float));
+      CK(cudaMemcpyAsync(m->y_dev, m->y_pin, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+      CK(launch_run(m, make_args(s, m, 0.0f, m->y_dev, m->rec_dev + 1), n));
+      CK(cudaMemcpyAsync(m->rec_pin + 1, m->rec_dev + 1, n * sizeof(BpfTickRecord), cudaMemcpyDeviceToHost, m->stream));
+      CK(cudaStreamSynchronize(m->stream));
+      g_launches += 1;
+      m->ticks_enqueued += n;
+      for (int k = 0; k < n; ++k) {
+        if (out) out[t + k] = to_result(m, m->rec_pin[1 + k]);
+        if (rec) rec[t + k] = m->rec_pin[1 + k];
+      }
+      t += n;
+      last = n - 1;
+    }
+  } else if (!m->profiling && !m->learn_mode) {     // learning updates need the host every K ticks
     while (n_ticks - t >= kGraphChunk) {
       if (graph_stale(s, m)) { rc = build_graph(s, m); if (rc) return rc; }
       std::memcpy(m->y_pin, y + t, kGraphChunk * sizeof(float));
       CK(cudaGraphLaunch(m->graph, m->stream));
       CK(cudaStreamSynchronize(m->stream));
-      g_launches += one_launch(m, make_args(s, m, 0.0f, nullptr, nullptr))
-                        ? 1 : (long long)tick_launches(m, make_args(s, m, 0.0f, nullptr, nullptr)) * kGraphChunk;
+      g_launches += (long long)tick_launches(m, make_args(s, m, 0.0f, nullptr, nullptr)) * kGraphChunk;
       m->ticks_enqueued += kGraphChunk;
       for (int k = 0; k < kGraphChunk; ++k) {
         if (out) out[t + k] = to_result(m, m->rec_pin[1 + k]);
         if (rec) rec[t + k] = m->rec_pin[1 + k];
       }
       t += kGraphChunk;
+      last = kGraphChunk - 1;
     }
   }
   // remainder (and the profiled path): direct launches into the same record slots
@@ -755,11 +769,11 @@ int gpu_bpf_step_many(GpuBpfState* s, const float* y, int n_ticks, BpfResult* ou
       if (rec) rec[t + k] = m->rec_pin[1 + k];
     }
     t += n;
+    last = n - 1;
   }
   // keep slot 0 = last tick so get_result/get_record see it
   if (n_ticks > 0) {
     m->last_in_map = false;
-    const int last = (n_ticks - 1) % kGraphChunk;
     const BpfTickRecord& lr = m->rec_pin[1 + last];
     CK(cudaMemcpyAsync(m->rec_dev, m->rec_dev + 1 + last, sizeof(BpfTickRecord), cudaMemcpyDeviceToDevice, m->stream));
     CK(cudaMemcpyAsync(m->st_pin, m->plan.st, sizeof(DevState), cudaMemcpyDeviceToHost, m->stream));

@@ -108,3 +108,28 @@ def test_resident_apf_matches_kernel_launches(bpf, N, nu_obs, nu_state, outliers
         out.append(([bytes(r) for r in recs], bytes(f.get_particles()), f.get_loglik_total()))
         f.close()
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("N", [3, 65537, 700001, 1300000])
+def test_resident_tape_matches_plain_ticks(bpf, N):
+    """Child lists, records and checkpoint-driven gradient inputs of a taped run: the ancestors of single
+    plain ticks (three kernels), bit for bit, outliers included."""
+    import torch
+    T = 12
+    y = _series(T, 31, True)
+    tape = bpf.GradTape(N, T, checkpoint_every=4)
+    ll = tape.forward((MU, RHO, SIG), torch.tensor(y, device="cuda"), seed=8).item()
+    f = bpf.GpuBpf(N, RHO, SIG, MU, seed=8, ess_threshold=0.0)
+    f.set_fused_small(False)
+    f.record_ancestors(True)
+    recs = tape.records()
+    for t in range(T):
+        f.step(float(y[t]))
+        assert bytes(f.get_record()) == bytes(recs[t])
+        np.testing.assert_array_equal(tape.ancestors(t), np.frombuffer(f.get_ancestors()[1], dtype=np.int32))
+    assert ll == f.get_record().loglik_total
+    g = tape.backward().cpu().numpy()
+    ref = tape.replay((MU, RHO, SIG)).cpu().numpy()[1:]
+    assert np.max(np.abs(g - ref)) <= 1e-4 * np.max(np.abs(ref))     # the gradient tests' bound
+    f.close()
+    tape.close()
