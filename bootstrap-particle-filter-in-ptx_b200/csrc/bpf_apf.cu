@@ -112,7 +112,10 @@ cudaError_t launch3(ApfImpl* m, const TickArgs& a) {
 // Runs of ticks of a filter that fits on the chip are one resident launch (bpf_resident.cu: both
 // stages of every tick, the same results) instead of six dependent kernels a tick; recorded ancestors
 // are those of single ticks, so recording filters keep the kernels. N = 4096: 31 -> 12 us per tick.
-bool use_resident(const ApfImpl* m) { return m->plan.G <= m->res_tiles && !m->record_anc; }
+bool use_resident(const GpuApfState* s, const ApfImpl* m) {
+  return m->plan.G <= m->res_tiles && !m->record_anc &&
+         resident_ready(m->device, m->plan.G, m->res_tiles, s->nu_state > 0.0f, !(m->obs.nu > 0.0f), true);
+}
 
 // One APF tick (tick index `t` on the host): a bootstrap tick at t = 0, else
 // the two stages. Returns the kernels launched, or -1 on a launch error.
@@ -261,7 +264,7 @@ int gpu_apf_step_many(GpuApfState* s, const float* y, int n_ticks, BpfResult* ou
   if (rc) return rc;
   int t = 0;
   while (t < n_ticks) {
-    const bool resident = use_resident(m);
+    const bool resident = use_resident(s, m);
     const int n = std::min(resident ? kApfRun : kApfChunk, n_ticks - t);
     if (resident) {
       std::memcpy(m->y_pin, y + t, n * sizeof(float));

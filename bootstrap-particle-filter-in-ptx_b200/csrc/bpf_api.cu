@@ -143,7 +143,8 @@ bool use_small(const Impl* m, const TickArgs& a) {
 // conditions, same results).
 bool use_resident(const Impl* m, const TickArgs& a) {
   return m->fused_small && !m->profiling && !use_small(m, a) && m->plan.G <= m->res_tiles && !a.learn && a.apf == 0 &&
-         !(a.silverman > 0.0f);
+         !(a.silverman > 0.0f) &&
+         resident_ready(m->device, m->plan.G, m->res_tiles, a.nu_int > 0, !(a.obs.nu > 0.0f), false);
 }
 // Whether a run of ticks is one launch, and that launch (a.y_ptr, a.rec: the run's first tick).
 bool one_launch(const Impl* m, const TickArgs& a) { return use_small(m, a) || use_resident(m, a); }
@@ -373,10 +374,11 @@ constexpr int kMaxGraphTicks = 16384;   // larger device runs launch directly
 int build_device_graph(GpuBpfState* s, Impl* m, const float* y_dev, int n, BpfTickRecord* rec_dev) {
   if (m->dgraph) { cudaGraphExecDestroy(m->dgraph); m->dgraph = nullptr; }
   cudaGraph_t g = nullptr;
+  const TickArgs a0 = make_args(s, m, 0.0f, y_dev, rec_dev);
+  const bool one = one_launch(m, a0);                                   // (configures outside the capture)
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
-  const TickArgs a0 = make_args(s, m, 0.0f, y_dev, rec_dev);
-  if (one_launch(m, a0)) {
+  if (one) {
     err = launch_run(m, a0, n);                                         // the whole run as one launch
   } else {
     for (int k = 0; k < n && err == cudaSuccess; ++k) {

@@ -104,6 +104,7 @@ struct GpuBpfGrad {
 
   // the taped run
   bool have_fwd = false;
+  bool resident = false;             // the forward run is one resident launch
   FwdKey cur;
   std::vector<PcgTick> pcs;          // noise constants of ticks 0..T
 
@@ -138,7 +139,7 @@ cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
   const float std_stat = sqrtf((k.sigma * k.sigma) / fmaxf(1.0f - k.rho * k.rho, 1e-6f));   // gpu_bpf_ptx_full.cu:430
   cudaError_t e = launch_init(g->plan, k.mu, std_stat, k.seed, g->stream);
   const ObsModel obs = make_obs(k.nu);
-  if (e == cudaSuccess && k.T > 0 && g->plan.G <= g->res_tiles) {
+  if (e == cudaSuccess && k.T > 0 && g->resident) {
     // The whole taped run as one resident launch: N = 2^20 26 -> 13 us per tick, and three nodes to
     // capture anew for every theta instead of three per tick.
     TickArgs a{};
@@ -157,7 +158,7 @@ cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
     tape.aux = g->aux;
     e = launch_resident(g->plan, a, tape, false, k.T, g->res_tiles, g->stream);
   }
-  for (int t = 0; t < k.T && e == cudaSuccess && g->plan.G > g->res_tiles; ++t) {
+  for (int t = 0; t < k.T && e == cudaSuccess && !g->resident; ++t) {
     TickArgs a{};
     a.mu = k.mu; a.rho = k.rho; a.sigma = k.sigma;
     a.ess_threshold = 0.0f;
@@ -323,12 +324,13 @@ int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, floa
   FwdKey k;
   k.T = n_ticks; k.seed = seed; k.mu = mu; k.rho = rho; k.sigma = sigma_z; k.nu = nu_obs; k.nu_state = nu_state;
   k.y = y_dev; k.ll = loglik_dev;
+  g->resident = resident_ready(g->device, g->plan.G, g->res_tiles, nu_int_of(nu_state) > 0, !(nu_obs > 0.0f), false);
   if (!g->fgraph || !(g->fkey == k)) {
     GCK(capture(g, &g->fgraph, [&]() { return enqueue_forward(g, k); }));
     g->fkey = k;
   }
   GCK(cudaGraphLaunch(g->fgraph, g->stream));
-  bpf_note_launches(g->plan.G <= g->res_tiles ? 2 : 1 + 3LL * n_ticks);
+  bpf_note_launches(g->resident ? 2 : 1 + 3LL * n_ticks);
   g->cur = k;
   g->have_fwd = true;
   g->pcs.resize(n_ticks + 1);

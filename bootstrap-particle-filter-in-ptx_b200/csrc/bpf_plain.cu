@@ -1737,11 +1737,12 @@ cudaError_t plan_alloc(Plan& p, int N) {
   al(&p.P, p.G * sizeof(unsigned long long));
   al(&p.ofirst, (p.G + 1) * sizeof(int));
   al(&p.items, p.max_items * sizeof(int4));
-  al(&p.jpart, p.G * sizeof(double));
+  const size_t jbytes = (p.G * sizeof(double) + 255) & ~(size_t)255;
+  al(&p.jpart, jbytes + resident_xbuf_bytes(p.G));     // one allocation for both
+  if (e == cudaSuccess) p.xbuf = reinterpret_cast<unsigned char*>(p.jpart) + jbytes;
   al(&p.jticket, sizeof(unsigned));
   al(&p.pticket, sizeof(unsigned));
   al(&p.st, sizeof(DevState));
-  al(&p.xbuf, resident_xbuf_bytes(p.G));
   if (e == cudaSuccess) e = cudaMemset(p.nexp, 0, p.G * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(p.jticket, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(p.pticket, 0, sizeof(unsigned));
@@ -1754,7 +1755,7 @@ void plan_free(Plan& p) {
   bpf_free(p.h0); bpf_free(p.h1); bpf_free(p.w);
   bpf_free(p.nexp); bpf_free(p.E); bpf_free(p.rec); bpf_free(p.rec2);
   bpf_free(p.P); bpf_free(p.ofirst); bpf_free(p.items); bpf_free(p.st);
-  bpf_free(p.jpart); bpf_free(p.jticket); bpf_free(p.pticket); bpf_free(p.xbuf);
+  bpf_free(p.jpart); bpf_free(p.jticket); bpf_free(p.pticket);
   p = Plan{};
 }
 

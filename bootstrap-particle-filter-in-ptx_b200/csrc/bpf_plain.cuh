@@ -140,6 +140,8 @@ struct ResidentTape {        // gradient tape of a taped run from tick 0 (all nu
 constexpr int kResMaxTilesPerCta = 4;
 size_t resident_xbuf_bytes(int G);
 int resident_max_tiles(int device);    // 0: the device takes no resident runs
+// Whether the kernel of such a run (G tiles, observation and state noise model) is ready on the device.
+bool resident_ready(int device, int G, int max_tiles, bool tstate, bool gauss, bool apf);
 cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
                             int max_tiles, cudaStream_t s);
 int pass2_grid_size(int device);

@@ -845,6 +845,7 @@ ResidentKernel pick(int nt, bool tstate, bool gauss, bool apf, size_t* smem) {
 constexpr int kMaxConfiguredDevices = 64;
 std::mutex g_lock;
 int g_sms[kMaxConfiguredDevices] = {};       // 0: not looked at yet, -1: no resident runs on this device
+signed char g_ready[kMaxConfiguredDevices][24] = {};   // per kernel: 0 not configured yet, 1 ready, -1 does not fit
 
 }  // namespace
 
@@ -853,21 +854,33 @@ int resident_max_tiles(int device) {
   std::lock_guard<std::mutex> guard(g_lock);
   if (g_sms[device] == 0) {
     int sms = 0, coop = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-    bool ok = coop != 0 && sms > 0 && sms * kResMaxTilesPerCta <= kResMaxTiles;
-    for (int m = 0; m < 8 && ok; ++m)
-      for (int nt : {1, 2, 4}) {
-        size_t smem = 0;
-        ResidentKernel k = pick(nt, m & 1, m & 2, m & 4, &smem);
-        int per = 0;
-        ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kResThreads, smem) == cudaSuccess && per >= 1;
-      }
+    const bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
+                    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop != 0 &&
+                    sms > 0 && sms * kResMaxTilesPerCta <= kResMaxTiles;
     if (!ok) cudaGetLastError();
     g_sms[device] = ok ? sms : -1;
   }
   return g_sms[device] > 0 ? g_sms[device] * kResMaxTilesPerCta : 0;
+}
+
+// Called with `device` current, outside any stream capture; a kernel is loaded and given its shared
+// memory when the first filter that runs it asks.
+bool resident_ready(int device, int G, int max_tiles, bool tstate, bool gauss, bool apf) {
+  if (G < 1 || G > max_tiles || device < 0 || device >= kMaxConfiguredDevices) return false;
+  const int sms = max_tiles / kResMaxTilesPerCta, nt = (G + sms - 1) / sms;
+  const int shape = nt <= 1 ? 0 : (nt <= 2 ? 1 : 2);
+  std::lock_guard<std::mutex> guard(g_lock);
+  signed char& state = g_ready[device][shape * 8 + (tstate ? 1 : 0) + (gauss ? 2 : 0) + (apf ? 4 : 0)];
+  if (state == 0) {
+    size_t smem = 0;
+    int per = 0;
+    ResidentKernel k = pick(nt, tstate, gauss, apf, &smem);
+    const bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kResThreads, smem) == cudaSuccess && per >= 1;
+    if (!ok) cudaGetLastError();
+    state = ok ? 1 : -1;
+  }
+  return state > 0;
 }
 
 cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
