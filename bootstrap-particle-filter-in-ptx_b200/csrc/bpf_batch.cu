@@ -24,6 +24,7 @@
 // per filter.
 #include "bpf_batch.cuh"
 #include "bpf_block.cuh"
+#include "bpf_tick.cuh"
 
 namespace bpf {
 
@@ -50,6 +51,16 @@ struct BatchShared {
 // The tick's decision runs on thread 0; the FP64 logarithm of the weight sum, the increment and
 // the running log-likelihood on the first lane of the second warp (kLogTid), concurrently.
 constexpr int kLogTid = 32;
+
+// exact_count of a chunk whose particle e is at a0 ^ e: its first n particles.
+static __device__ __noinline__ int exact_count_chunk(const float* wt, int a0, int n, unsigned long long R0,
+                                                     unsigned long long D, int cap) {
+  unsigned long long l = 0ull;
+  for (int i = 0; i < n; ++i) l += fix_weight(tile_weight(wt[a0 ^ i]));
+  if (l < R0) return 0;
+  const unsigned long long c = udiv_fp64(l - R0, D) + 1ull;
+  return c >= (unsigned long long)cap ? cap : (int)c;
+}
 
 size_t batch_smem_bytes(int maxn, bool sort_perm) {
   const size_t u16 = (((size_t)maxn * 2 + 15) / 16) * 16;
@@ -450,6 +461,20 @@ __device__ void batch_run_filter(const BatchArgs& a, const BatchFilterDev& f, in
   __syncthreads();
 }
 
+__device__ __forceinline__ void step_epilogue(const BatchArgs& a) {
+  // every CTA has taken its last work item and read the tick before it counts
+  // itself done, so the last one may reset the counters and advance the tick
+  if (a.ep_done && threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(a.ep_done, 1) == a.ep_total - 1) {
+      for (int c = 0; c < a.ep_n; ++c) a.ep_counters[c] = 0;
+      if (a.ep_tick) *a.ep_tick += a.ep_add;
+      *a.ep_done = 0;
+      __threadfence();
+    }
+  }
+}
+
 template <int NT, bool NOISE>
 __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_kernel(BatchArgs a, int maxn) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -468,17 +493,451 @@ __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_ker
     const BatchFilterDev f = a.filters[b];
     batch_run_filter<NT, true, NOISE>(a, f, b, bufA, bufB, marks, sh, maxn, perm);
   }
-  // every CTA has taken its last work item and read the tick before it counts
-  // itself done, so the last one may reset the counters and advance the tick
-  if (a.ep_done && threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(a.ep_done, 1) == a.ep_total - 1) {
-      for (int c = 0; c < a.ep_n; ++c) a.ep_counters[c] = 0;
-      if (a.ep_tick) *a.ep_tick += a.ep_add;
-      *a.ep_done = 0;
-      __threadfence();
+  step_epilogue(a);
+}
+
+// ---------------------------------------------------------------------------
+// The same filter with at most EPT (4, 8 or 16) particles a thread, unrolled: the shapes that the
+// classes run with by default. Bit for bit the generic form's values: pass 1 keeps its strided
+// element order and reduction trees.
+// What bounded the generic form was issue: about 120 thread-instructions per particle and tick (64-bit
+// stream multiplies, swizzle arithmetic and bounds per element, the exact masses on every tick,
+// butterflies per sum) and 100 more where it resamples (64-bit compares per child). Here the PCG32
+// state is stepped, the log2-weights stay in registers between the two passes, the sums of all tiles
+// are reduced together, the exact masses are formed only on resampling ticks (from the chunk scan),
+// and the children come from pass 2's FP32 estimate with exact recounts, start marks and a vote scan.
+// ---------------------------------------------------------------------------
+template <int NT>
+struct BatchFastShared {
+  static constexpr int W = NT / 32;
+  float tmax[kBatchMaxTiles][W];
+  double sred[3 * kBatchMaxTiles][W];          // warp sums: value 3 k + {S, Q, H} of tile k
+  unsigned long long wsum[W];                  // chunk masses of each warp
+  unsigned long long Pk[kBatchMaxTiles];
+  unsigned long long base, delta, magic;
+  double fin_ll, fin_logS;
+  float carry_off[kBatchMaxTiles];
+  int rk[kBatchMaxTiles];
+  unsigned carry_mark[W];                      // ancestor mark of each warp's first gather slot
+  int resample, carry, next;
+  float hm_last;
+};
+
+// Sums of NV values at once over the WIDTH low lanes by the tree of warp_sum_d_w<WIDTH> (xor WIDTH/2
+// .. 1; addition commutes, so the values are the same): at each level a lane passes on the half of the
+// values that its partner keeps, about 2 NV exchanges in place of NV log2(WIDTH). The sum of value
+// fold_index<NV, WIDTH>(lane) ends in that lane.
+template <int NV, int WIDTH>
+__device__ __forceinline__ double fold_sums(double (&v)[NV], int lane) {
+  int n = NV;
+#pragma unroll
+  for (int o = WIDTH / 2; o; o >>= 1) {
+    if (n > 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < NV / 2; ++i)
+        if (i < n / 2) {
+          const double keep = up ? v[i + n / 2] : v[i], give = up ? v[i] : v[i + n / 2];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      n >>= 1;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
     }
   }
+  return v[0];
+}
+template <int NV, int WIDTH>
+__device__ __forceinline__ int fold_index(int lane) {
+  int idx = 0, n = NV;
+#pragma unroll
+  for (int o = WIDTH / 2; o; o >>= 1)
+    if (n > 1) { n >>= 1; if (lane & o) idx += n; }
+  return idx;
+}
+// Exact sum over the warp of values below 2^59: three integer warp reductions.
+__device__ __forceinline__ unsigned long long warp_sum_u59(unsigned long long v) {
+  constexpr unsigned m = (1u << 27) - 1u;
+  const unsigned a = __reduce_add_sync(0xffffffffu, (unsigned)v & m);
+  const unsigned b = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 27) & m);
+  const unsigned c = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 54));
+  return (unsigned long long)a + ((unsigned long long)b << 27) + ((unsigned long long)c << 54);
+}
+
+template <int NT, int EPT, bool GAUSS>
+__device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const BatchFilterDev& f, int b, float* bufA, float* bufB,
+                                                  unsigned short* marks, BatchFastShared<NT>& sh, int maxn) {
+  constexpr int W = NT / 32;
+  constexpr int TM = NT < kTile ? kTile / NT : 1;        // elements of a thread per tile
+  constexpr int GM = (EPT + TM - 1) / TM;                // tiles a filter of this shape can have
+  constexpr int NV = GM == 1 ? 4 : (GM == 2 ? 8 : 16);   // sums, padded to a power of two
+  static_assert(GM <= kBatchMaxTiles && NV >= 3 * GM, "sums of every tile");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int N = f.n;
+  const int G = (N + kTile - 1) / kTile;
+  ObsModel obs;
+  obs.y = 0.0f; obs.nu = f.nu; obs.c_obs = f.c_obs; obs.inv_nu = f.inv_nu; obs.nu_p1h = f.nu_p1h;
+  float* H = bufA;
+  float* Wt = bufB;
+  uint64_t At = 1ull, Bt = 0ull;
+  const double logN = log((double)N);
+  double logS_prev = logN, ll_total = 0.0;               // kept by thread kLogTid
+  uint64_t ustate = (unsigned long long)f.seed * 67890ULL + 12345ULL;   // thread 0
+  int n_res = 0;
+  float hm_last = 0.0f;                                  // kLogTid
+  const int t0 = a.t0_dev ? *a.t0_dev : 0;
+  BatchFilterState* fs = a.st ? a.st + b : nullptr;
+  const long long soff = a.st ? a.st_off[b] : 0;
+  // element m of this thread is particle tid + NT m, at swz(tid + NT m)
+  const int p0 = (tid & ~31) | ((lane ^ warp) & 31);
+  auto at = [&](int m) { return (p0 ^ (((NT / 32) * m) & 31)) + NT * m; };
+  if (fs && t0 > 0) {
+    const BatchFilterState r = *fs;
+    for (int i = tid; i < N; i += NT) H[swz(i)] = a.st_h[soff + i];
+    if (r.carry)
+      for (int i = tid; i < N; i += NT) Wt[swz(i)] = a.st_w[soff + i];
+    pcg_jump((uint64_t)t0, &At, &Bt);
+    logS_prev = r.logS_prev; ll_total = r.ll_total; ustate = r.ustate; n_res = r.n_res; hm_last = r.hm_last;
+    if (tid == 0) {
+      sh.carry = r.carry;
+      for (int k = 0; k < kBatchMaxTiles; ++k) sh.carry_off[k] = r.carry_off[k];
+    }
+  } else {
+    const PcgTick c = pcg_tick_consts(f.seed, 1ull, 0ull);
+    for (int i = tid; i < N; i += NT) {
+      const uint64_t s = c.k1 + c.k2 * pcg_inc((uint32_t)i);
+      bufA[swz(i)] = fmaf(f.std_stat, icdf_normal(pcg_uniform(pcg_output(s))), f.mu);
+    }
+    if (tid == 0) sh.carry = 0;
+  }
+  __syncthreads();
+  const int region = ((N + W - 1) / W + 127) & ~127;     // gather slots of a warp
+
+  for (int t = t0; t < t0 + a.T; ++t) {
+    const float y = __ldg(a.y + (a.y_abs ? t : t - t0));
+    const float y2 = y * y;
+    obs.y = y;
+    const bool carry = sh.carry != 0;
+    const PcgTick c = pcg_tick_consts(f.seed, At, Bt);
+    float* ck = (a.g_ckpt && t % a.g_K == 0) ? a.g_ckpt + (size_t)(t / a.g_K) * maxn : nullptr;
+
+    // 1. propagate + log2-weight, per-tile max
+    float x[EPT];
+    {
+      uint64_t s = c.k1 + c.k2 * pcg_inc((uint32_t)tid);
+      const uint64_t step = (uint64_t)(2 * NT) * c.k2;
+      const float y2nu = __fmul_rn(y2, obs.inv_nu);
+#pragma unroll
+      for (int k = 0; k < GM; ++k) {
+        float mx = -INFINITY;
+        const float coff = carry && k < G ? sh.carry_off[k] : 0.0f;
+        const float gc = kGaussLog2C + coff, tc = __fmul_rn(obs.c_obs, kLog2e) + coff;
+#pragma unroll
+        for (int mm = 0; mm < TM; ++mm) {
+          const int m = k * TM + mm;
+          if (m >= EPT) continue;
+          x[m] = -INFINITY;
+          if (NT * m < N) {                              // the same for the whole CTA
+            const bool in = tid + NT * m < N;
+            const int si = at(m);
+            float h = in ? H[si] : 0.0f;
+            if (ck && in) ck[tid + NT * m] = h;
+            if (t > 0) {
+              float z = icdf_normal_warp(pcg_uniform(pcg_output(s)));
+              if (f.nu_int > 0) z *= tstate_scale_warp(s, c.k2 << 33, f.nu_int, f.nu_state);
+              h = propagate(h, f.mu, f.rho, f.sigma, z);
+              if (in) H[si] = h;
+            }
+            float v = GAUSS ? obs_log2pdf_gauss_plus(y2, h, gc) : obs_log2pdf_t_plus(obs, y2nu, h, tc);
+            if (carry && in) v += Wt[si];                // carried tile-relative log2-weight
+            if (in) { x[m] = v; mx = fmaxf(mx, v); }
+            s += step;
+          }
+        }
+        if (k < G) {
+          mx = warp_max_f(mx);
+          if (lane == 0) sh.tmax[k][warp] = mx;
+        }
+      }
+    }
+    __syncthreads();
+
+    // 2. tile-relative weights and partial sums
+    int nk[GM];
+    double v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = 0.0;
+#pragma unroll
+    for (int k = 0; k < GM; ++k) {
+      nk[k] = kNkEmpty;
+      if (k >= G) continue;
+      const float mx = warp_max_f(sh.tmax[k][lane % W]);
+      nk[k] = (mx == -INFINITY) ? kNkEmpty : (int)ceilf(fmaxf(mx, -1.0e9f));
+      const float fnk = (nk[k] == kNkEmpty) ? INFINITY : (float)nk[k];
+      float fS = 0.f, fQ = 0.f, fH = 0.f;
+#pragma unroll
+      for (int mm = 0; mm < TM; ++mm) {
+        const int m = k * TM + mm;
+        if (m >= EPT) continue;
+        if (NT * m < N && tid + NT * m < N) {
+          const int si = at(m);
+          const float d = x[m] - fnk;
+          const float w = tile_weight(d);
+          Wt[si] = d;
+          fS += w;
+          fQ = fmaf(w, w, fQ);
+          fH = fmaf(w, H[si], fH);
+        }
+      }
+      v[3 * k] = (double)fS; v[3 * k + 1] = (double)fQ; v[3 * k + 2] = (double)fH;
+    }
+    {
+      const double r = fold_sums<NV, 32>(v, lane);
+      const int idx = fold_index<NV, 32>(lane);
+      if ((lane & (32 / NV - 1)) == 0 && idx < 3 * GM) sh.sred[idx][warp] = r;
+    }
+    __syncthreads();
+
+    // 3. decision (warp 0), log-likelihood and mean (warp 1), from the same sums
+    if (warp < 2) {
+      double tot[3 * GM];
+#pragma unroll
+      for (int i = 0; i < 3 * GM; ++i) {
+        tot[i] = 0.0;
+        if (i / 3 < G) tot[i] = warp_sum_d_w<W>(lane < W ? sh.sred[i][lane] : 0.0);
+      }
+      if (lane == 0) {
+        int nM = kNkEmpty;
+#pragma unroll
+        for (int k = 0; k < GM; ++k) nM = max(nM, nk[k]);
+        double S = 0.0, Q = 0.0, Hm = 0.0;
+#pragma unroll
+        for (int k = 0; k < GM; ++k) {
+          if (k >= G || nk[k] == kNkEmpty) continue;
+          const double sc = pow2d(nk[k] - nM);
+          S += tot[3 * k] * sc; Q += tot[3 * k + 1] * sc * sc; Hm += tot[3 * k + 2] * sc;
+        }
+        const bool degenerate = (nM == kNkEmpty) || !(S > 0.0);
+        int resample = 0;
+        if (!degenerate) {
+          const double ess = S * S / Q;
+          resample = (a.ess_threshold <= 0.0f) || (ess / (double)N < (double)a.ess_threshold);
+        }
+        if (warp == 1) {
+          const double lS = degenerate ? 0.0 : log(S);
+          const double dll = degenerate ? -INFINITY
+                                        : (double)nM * 0.693147180559945309417232121458 + lS - logS_prev;
+          ll_total += dll;
+          if (a.dll) a.dll[(size_t)b * a.T + (t - t0)] = dll;
+          logS_prev = (resample || degenerate) ? logN : lS;
+          const float hm = degenerate ? __int_as_float(0x7fc00000) : (float)(Hm / S);
+          hm_last = hm;
+          if (a.g_norm)
+            a.g_norm[t] = degenerate ? make_float2(0.0f, 0.0f) : make_float2((float)(1.0 / S), __int_as_float(nM));
+          if (a.hmean) a.hmean[(size_t)b * a.T + (t - t0)] = hm;
+        } else {
+          if (resample) {
+            ++n_res;
+            const int Fg = min(kFixF, 62 - ceil_log2_u((unsigned)N));
+#pragma unroll
+            for (int k = 0; k < GM; ++k) sh.rk[k] = (k < G && nk[k] != kNkEmpty) ? nM - nk[k] + kFixF - Fg : 64;
+            sh.carry = 0;
+          } else if (degenerate) {
+            sh.carry = 0;
+          } else {
+#pragma unroll
+            for (int k = 0; k < GM; ++k)
+              sh.carry_off[k] = (k < G && nk[k] != kNkEmpty) ? (float)(nk[k] - nM) : -INFINITY;
+            sh.carry = 1;
+          }
+          sh.resample = resample;
+        }
+      }
+    }
+    At = At * kPcgMult;
+    Bt = Bt * kPcgMult + 1ull;
+    __syncthreads();
+
+    // 4. systematic resampling (the plain filter's fixed-point rule), EPT consecutive particles a thread
+    if (sh.resample) {
+      const int j0 = tid * EPT;
+      const int q0a = swz(j0);                             // particle j0 + e is at q0a ^ e
+      const int nl = min(max(N - j0, 0), EPT);
+      unsigned long long run = 0ull;
+      float lfT = 0.0f;
+#pragma unroll
+      for (int e = 0; e < EPT; ++e) {
+        const float w = e < nl ? tile_weight(Wt[q0a ^ e]) : 0.0f;
+        run += fix_weight(w);
+        lfT += w;
+      }
+      const unsigned long long incl = warp_incl_scan_add(run, lane);
+      if (lane == 31) sh.wsum[warp] = incl;
+      for (int i = tid; i < (N + 7) / 8; i += NT) reinterpret_cast<uint4*>(marks)[i] = make_uint4(0u, 0u, 0u, 0u);
+      __syncthreads();
+      constexpr int TW = kTile / (32 * EPT) < W ? kTile / (32 * EPT) : W;   // warps of a tile
+      const int k = (warp / TW) < kBatchMaxTiles ? warp / TW : 0;
+      const unsigned long long ws = lane < W ? sh.wsum[lane] : 0ull;
+      const unsigned long long loc = warp_sum_u59(lane >= k * TW && lane < warp ? ws : 0ull) + incl - run;
+      if (warp == 0) {                                     // the targets and the tiles' prefixes
+        unsigned long long P = 0ull;
+#pragma unroll
+        for (int kk = 0; kk < GM; ++kk) {
+          const unsigned long long m = warp_sum_u59(lane / TW == kk ? ws : 0ull);
+          if (lane == 0) sh.Pk[kk] = P;
+          P += shr64(m, sh.rk[kk]);
+        }
+        if (lane == 0) {
+          const uint64_t old = ustate;
+          ustate = old * kPcgMult + kHostInc;
+          const unsigned long long u = pcg_output(old) >> 9;
+          unsigned long long delta = udiv_fp64(P, (unsigned long long)N);
+          if (delta == 0ull) delta = 1ull;
+          const unsigned long long hi = __umul64hi(u, delta), lo = u * delta;
+          sh.base = (hi << 41) | (lo >> 23);
+          sh.delta = delta;
+          sh.magic = udiv_magic_of(delta);
+        }
+      }
+      __syncthreads();
+      {
+        const unsigned long long base = sh.base, delta = sh.delta;
+        const int r = j0 < N ? sh.rk[k] : 64;
+        const unsigned long long Pk = sh.Pk[k];
+        ChunkTargets<EPT> ct;                              // (its weights are read again below, not kept)
+        chunk_thresholds<EPT>(N, loc, Pk, r, j0 < N, base, delta, sh.magic, ct);
+        const unsigned long long R0 = ct.th, D = ct.D;
+        const bool none = R0 >= kThCap;
+        // the running count's FP32 estimate and its error bound (chunk_child_ends)
+        const float R0w = (float)R0 * 0x1p-50f;
+        const float invDw = 1.0f / ((float)D * 0x1p-50f);
+        const float R0x = R0w * invDw;
+        const float eL = 0x1p-18f * invDw, e0 = fmaf(R0w, eL, 0x1p-44f * invDw);
+        const float xT = fmaf(lfT, invDw, -R0x);
+        float err = fmaf(lfT, eL, fmaf(fmaxf(fabsf(xT), R0x), 0x1p-21f, e0));
+        if (!(xT < 0x1p22f)) err = 1.0f;
+        const float err_hi = 1.0f - err;
+        const int q0 = j0 < N ? ct.q : N, Kq = 0x4AFFFFFF - q0;
+        unsigned short* lst = a.g_list ? a.g_list + (size_t)t * maxn : nullptr;
+        // the next gather region that starts at or after the chunk's first child slot
+        int rg = (q0 + region - 1) / region, rslot = rg * region;
+        float lf = 0.0f;
+        int qp = q0;
+#pragma unroll 1
+        for (int g = 0; g < EPT / 4; ++g) {
+          int qq[4];
+          bool rc[4], any = false;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = 4 * g + e;
+            lf += i < nl ? tile_weight(Wt[q0a ^ i]) : 0.0f;
+            const float xx = fmaf(lf, invDw, -R0x);
+            const float fl = floorf(xx);
+            const float fr = xx - fl;                      // exact
+            rc[e] = !none && !(fr > err && fr < err_hi);
+            any |= rc[e];
+            qq[e] = none ? q0 : min(max(__float_as_int(fl + 0x1p23f) - Kq, q0), N);
+          }
+          if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (rc[e]) qq[e] = min(q0 + exact_count_chunk(Wt, q0a, min(4 * g + e + 1, nl), R0, D, N), N);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = 4 * g + e;
+            if (lst) lst[i * NT + tid] = (unsigned short)(i < nl ? qp : N);   // children of j start at slot qp
+            if (qq[e] > qp) {
+              marks[qp] = (unsigned short)(j0 + i + 1);
+              while (rslot < qq[e]) {                      // the ancestor of a region's first slot
+                if (rg < W) sh.carry_mark[rg] = (unsigned)(j0 + i + 1);
+                ++rg; rslot += region;
+              }
+            }
+            qp = qq[e];
+          }
+        }
+      }
+      __syncthreads();
+      {
+        // gather: warp w the slots [w region, (w + 1) region), four a lane
+        const int rs = warp * region, re = min(rs + region, N);
+        unsigned last = rs < N ? sh.carry_mark[warp] : 0u;
+        for (int o0 = rs; o0 < re; o0 += 128) {
+          const int o = o0 + 4 * lane;
+          const uint2 mv = o < re ? *reinterpret_cast<const uint2*>(marks + o) : make_uint2(0u, 0u);
+          unsigned am[4];
+          am[0] = mv.x & 0xffffu;
+          am[1] = max(am[0], mv.x >> 16);
+          am[2] = max(am[1], mv.y & 0xffffu);
+          am[3] = max(am[2], mv.y >> 16);
+          unsigned pr, nl2;
+          marks_before(am[3], lane, last, pr, nl2);
+          last = nl2;
+          const int so = swz(o);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (o + e < re) {
+              const int anc = (int)max(pr, am[e]) - 1;
+              Wt[so ^ e] = H[swz(anc)];
+              if (a.anc) a.anc[((size_t)b * a.T + (t - t0)) * kBatchMaxN + o + e] = anc;
+            }
+          }
+        }
+      }
+      __syncthreads();
+      float* tmp = H; H = Wt; Wt = tmp;
+    }
+  }
+  if (a.particles)
+    for (int i = tid; i < N; i += NT) a.particles[(size_t)b * kBatchMaxN + i] = H[swz(i)];
+  if (fs) {
+    for (int i = tid; i < N; i += NT) a.st_h[soff + i] = H[swz(i)];
+    if (sh.carry)
+      for (int i = tid; i < N; i += NT) a.st_w[soff + i] = Wt[swz(i)];
+  }
+  if (tid == kLogTid) { sh.fin_ll = ll_total; sh.fin_logS = logS_prev; sh.hm_last = hm_last; }
+  __syncthreads();
+  if (tid == 0) {
+    a.loglik[b] = sh.fin_ll;
+    a.h_final[b] = sh.hm_last;
+    a.resamples[b] = n_res;
+    if (fs) {
+      BatchFilterState r;
+      r.logS_prev = sh.fin_logS; r.ll_total = sh.fin_ll; r.ustate = ustate;
+      r.carry = sh.carry; r.n_res = n_res; r.hm_last = sh.hm_last; r.pad = 0;
+      for (int k = 0; k < kBatchMaxTiles; ++k) r.carry_off[k] = sh.carry_off[k];
+      *fs = r;
+    }
+  }
+  __syncthreads();
+}
+
+// Particles per thread of the unrolled form for a class of filters of at most maxn particles (0: the
+// generic form).
+__host__ __device__ constexpr int batch_ept(int threads, int maxn) {
+  return maxn <= 4 * threads ? 4 : (maxn <= 8 * threads ? 8 : (maxn <= 16 * threads ? 16 : 0));
+}
+
+template <int NT, int EPT>
+__global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_fast_kernel(BatchArgs a, int maxn) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ BatchFastShared<NT> sh;
+  float* bufA = reinterpret_cast<float*>(smem);
+  float* bufB = bufA + maxn;
+  unsigned short* marks = reinterpret_cast<unsigned short*>(bufB + maxn);
+  for (;;) {
+    if (threadIdx.x == 0) sh.next = atomicAdd(a.counter, 1);
+    __syncthreads();
+    const int idx = sh.next;
+    __syncthreads();
+    if (idx >= a.n_order) break;
+    const int b = a.order[idx];
+    const BatchFilterDev f = a.filters[b];
+    if (f.nu > 0.0f) batch_fast_filter<NT, EPT, false>(a, f, b, bufA, bufB, marks, sh, maxn);
+    else batch_fast_filter<NT, EPT, true>(a, f, b, bufA, bufB, marks, sh, maxn);
+  }
+  step_epilogue(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -744,6 +1203,17 @@ __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_gra
   }
 }
 
+// The kernel that runs a class without correlated noise: unrolled where its shape has a form.
+template <int NT, class F>
+static void with_plain_kernel(int maxn, F f) {
+  switch (batch_ept(NT, maxn)) {
+    case 4: f(batch_fast_kernel<NT, 4>); break;
+    case 8: f(batch_fast_kernel<NT, 8>); break;
+    case 16: f(batch_fast_kernel<NT, 16>); break;
+    default: f(batch_kernel<NT, false>); break;
+  }
+}
+
 // The dynamic shared-memory attribute is set by batch_occupancy (called when
 // a class is configured, outside any stream capture).
 template <int NT>
@@ -751,7 +1221,7 @@ static cudaError_t launch_nt(const BatchArgs& a, int maxn, int grid, cudaStream_
   if (a.nz_out)
     batch_kernel<NT, true><<<grid, NT, batch_smem_bytes(maxn, a.anc != nullptr), s>>>(a, maxn);
   else
-    batch_kernel<NT, false><<<grid, NT, batch_smem_bytes(maxn), s>>>(a, maxn);
+    with_plain_kernel<NT>(maxn, [&](auto k) { k<<<grid, NT, batch_smem_bytes(maxn), s>>>(a, maxn); });
   return cudaGetLastError();
 }
 
@@ -769,11 +1239,13 @@ cudaError_t launch_batch_class(const BatchArgs& a, int threads, int maxn, int gr
 template <int NT>
 static int occ_nt(int maxn) {
   const size_t smem = batch_smem_bytes(maxn);
-  cudaFuncSetAttribute(batch_kernel<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaFuncSetAttribute(batch_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)batch_smem_bytes(maxn, true));
   int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_kernel<NT, false>, NT, smem);
+  with_plain_kernel<NT>(maxn, [&](auto k) {
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, NT, smem);
+  });
   return per;
 }
 
