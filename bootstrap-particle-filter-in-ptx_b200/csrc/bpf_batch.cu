@@ -25,6 +25,7 @@
 #include "bpf_batch.cuh"
 #include "bpf_block.cuh"
 #include "bpf_tick.cuh"
+#include <type_traits>
 
 namespace bpf {
 
@@ -44,7 +45,6 @@ struct BatchShared {
   int rk[kBatchMaxTiles];
   unsigned long long base, delta, magic;
   int resample, carry, next;
-  double gred[5][NT / 32];
   double fin_ll, fin_logS;                     // the log-likelihood keeper's state at the end of a run
 };
 
@@ -515,7 +515,12 @@ struct BatchFastShared {
   unsigned long long wsum[W];                  // chunk masses of each warp
   unsigned long long Pk[kBatchMaxTiles];
   unsigned long long base, delta, magic;
-  double fin_ll, fin_logS;
+  // the filter's table entry and the state that one thread keeps (registers are the batch's limit)
+  BatchFilterDev f;
+  unsigned long long k1, k2;                   // PCG32 stream constants of the next tick (thread 0)
+  unsigned long long ustate;                   // thread 0
+  double logN, logS_prev, ll_total;            // thread kLogTid
+  int n_res;                                   // thread 0
   float carry_off[kBatchMaxTiles];
   int rk[kBatchMaxTiles];
   unsigned carry_mark[W];                      // ancestor mark of each warp's first gather slot
@@ -564,9 +569,16 @@ __device__ __forceinline__ unsigned long long warp_sum_u59(unsigned long long v)
   return (unsigned long long)a + ((unsigned long long)b << 27) + ((unsigned long long)c << 54);
 }
 
-template <int NT, int EPT, bool GAUSS>
-__device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const BatchFilterDev& f, int b, float* bufA, float* bufB,
+// Position of output slot o's mark (u16): groups of four stay together, groups are spread so that the
+// marks of a warp's lanes, EPT slots apart, fall on different banks.
+__device__ __forceinline__ int mark_pos(int o) { return (((o >> 2) ^ ((o >> 6) & 15)) << 2) | (o & 3); }
+
+// Slots past N up to the last group of NT particles hold finite particles and weight 0 (log2-weight
+// -inf), so no element tests its index; TAPE: a gradient run's taped forward.
+template <int NT, int EPT, bool GAUSS, bool TAPE>
+__device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, int b, float* bufA, float* bufB,
                                                   unsigned short* marks, BatchFastShared<NT>& sh, int maxn) {
+  const BatchFilterDev& f = sh.f;
   constexpr int W = NT / 32;
   constexpr int TM = NT < kTile ? kTile / NT : 1;        // elements of a thread per tile
   constexpr int GM = (EPT + TM - 1) / TM;                // tiles a filter of this shape can have
@@ -575,91 +587,105 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = f.n;
   const int G = (N + kTile - 1) / kTile;
-  ObsModel obs;
-  obs.y = 0.0f; obs.nu = f.nu; obs.c_obs = f.c_obs; obs.inv_nu = f.inv_nu; obs.nu_p1h = f.nu_p1h;
   float* H = bufA;
   float* Wt = bufB;
-  uint64_t At = 1ull, Bt = 0ull;
-  const double logN = log((double)N);
-  double logS_prev = logN, ll_total = 0.0;               // kept by thread kLogTid
-  uint64_t ustate = (unsigned long long)f.seed * 67890ULL + 12345ULL;   // thread 0
-  int n_res = 0;
-  float hm_last = 0.0f;                                  // kLogTid
   const int t0 = a.t0_dev ? *a.t0_dev : 0;
   BatchFilterState* fs = a.st ? a.st + b : nullptr;
   const long long soff = a.st ? a.st_off[b] : 0;
+  const int npad = (N + NT - 1) / NT * NT;
   // element m of this thread is particle tid + NT m, at swz(tid + NT m)
   const int p0 = (tid & ~31) | ((lane ^ warp) & 31);
   auto at = [&](int m) { return (p0 ^ (((NT / 32) * m) & 31)) + NT * m; };
   if (fs && t0 > 0) {
     const BatchFilterState r = *fs;
-    for (int i = tid; i < N; i += NT) H[swz(i)] = a.st_h[soff + i];
+    for (int i = tid; i < npad; i += NT) H[swz(i)] = i < N ? a.st_h[soff + i] : 0.0f;
     if (r.carry)
       for (int i = tid; i < N; i += NT) Wt[swz(i)] = a.st_w[soff + i];
-    pcg_jump((uint64_t)t0, &At, &Bt);
-    logS_prev = r.logS_prev; ll_total = r.ll_total; ustate = r.ustate; n_res = r.n_res; hm_last = r.hm_last;
     if (tid == 0) {
+      uint64_t At, Bt;
+      pcg_jump((uint64_t)t0, &At, &Bt);
+      const PcgTick c = pcg_tick_consts(f.seed, At, Bt);
+      sh.k1 = c.k1; sh.k2 = c.k2;
+      sh.logN = log((double)N);
+      sh.logS_prev = r.logS_prev; sh.ll_total = r.ll_total; sh.ustate = r.ustate; sh.n_res = r.n_res; sh.hm_last = r.hm_last;
       sh.carry = r.carry;
       for (int k = 0; k < kBatchMaxTiles; ++k) sh.carry_off[k] = r.carry_off[k];
     }
   } else {
     const PcgTick c = pcg_tick_consts(f.seed, 1ull, 0ull);
-    for (int i = tid; i < N; i += NT) {
+    for (int i = tid; i < npad; i += NT) {
       const uint64_t s = c.k1 + c.k2 * pcg_inc((uint32_t)i);
       bufA[swz(i)] = fmaf(f.std_stat, icdf_normal(pcg_uniform(pcg_output(s))), f.mu);
     }
-    if (tid == 0) sh.carry = 0;
+    if (tid == 0) {
+      sh.k1 = c.k1; sh.k2 = c.k2;
+      sh.logN = sh.logS_prev = log((double)N);
+      sh.ll_total = 0.0;
+      sh.ustate = (unsigned long long)f.seed * 67890ULL + 12345ULL;
+      sh.n_res = 0; sh.hm_last = 0.0f; sh.carry = 0;
+    }
   }
   __syncthreads();
   const int region = ((N + W - 1) / W + 127) & ~127;     // gather slots of a warp
+  int llog = 0;                                          // TAPE: log2 of the backward's parents a thread
+  if (TAPE) while ((NT << llog) < N) ++llog;
+  const int lchunk = 1 << llog;
 
   for (int t = t0; t < t0 + a.T; ++t) {
     const float y = __ldg(a.y + (a.y_abs ? t : t - t0));
     const float y2 = y * y;
-    obs.y = y;
     const bool carry = sh.carry != 0;
-    const PcgTick c = pcg_tick_consts(f.seed, At, Bt);
-    float* ck = (a.g_ckpt && t % a.g_K == 0) ? a.g_ckpt + (size_t)(t / a.g_K) * maxn : nullptr;
+    if (TAPE && t % a.g_K == 0) {
+      float* ck = a.g_ckpt + (size_t)(t / a.g_K) * maxn;
+      for (int i = tid; i < N; i += NT) ck[i] = H[swz(i)];
+    }
 
     // 1. propagate + log2-weight, per-tile max
     float x[EPT];
-    {
+    const int lim = N - tid;
+    // compiled once each without propagation (tick 0), with Gaussian and with Student-t state noise
+    auto particles = [&](auto prop_tag, auto ts_tag) {
+      constexpr bool PROP = decltype(prop_tag)::value, TS = decltype(ts_tag)::value;
+      const PcgTick c{sh.k1, sh.k2};
+      ObsModel obs;
+      obs.y = y; obs.nu = f.nu; obs.c_obs = f.c_obs; obs.inv_nu = f.inv_nu; obs.nu_p1h = f.nu_p1h;
+      const float mu = f.mu, rho = f.rho, sigma = f.sigma;
       uint64_t s = c.k1 + c.k2 * pcg_inc((uint32_t)tid);
       const uint64_t step = (uint64_t)(2 * NT) * c.k2;
       const float y2nu = __fmul_rn(y2, obs.inv_nu);
 #pragma unroll
       for (int k = 0; k < GM; ++k) {
+        if (k > 0 && k >= G) continue;
         float mx = -INFINITY;
-        const float coff = carry && k < G ? sh.carry_off[k] : 0.0f;
+        const float coff = carry ? sh.carry_off[k] : 0.0f;
         const float gc = kGaussLog2C + coff, tc = __fmul_rn(obs.c_obs, kLog2e) + coff;
 #pragma unroll
         for (int mm = 0; mm < TM; ++mm) {
           const int m = k * TM + mm;
           if (m >= EPT) continue;
-          x[m] = -INFINITY;
           if (NT * m < N) {                              // the same for the whole CTA
-            const bool in = tid + NT * m < N;
             const int si = at(m);
-            float h = in ? H[si] : 0.0f;
-            if (ck && in) ck[tid + NT * m] = h;
-            if (t > 0) {
+            float h = H[si];
+            if (PROP) {
               float z = icdf_normal_warp(pcg_uniform(pcg_output(s)));
-              if (f.nu_int > 0) z *= tstate_scale_warp(s, c.k2 << 33, f.nu_int, f.nu_state);
-              h = propagate(h, f.mu, f.rho, f.sigma, z);
-              if (in) H[si] = h;
+              if (TS) z *= tstate_scale_warp(s, c.k2 << 33, f.nu_int, f.nu_state);
+              h = propagate(h, mu, rho, sigma, z);
+              H[si] = h;
+              s += step;
             }
             float v = GAUSS ? obs_log2pdf_gauss_plus(y2, h, gc) : obs_log2pdf_t_plus(obs, y2nu, h, tc);
-            if (carry && in) v += Wt[si];                // carried tile-relative log2-weight
-            if (in) { x[m] = v; mx = fmaxf(mx, v); }
-            s += step;
+            if (carry) v += Wt[si];                      // carried tile-relative log2-weight
+            x[m] = NT * m < lim ? v : -INFINITY;
+            mx = fmaxf(mx, x[m]);
           }
         }
-        if (k < G) {
-          mx = warp_max_f(mx);
-          if (lane == 0) sh.tmax[k][warp] = mx;
-        }
+        mx = warp_max_f(mx);
+        if (lane == 0) sh.tmax[k][warp] = mx;
       }
-    }
+    };
+    if (t == 0) particles(std::false_type{}, std::false_type{});
+    else if (f.nu_int > 0) particles(std::true_type{}, std::true_type{});
+    else particles(std::true_type{}, std::false_type{});
     __syncthreads();
 
     // 2. tile-relative weights and partial sums
@@ -679,7 +705,7 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
       for (int mm = 0; mm < TM; ++mm) {
         const int m = k * TM + mm;
         if (m >= EPT) continue;
-        if (NT * m < N && tid + NT * m < N) {
+        if (NT * m < N) {
           const int si = at(m);
           const float d = x[m] - fnk;
           const float w = tile_weight(d);
@@ -726,18 +752,18 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
         if (warp == 1) {
           const double lS = degenerate ? 0.0 : log(S);
           const double dll = degenerate ? -INFINITY
-                                        : (double)nM * 0.693147180559945309417232121458 + lS - logS_prev;
-          ll_total += dll;
+                                        : (double)nM * 0.693147180559945309417232121458 + lS - sh.logS_prev;
+          sh.ll_total += dll;
           if (a.dll) a.dll[(size_t)b * a.T + (t - t0)] = dll;
-          logS_prev = (resample || degenerate) ? logN : lS;
+          sh.logS_prev = (resample || degenerate) ? sh.logN : lS;
           const float hm = degenerate ? __int_as_float(0x7fc00000) : (float)(Hm / S);
-          hm_last = hm;
+          sh.hm_last = hm;
           if (a.g_norm)
             a.g_norm[t] = degenerate ? make_float2(0.0f, 0.0f) : make_float2((float)(1.0 / S), __int_as_float(nM));
           if (a.hmean) a.hmean[(size_t)b * a.T + (t - t0)] = hm;
         } else {
           if (resample) {
-            ++n_res;
+            ++sh.n_res;
             const int Fg = min(kFixF, 62 - ceil_log2_u((unsigned)N));
 #pragma unroll
             for (int k = 0; k < GM; ++k) sh.rk[k] = (k < G && nk[k] != kNkEmpty) ? nM - nk[k] + kFixF - Fg : 64;
@@ -751,29 +777,29 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
             sh.carry = 1;
           }
           sh.resample = resample;
+          sh.k1 = sh.k1 * kPcgMult;
+          sh.k2 = sh.k2 * kPcgMult + 1ull;
         }
       }
     }
-    At = At * kPcgMult;
-    Bt = Bt * kPcgMult + 1ull;
     __syncthreads();
 
     // 4. systematic resampling (the plain filter's fixed-point rule), EPT consecutive particles a thread
     if (sh.resample) {
       const int j0 = tid * EPT;
-      const int q0a = swz(j0);                             // particle j0 + e is at q0a ^ e
-      const int nl = min(max(N - j0, 0), EPT);
+      const int q0a = swz(j0 < npad ? j0 : 0);             // particle j0 + e is at q0a ^ e (a thread past npad counts none)
       unsigned long long run = 0ull;
       float lfT = 0.0f;
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
-        const float w = e < nl ? tile_weight(Wt[q0a ^ e]) : 0.0f;
+        // (particles past the last group of NT were never written)
+        const float w = j0 < npad ? tile_weight(Wt[q0a ^ e]) : 0.0f;
         run += fix_weight(w);
         lfT += w;
       }
       const unsigned long long incl = warp_incl_scan_add(run, lane);
       if (lane == 31) sh.wsum[warp] = incl;
-      for (int i = tid; i < (N + 7) / 8; i += NT) reinterpret_cast<uint4*>(marks)[i] = make_uint4(0u, 0u, 0u, 0u);
+      for (int i = tid; i < (N + 63) / 64 * 8; i += NT) reinterpret_cast<uint4*>(marks)[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncthreads();
       constexpr int TW = kTile / (32 * EPT) < W ? kTile / (32 * EPT) : W;   // warps of a tile
       const int k = (warp / TW) < kBatchMaxTiles ? warp / TW : 0;
@@ -788,8 +814,8 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
           P += shr64(m, sh.rk[kk]);
         }
         if (lane == 0) {
-          const uint64_t old = ustate;
-          ustate = old * kPcgMult + kHostInc;
+          const uint64_t old = sh.ustate;
+          sh.ustate = old * kPcgMult + kHostInc;
           const unsigned long long u = pcg_output(old) >> 9;
           unsigned long long delta = udiv_fp64(P, (unsigned long long)N);
           if (delta == 0ull) delta = 1ull;
@@ -818,7 +844,7 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
         if (!(xT < 0x1p22f)) err = 1.0f;
         const float err_hi = 1.0f - err;
         const int q0 = j0 < N ? ct.q : N, Kq = 0x4AFFFFFF - q0;
-        unsigned short* lst = a.g_list ? a.g_list + (size_t)t * maxn : nullptr;
+        unsigned short* lst = TAPE ? a.g_list + (size_t)t * maxn : nullptr;
         // the next gather region that starts at or after the chunk's first child slot
         int rg = (q0 + region - 1) / region, rslot = rg * region;
         float lf = 0.0f;
@@ -829,33 +855,36 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
           bool rc[4], any = false;
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int i = 4 * g + e;
-            lf += i < nl ? tile_weight(Wt[q0a ^ i]) : 0.0f;
+            lf += tile_weight(Wt[q0a ^ (4 * g + e)]);
             const float xx = fmaf(lf, invDw, -R0x);
             const float fl = floorf(xx);
             const float fr = xx - fl;                      // exact
-            rc[e] = !none && !(fr > err && fr < err_hi);
+            rc[e] = !(fr > err && fr < err_hi);
             any |= rc[e];
-            qq[e] = none ? q0 : min(max(__float_as_int(fl + 0x1p23f) - Kq, q0), N);
+            qq[e] = min(max(__float_as_int(fl + 0x1p23f) - Kq, q0), N);
           }
+          if (none) { any = false; qq[0] = qq[1] = qq[2] = qq[3] = q0; }
           if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              if (rc[e]) qq[e] = min(q0 + exact_count_chunk(Wt, q0a, min(4 * g + e + 1, nl), R0, D, N), N);
+              if (any && rc[e]) qq[e] = min(q0 + exact_count_chunk(Wt, q0a, 4 * g + e + 1, R0, D, N), N);
           }
+          const int jm = j0 + 4 * g + 1;
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int i = 4 * g + e;
-            if (lst) lst[i * NT + tid] = (unsigned short)(i < nl ? qp : N);   // children of j start at slot qp
-            if (qq[e] > qp) {
-              marks[qp] = (unsigned short)(j0 + i + 1);
-              while (rslot < qq[e]) {                      // the ancestor of a region's first slot
-                if (rg < W) sh.carry_mark[rg] = (unsigned)(j0 + i + 1);
-                ++rg; rslot += region;
-              }
+            const int b0 = e ? qq[e - 1] : qp;
+            if (TAPE) {                                    // children of j start at b0 (rows in the backward's chunk order)
+              const int j = j0 + 4 * g + e;
+              if (j < N) lst[(j & (lchunk - 1)) * NT + (j >> llog)] = (unsigned short)b0;
             }
-            qp = qq[e];
+            if (qq[e] > b0) marks[mark_pos(b0)] = (unsigned short)(jm + e);
           }
+          while (rslot < qq[3]) {                          // the ancestor of a region's first slot (rare)
+            const int e = (qq[0] <= rslot) + (qq[1] <= rslot) + (qq[2] <= rslot);
+            if (rg < W) sh.carry_mark[rg] = (unsigned)(jm + e);
+            ++rg; rslot += region;
+          }
+          qp = qq[3];
         }
       }
       __syncthreads();
@@ -865,7 +894,7 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
         unsigned last = rs < N ? sh.carry_mark[warp] : 0u;
         for (int o0 = rs; o0 < re; o0 += 128) {
           const int o = o0 + 4 * lane;
-          const uint2 mv = o < re ? *reinterpret_cast<const uint2*>(marks + o) : make_uint2(0u, 0u);
+          const uint2 mv = o < re ? *reinterpret_cast<const uint2*>(marks + mark_pos(o)) : make_uint2(0u, 0u);
           unsigned am[4];
           am[0] = mv.x & 0xffffu;
           am[1] = max(am[0], mv.x >> 16);
@@ -884,6 +913,7 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
             }
           }
         }
+        if (N + tid < npad) Wt[swz(N + tid)] = 0.0f;       // the last group's slots past N
       }
       __syncthreads();
       float* tmp = H; H = Wt; Wt = tmp;
@@ -896,16 +926,15 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, const Batc
     if (sh.carry)
       for (int i = tid; i < N; i += NT) a.st_w[soff + i] = Wt[swz(i)];
   }
-  if (tid == kLogTid) { sh.fin_ll = ll_total; sh.fin_logS = logS_prev; sh.hm_last = hm_last; }
   __syncthreads();
   if (tid == 0) {
-    a.loglik[b] = sh.fin_ll;
+    a.loglik[b] = sh.ll_total;
     a.h_final[b] = sh.hm_last;
-    a.resamples[b] = n_res;
+    a.resamples[b] = sh.n_res;
     if (fs) {
       BatchFilterState r;
-      r.logS_prev = sh.fin_logS; r.ll_total = sh.fin_ll; r.ustate = ustate;
-      r.carry = sh.carry; r.n_res = n_res; r.hm_last = sh.hm_last; r.pad = 0;
+      r.logS_prev = sh.logS_prev; r.ll_total = sh.ll_total; r.ustate = sh.ustate;
+      r.carry = sh.carry; r.n_res = sh.n_res; r.hm_last = sh.hm_last; r.pad = 0;
       for (int k = 0; k < kBatchMaxTiles; ++k) r.carry_off[k] = sh.carry_off[k];
       *fs = r;
     }
@@ -933,9 +962,10 @@ __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_fas
     __syncthreads();
     if (idx >= a.n_order) break;
     const int b = a.order[idx];
-    const BatchFilterDev f = a.filters[b];
-    if (f.nu > 0.0f) batch_fast_filter<NT, EPT, false>(a, f, b, bufA, bufB, marks, sh, maxn);
-    else batch_fast_filter<NT, EPT, true>(a, f, b, bufA, bufB, marks, sh, maxn);
+    if (threadIdx.x == 0) sh.f = a.filters[b];
+    __syncthreads();
+    if (sh.f.nu > 0.0f) batch_fast_filter<NT, EPT, false, false>(a, b, bufA, bufB, marks, sh, maxn);
+    else batch_fast_filter<NT, EPT, true, false>(a, b, bufA, bufB, marks, sh, maxn);
   }
   step_epilogue(a);
 }
@@ -948,14 +978,40 @@ constexpr int kBatchHeavy = 32;   // children above which a parent's walk is sha
 
 
 template <int NT>
-__device__ void batch_run_backward(const BatchArgs& a, const BatchFilterDev& f, int b, int maxn, float* lam,
-                                   float* hA, float* hB, BatchShared<NT>& sh) {
+__device__ __forceinline__ void batch_grad_store(const BatchArgs& a, const BatchFilterDev& f, int b, const double (&acc)[5],
+                                                 double (&gred)[5][NT / 32]) {
   constexpr int W = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // per-filter sums -> gradient (initial draw h_0 = mu + sigma z / sqrt(max(1-rho^2, 1e-6)))
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const double v = warp_sum_d(acc[k]);
+    if (lane == 0) gred[k][warp] = v;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    double tt[5];
+    for (int k = 0; k < 5; ++k) {
+      tt[k] = 0.0;
+      for (int w = 0; w < W; ++w) tt[k] += gred[k][w];
+    }
+    const double r = (double)f.rho, sg = (double)f.sigma;
+    const double one_m = 1.0 - r * r;
+    const double s2 = fmax(one_m, 1e-6), sd = sqrt(s2);
+    const double ds_drho = one_m > 1e-6 ? sg * r / (s2 * sd) : 0.0;
+    a.grad[3 * (size_t)b + 0] = (1.0 - r) * tt[0] + tt[3];
+    a.grad[3 * (size_t)b + 1] = tt[1] + tt[4] * ds_drho;
+    a.grad[3 * (size_t)b + 2] = tt[2] + tt[4] / sd;
+  }
+  __syncthreads();
+}
+
+template <int NT>
+__device__ void batch_run_backward(const BatchArgs& a, const BatchFilterDev& f, int b, int maxn, int chunk, float* lam,
+                                   float* hA, float* hB, double (&gred)[5][NT / 32]) {
+  const int tid = threadIdx.x, lane = tid & 31;
   const int N = f.n, T = a.T, K = a.g_K;
-  int chunk = 1;
-  while (chunk * NT < N) chunk <<= 1;
-  const int j0 = tid * chunk;
+  const int j0 = tid * chunk;                  // the tape's parents of this thread: j0 .. j0 + chunk - 1
   const bool gauss = !(f.nu > 0.0f);
   ObsModel obs;
   obs.y = 0.0f; obs.nu = f.nu; obs.c_obs = f.c_obs; obs.inv_nu = f.inv_nu; obs.nu_p1h = f.nu_p1h;
@@ -1100,28 +1156,208 @@ __device__ void batch_run_backward(const BatchArgs& a, const BatchFilterDev& f, 
       __syncthreads();                     // lambda_t complete
     }
   }
-  // 4. per-filter sums -> gradient (initial draw h_0 = mu + sigma z / sqrt(max(1-rho^2, 1e-6)))
+  batch_grad_store<NT>(a, f, b, acc, gred);
+}
+
+// The adjoint backward of a filter of the unrolled shapes: batch_run_backward's operations and sums in
+// its order, arranged so that nothing expensive diverges. There a thread drew each child's noise while
+// it walked its parents' children, one parent after another with the list entries fetched in between:
+// a warp waits for its longest run, about four children where the mean is one. Here the noise of all
+// slots is formed slot by slot beforehand (into the array that is free at the time), a walk only adds
+// two values per child, list entries are fetched ahead, and lambda_t takes the place of h_t at once.
+template <int NT, int EPT, bool GAUSS>
+__device__ __forceinline__ void batch_fast_backward(const BatchArgs& a, const BatchFilterDev& f, int b, int maxn, float* lam,
+                                                    float* hA, float* hB, double (&gred)[5][NT / 32]) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int N = f.n, T = a.T, K = a.g_K;
+  int chunk = 1;
+  while (chunk * NT < N) chunk <<= 1;
+  const int j0 = tid * chunk;                  // chunk consecutive parents: j0 + e at q0a ^ e
+  const int q0a = swz(j0 < maxn ? j0 : 0);
+  const PcgTick pc0 = pcg_tick_consts(f.seed, 1ull, 0ull);
+  const int p0 = (tid & ~31) | ((lane ^ warp) & 31);
+  auto at = [&](int m) { return (p0 ^ (((NT / 32) * m) & 31)) + NT * m; };   // swz(tid + NT m)
+  double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  // The thread's parents in order, four at a time with the next four's list entries on the way:
+  // body(e, lo, hi) gets parent j0 + e and its children [lo, hi).
+  auto each_parent = [&](const unsigned short* lst, auto body) {
+    auto entry = [&](int e) {
+      int v = N;
+      if (e < chunk) {
+        if (j0 + e < N) v = (int)lst[e * NT + tid];
+      } else if (e == chunk) {
+        if (tid + 1 < NT && j0 + chunk < N) v = (int)lst[tid + 1];
+      }
+      return min(v, N);
+    };
+    int fc[4], nx[4];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    const double v = warp_sum_d(acc[k]);
-    if (lane == 0) sh.gred[k][warp] = v;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double tt[5];
-    for (int k = 0; k < 5; ++k) {
-      tt[k] = 0.0;
-      for (int w = 0; w < W; ++w) tt[k] += sh.gred[k][w];
+    for (int e = 0; e < 4; ++e) fc[e] = entry(e);
+#pragma unroll 1
+    for (int g = 0; 4 * g < chunk; ++g) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) nx[e] = entry(4 * g + 4 + e);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int lo = fc[e], hi = e < 3 ? fc[e < 3 ? e + 1 : 3] : nx[0];
+        if (4 * g + e < chunk) body(4 * g + e, lo, max(lo, hi));     // (chunk is the same for the whole CTA)
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) fc[e] = nx[e];
     }
-    const double r = (double)f.rho, sg = (double)f.sigma;
-    const double one_m = 1.0 - r * r;
-    const double s2 = fmax(one_m, 1e-6), sd = sqrt(s2);
-    const double ds_drho = one_m > 1e-6 ? sg * r / (s2 * sd) : 0.0;
-    a.grad[3 * (size_t)b + 0] = (1.0 - r) * tt[0] + tt[3];
-    a.grad[3 * (size_t)b + 1] = tt[1] + tt[4] * ds_drho;
-    a.grad[3 * (size_t)b + 2] = tt[2] + tt[4] / sd;
+  };
+  // noise of slot tid + NT m at the tick of pc, for every m in turn
+  auto each_noise = [&](const PcgTick& pc, auto use) {
+    uint64_t sx = pc.k1 + pc.k2 * pcg_inc((uint32_t)tid);
+    const uint64_t step = (uint64_t)(2 * NT) * pc.k2;
+#pragma unroll
+    for (int m = 0; m < EPT; ++m) {
+      if (NT * m >= N) continue;                       // the same for the whole CTA
+      float z = icdf_normal_warp(pcg_uniform(pcg_output(sx)));
+      if (f.nu_int > 0) z *= tstate_scale_warp(sx, pc.k2 << 33, f.nu_int, f.nu_state);
+      use(m, z);
+      sx += step;
+    }
+  };
+
+  const int nseg = (T + K - 1) / K;
+  for (int s = nseg - 1; s >= 0; --s) {
+    const int c = s * K, last = min(c + K, T) - 1;
+    // 1. particles of tick c from the checkpoint
+    {
+      const float* ck = a.g_ckpt + (size_t)s * maxn;
+      const PcgTick pc = pcg_tick_consts(f.seed, a.g_AB[c].x, a.g_AB[c].y);
+      if (c > 0) {
+        each_noise(pc, [&](int m, float z) {
+          const int i = tid + NT * m;
+          if (i < N) hA[at(m)] = propagate(ck[i], f.mu, f.rho, f.sigma, z);
+        });
+      } else {
+        for (int i = tid; i < N; i += NT) hA[swz(i)] = ck[i];
+      }
+      if (last > c)
+        for (int i = tid; i < N; i += NT) a.g_seg[i] = hA[swz(i)];
+    }
+    __syncthreads();
+    float* hp = hA;
+    float* hc = hB;
+    // 2. ticks c+1..last: every parent's particle to its children's slots, then slot by slot
+    for (int t = c + 1; t <= last; ++t) {
+      const PcgTick pc = pcg_tick_consts(f.seed, a.g_AB[t].x, a.g_AB[t].y);
+      each_parent(a.g_list + (size_t)(t - 1) * maxn, [&](int e, int lo, int hi) {
+        const float hpar = hp[q0a ^ e];
+        const bool light = hi - lo <= kBatchHeavy;
+        if (light)
+          for (int i = lo; i < hi; ++i) hc[swz(i)] = hpar;
+        unsigned heavy = __ballot_sync(0xffffffffu, !light);
+        while (heavy) {
+          const int src = __ffs(heavy) - 1;
+          heavy &= heavy - 1u;
+          const int flo = __shfl_sync(0xffffffffu, lo, src), fhi = __shfl_sync(0xffffffffu, hi, src);
+          const float fh = __shfl_sync(0xffffffffu, hpar, src);
+          for (int i = flo + lane; i < fhi; i += 32) hc[swz(i)] = fh;
+        }
+      });
+      __syncthreads();
+      float* sg = t < last ? a.g_seg + (size_t)(t - c) * maxn : nullptr;
+      each_noise(pc, [&](int m, float z) {
+        const int i = tid + NT * m;
+        if (i < N) {
+          const float h = propagate(hc[at(m)], f.mu, f.rho, f.sigma, z);
+          hc[at(m)] = h;
+          if (sg) sg[i] = h;
+        }
+      });
+      __syncthreads();
+      float* tmp = hp; hp = hc; hc = tmp;
+    }
+    // 3. adjoint, ticks last..c (hp holds h_last)
+    for (int t = last; t >= c; --t) {
+      if (t < last) {
+        const float* sg = a.g_seg + (size_t)(t - c) * maxn;
+        for (int i = tid; i < N; i += NT) hp[swz(i)] = sg[i];
+      }
+      const bool inner = t < T - 1;
+      const unsigned short* lst = a.g_list + (size_t)t * maxn;
+      if (inner) {
+        const PcgTick pcn = pcg_tick_consts(f.seed, a.g_AB[t + 1].x, a.g_AB[t + 1].y);
+        each_noise(pcn, [&](int m, float z) { if (tid + NT * m < N) hc[at(m)] = z; });
+      }
+      __syncthreads();                     // the noise of tick t + 1 and h_t in place
+      const float2 nz = a.g_norm[t];
+      const float invS = nz.x, nM = (float)__float_as_int(nz.y);
+      const float y = __ldg(a.y + t), y2 = y * y;
+      ObsModel obs;
+      obs.y = y; obs.nu = f.nu; obs.c_obs = f.c_obs; obs.inv_nu = f.inv_nu; obs.nu_p1h = f.nu_p1h;
+      float acc_eps = 0.0f, acs = 0.f, acsh = 0.f, al0 = 0.f, al0z = 0.f;
+      // lambda_t of parent j0 + e from its children sum, in the place of its particle (read by this
+      // thread alone)
+      auto adjoint = [&](int e, float cs) {
+        const int j = j0 + e;
+        if (j >= N) return;
+        const float h = hp[q0a ^ e];
+        float x, g;
+        if (GAUSS) {
+          x = obs_log2pdf_gauss(y2, h);
+          g = 0.5f * fmaf(y2, ex2_approx(h * -kLog2e), -1.0f);
+        } else {
+          x = obs_log2pdf_t_plus(obs, __fmul_rn(y2, obs.inv_nu), h, __fmul_rn(obs.c_obs, kLog2e));
+          const float q = y2 * ex2_approx(h * -kLog2e) * obs.inv_nu;
+          g = fmaf(obs.nu_p1h, div_approx(q, 1.0f + q), -0.5f);
+        }
+        const float l = fmaf(f.rho, cs, (ex2_approx(x - nM) * invS) * g);
+        hp[q0a ^ e] = l;
+        acs += cs;
+        acsh = fmaf(cs, h - f.mu, acsh);
+        if (t == 0) {
+          const float z0 = state_noise(pc0, (uint32_t)j, 0, 0.0f);
+          al0 += l;
+          al0z = fmaf(l, z0, al0z);
+        }
+      };
+      if (inner) {
+        // children sums of lambda_t+1, and sum lambda eps over the children
+        each_parent(lst, [&](int e, int lo, int hi) {
+          float sum = 0.0f;
+          const bool light = hi - lo <= kBatchHeavy;
+          if (light) {
+            for (int i = lo; i < hi; ++i) {
+              const int si = swz(i);
+              const float l = lam[si];
+              sum += l;
+              acc_eps = fmaf(l, hc[si], acc_eps);
+            }
+          }
+          unsigned heavy = __ballot_sync(0xffffffffu, !light);
+          while (heavy) {
+            const int src = __ffs(heavy) - 1;
+            heavy &= heavy - 1u;
+            const int flo = __shfl_sync(0xffffffffu, lo, src), fhi = __shfl_sync(0xffffffffu, hi, src);
+            float p = 0.0f;
+            for (int i = flo + lane; i < fhi; i += 32) {
+              const int si = swz(i);
+              const float l = lam[si];
+              p += l;
+              acc_eps = fmaf(l, hc[si], acc_eps);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+            if (lane == src) sum = p;
+          }
+          adjoint(e, sum);
+        });
+      } else {
+        for (int e = 0; e < chunk; ++e) adjoint(e, 0.0f);
+      }
+      acc[0] += (double)acs; acc[1] += (double)acsh; acc[2] += (double)acc_eps;
+      acc[3] += (double)al0; acc[4] += (double)al0z;
+      __syncthreads();                     // lambda_t complete, lambda_t+1 fully read
+      float* tmp = lam; lam = hp; hp = tmp;
+    }
+    hA = hp;                               // the two arrays that the next segment starts with
+    hB = hc;
   }
-  __syncthreads();
+  batch_grad_store<NT>(a, f, b, acc, gred);
 }
 
 size_t batch_grad_smem_bytes(int maxn) { return (size_t)maxn * 12; }
@@ -1176,10 +1412,12 @@ cudaError_t launch_noise_gather(float* nz, const long long* src_off, const long 
   return cudaGetLastError();
 }
 
-template <int NT>
+// EPT: the unrolled forward (its list rows hold EPT NT = maxn entries), 0: the generic one.
+template <int NT, int EPT>
 __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_grad_kernel(BatchArgs a, int maxn) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ BatchShared<NT> sh;
+  __shared__ typename std::conditional<EPT == 0, BatchShared<NT>, BatchFastShared<NT>>::type sh;
+  __shared__ double gred[5][NT / 32];
   float* r0 = reinterpret_cast<float*>(smem);
   float* r1 = r0 + maxn;
   float* r2 = r1 + maxn;
@@ -1198,8 +1436,22 @@ __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_gra
     if (idx >= a.n_order) break;
     const int b = a.order[idx];
     const BatchFilterDev f = a.filters[b];
-    batch_run_filter<NT, false>(s, f, b, r0, r1, marks, sh, maxn);
-    batch_run_backward<NT>(s, f, b, maxn, r0, r1, r2, sh);
+    [[maybe_unused]] int chunk = 1;
+    if constexpr (EPT == 0) {
+      while (chunk * NT < f.n) chunk <<= 1;
+      batch_run_filter<NT, false>(s, f, b, r0, r1, marks, sh, maxn);
+    } else {
+      if (threadIdx.x == 0) sh.f = f;
+      __syncthreads();
+      if (f.nu > 0.0f) batch_fast_filter<NT, EPT, false, true>(s, b, r0, r1, marks, sh, maxn);
+      else batch_fast_filter<NT, EPT, true, true>(s, b, r0, r1, marks, sh, maxn);
+    }
+    if constexpr (EPT == 0) {
+      batch_run_backward<NT>(s, f, b, maxn, chunk, r0, r1, r2, gred);
+    } else {
+      if (f.nu > 0.0f) batch_fast_backward<NT, EPT, false>(s, sh.f, b, maxn, r0, r1, r2, gred);
+      else batch_fast_backward<NT, EPT, true>(s, sh.f, b, maxn, r0, r1, r2, gred);
+    }
   }
 }
 
@@ -1249,9 +1501,18 @@ static int occ_nt(int maxn) {
   return per;
 }
 
+template <int NT, class F>
+static void with_grad_kernel(int maxn, F f) {
+  const int ept = batch_ept(NT, maxn);
+  if (ept * NT != maxn) f(batch_grad_kernel<NT, 0>);
+  else if (ept == 4) f(batch_grad_kernel<NT, 4>);
+  else if (ept == 8) f(batch_grad_kernel<NT, 8>);
+  else f(batch_grad_kernel<NT, 16>);
+}
+
 template <int NT>
 static cudaError_t launch_grad_nt(const BatchArgs& a, int maxn, int grid, cudaStream_t s) {
-  batch_grad_kernel<NT><<<grid, NT, batch_grad_smem_bytes(maxn), s>>>(a, maxn);
+  with_grad_kernel<NT>(maxn, [&](auto k) { k<<<grid, NT, batch_grad_smem_bytes(maxn), s>>>(a, maxn); });
   return cudaGetLastError();
 }
 
@@ -1269,9 +1530,11 @@ cudaError_t launch_batch_grad_class(const BatchArgs& a, int threads, int maxn, i
 template <int NT>
 static int grad_occ_nt(int maxn) {
   const size_t smem = batch_grad_smem_bytes(maxn);
-  cudaFuncSetAttribute(batch_grad_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_grad_kernel<NT>, NT, smem);
+  with_grad_kernel<NT>(maxn, [&](auto k) {
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, NT, smem);
+  });
   return per;
 }
 
