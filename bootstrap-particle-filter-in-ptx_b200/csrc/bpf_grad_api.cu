@@ -93,6 +93,12 @@ struct GpuBpfGrad {
   float2* aux = nullptr;             // [T_max]
   BpfTickRecord* rec = nullptr;      // [T_max]
   float* seg = nullptr;              // [K][N4]
+  // Every tick's particles of a resident forward run, [T_max][G*4096]: with them the backward is one
+  // kernel per tick and recomputes nothing (N = 2^20 16.7 -> 10.2 us per tick). Allocated by the first
+  // such run of a tape with the default checkpoint interval, where an eighth of the free memory holds
+  // them; without them the checkpoints serve.
+  float* hist = nullptr;
+  bool default_k = false, hist_tried = false;
   float* lam[2] = {nullptr, nullptr};
   double* acc = nullptr;             // [G1][kGradAcc]
 
@@ -120,7 +126,7 @@ void free_grad(GpuBpfGrad* g) {
   if (g->fgraph) cudaGraphExecDestroy(g->fgraph);
   if (g->bgraph) cudaGraphExecDestroy(g->bgraph);
   plan_free(g->plan);
-  bpf_free(g->csr); bpf_free(g->ckpt); bpf_free(g->aux); bpf_free(g->rec); bpf_free(g->seg);
+  bpf_free(g->csr); bpf_free(g->ckpt); bpf_free(g->aux); bpf_free(g->rec); bpf_free(g->seg); bpf_free(g->hist);
   bpf_free(g->lam[0]); bpf_free(g->lam[1]); bpf_free(g->acc);
   bpf_free(g->rs[0]); bpf_free(g->rs[1]); bpf_free(g->part); bpf_free(g->per_tick); bpf_free(g->rtotal);
   if (g->stream) cudaStreamDestroy(g->stream);
@@ -156,6 +162,7 @@ cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
     tape.ckpt = g->ckpt; tape.ckpt_stride = g->ckpt_stride;
     tape.K = g->K;
     tape.aux = g->aux;
+    tape.hist = g->hist;
     e = launch_resident(g->plan, a, tape, false, k.T, g->res_tiles, g->stream);
   }
   for (int t = 0; t < k.T && e == cudaSuccess && !g->resident; ++t) {
@@ -186,13 +193,15 @@ cudaError_t enqueue_backward(GpuBpfGrad* g, const BwdKey& bk) {
   const ObsModel obs = make_obs(k.nu);
   const int nui = nu_int_of(k.nu_state);
   cudaError_t e = cudaMemsetAsync(g->acc, 0, (size_t)g->G1 * kGradAcc * sizeof(double), g->stream);
+  const bool kept = g->hist && g->resident;      // every tick's particles are on the tape
   const int nseg = (T + K - 1) / K;
   for (int s = nseg - 1; s >= 0 && e == cudaSuccess; --s) {
     const int c = s * K, last = std::min(c + K, T) - 1;
     // recompute h_c .. h_last into seg[0 .. last-c]
-    e = launch_grad_seed(N, g->ckpt + (size_t)s * g->ckpt_stride, g->seg, g->pcs[c], c > 0 ? 1 : 0, k.mu, k.rho,
+    if (!kept)
+      e = launch_grad_seed(N, g->ckpt + (size_t)s * g->ckpt_stride, g->seg, g->pcs[c], c > 0 ? 1 : 0, k.mu, k.rho,
                          k.sigma, nui, k.nu_state, g->stream, g->pdl);
-    for (int t = c + 1; t <= last && e == cudaSuccess; ++t)
+    for (int t = c + 1; t <= last && e == cudaSuccess && !kept; ++t)
       e = launch_grad_recompute(N, g->csr + (size_t)(t - 1) * g->N4, g->seg + (size_t)(t - 1 - c) * g->N4,
                                 g->seg + (size_t)(t - c) * g->N4, g->pcs[t], k.mu, k.rho, k.sigma, nui,
                                 k.nu_state, g->stream, g->pdl);
@@ -203,7 +212,7 @@ cudaError_t enqueue_backward(GpuBpfGrad* g, const BwdKey& bk) {
       a.mu = k.mu; a.rho = k.rho; a.sigma = k.sigma;
       a.obs = obs;
       a.y = k.y + t;
-      a.h = g->seg + (size_t)(t - c) * g->N4;
+      a.h = kept ? g->hist + (size_t)t * g->ckpt_stride : g->seg + (size_t)(t - c) * g->N4;
       a.csr = (t < T - 1) ? g->csr + (size_t)t * g->N4 : nullptr;
       a.lam_next = (t < T - 1) ? g->lam[(t + 1) & 1] : nullptr;
       a.lam = g->lam[t & 1];
@@ -278,6 +287,7 @@ GpuBpfGrad* gpu_bpf_grad_create(int n_particles, int max_ticks, int checkpoint_e
   g->N4 = grad_stride(n_particles);
   g->T_max = max_ticks;
   g->K = checkpoint_every > 0 ? checkpoint_every : kDefaultCheckpoint;
+  g->default_k = checkpoint_every == 0;
   g->n_ckpt = (max_ticks + g->K - 1) / g->K;
   if (const char* v = std::getenv("BPF_DISABLE_PDL")) g->pdl = (v[0] == '0');
   if ((e = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
@@ -325,6 +335,17 @@ int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, floa
   k.T = n_ticks; k.seed = seed; k.mu = mu; k.rho = rho; k.sigma = sigma_z; k.nu = nu_obs; k.nu_state = nu_state;
   k.y = y_dev; k.ll = loglik_dev;
   g->resident = resident_ready(g->device, g->plan.G, g->res_tiles, nu_int_of(nu_state) > 0, !(nu_obs > 0.0f), false);
+  if (g->resident && g->default_k && !g->hist_tried) {
+    g->hist_tried = true;
+    const size_t bytes = (size_t)g->T_max * g->ckpt_stride * sizeof(float);
+    size_t free_b = 0, total_b = 0;
+    GCK(cudaMemGetInfo(&free_b, &total_b));
+    if (bytes <= free_b / 8 && bpf_malloc(&g->hist, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      g->hist = nullptr;
+    }
+    if (g->hist && g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }
+  }
   if (!g->fgraph || !(g->fkey == k)) {
     GCK(capture(g, &g->fgraph, [&]() { return enqueue_forward(g, k); }));
     g->fkey = k;

@@ -136,6 +136,7 @@ struct ResidentTape {        // gradient tape of a taped run from tick 0 (all nu
   float* ckpt; size_t ckpt_stride;     // particles entering every K-th tick
   int K;
   float2* aux;                         // {1/S, nM} per tick
+  float* hist;                         // every tick's particles as weighted, at hist + t * ckpt_stride, or null
 };
 constexpr int kResMaxTilesPerCta = 4;
 size_t resident_xbuf_bytes(int G);

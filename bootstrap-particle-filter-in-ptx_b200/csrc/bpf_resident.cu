@@ -324,6 +324,8 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
             x[q][4 * rr + e] = xx;
           }
           if (!APF || stage != 1) st4(sh.h[j], l0, make_float4(hh[0], hh[1], hh[2], hh[3]));
+          if (tape.hist)
+            *reinterpret_cast<float4*>(tape.hist + (size_t)tick * tape.ckpt_stride + tile0 + l0) = make_float4(hh[0], hh[1], hh[2], hh[3]);
         }
         if (tile0 + kTile > N) {                     // padding slots carry no weight
 #pragma unroll

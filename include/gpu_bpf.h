@@ -475,7 +475,10 @@ long long    gpu_bpf_batch_noise_offset(GpuBpfBatch* batch, int filter, int n_ti
 typedef struct GpuBpfGrad GpuBpfGrad;
 
 /* Tape for up to max_ticks ticks of n_particles (checkpoint_every 0 = 16). NULL on error.
- * Device memory: gpu_bpf_grad_tape_bytes() (about 4 * n_particles * max_ticks bytes). */
+ * Device memory: gpu_bpf_grad_tape_bytes() (about 4 * n_particles * max_ticks bytes). With
+ * checkpoint_every 0 the first forward run also keeps every tick's particles where an eighth of
+ * the free device memory holds them (as much again; the backward pass then recomputes nothing);
+ * a checkpoint interval of the caller's choice never takes more. */
 GpuBpfGrad* gpu_bpf_grad_create(int n_particles, int max_ticks, int checkpoint_every);
 void        gpu_bpf_grad_destroy(GpuBpfGrad* grad);
 size_t      gpu_bpf_grad_tape_bytes(int n_particles, int max_ticks, int checkpoint_every);

@@ -133,3 +133,18 @@ def test_resident_tape_matches_plain_ticks(bpf, N):
     assert np.max(np.abs(g - ref)) <= 1e-4 * np.max(np.abs(ref))     # the gradient tests' bound
     f.close()
     tape.close()
+
+
+@pytest.mark.parametrize("N", [5, 70001, 700001])
+def test_resident_tape_with_and_without_kept_particles(bpf, N):
+    """The default tape keeps every tick's particles, one with an interval recomputes them: equal bits."""
+    import torch
+    T = 37
+    y = torch.tensor(_series(T, 6, True), device="cuda")
+    out = []
+    for every in (0, 16, 5):
+        tape = bpf.GradTape(N, T, checkpoint_every=every)
+        for seed in (3, 9):
+            out.append((tape.forward((MU, RHO, SIG), y, seed=seed).item(), tape.backward().cpu().numpy().tobytes()))
+        tape.close()
+    assert out[0:2] == out[2:4] == out[4:6]
