@@ -673,6 +673,7 @@ __device__ __forceinline__ void batch_fast_filter(const BatchArgs& a, int b, flo
               H[si] = h;
               s += step;
             }
+            if (TAPE && a.g_hist) a.g_hist[(size_t)t * maxn + tid + NT * m] = h;
             float v = GAUSS ? obs_log2pdf_gauss_plus(y2, h, gc) : obs_log2pdf_t_plus(obs, y2nu, h, tc);
             if (carry) v += Wt[si];                      // carried tile-relative log2-weight
             x[m] = NT * m < lim ? v : -INFINITY;
@@ -1220,11 +1221,12 @@ __device__ __forceinline__ void batch_fast_backward(const BatchArgs& a, const Ba
     }
   };
 
-  const int nseg = (T + K - 1) / K;
+  const bool kept = a.g_hist != nullptr;       // every tick's particles are on the tape: one segment, nothing recomputed
+  const int nseg = kept ? 1 : (T + K - 1) / K;
   for (int s = nseg - 1; s >= 0; --s) {
-    const int c = s * K, last = min(c + K, T) - 1;
+    const int c = s * K, last = kept ? T - 1 : min(c + K, T) - 1;
     // 1. particles of tick c from the checkpoint
-    {
+    if (!kept) {
       const float* ck = a.g_ckpt + (size_t)s * maxn;
       const PcgTick pc = pcg_tick_consts(f.seed, a.g_AB[c].x, a.g_AB[c].y);
       if (c > 0) {
@@ -1242,7 +1244,7 @@ __device__ __forceinline__ void batch_fast_backward(const BatchArgs& a, const Ba
     float* hp = hA;
     float* hc = hB;
     // 2. ticks c+1..last: every parent's particle to its children's slots, then slot by slot
-    for (int t = c + 1; t <= last; ++t) {
+    for (int t = c + 1; t <= last && !kept; ++t) {
       const PcgTick pc = pcg_tick_consts(f.seed, a.g_AB[t].x, a.g_AB[t].y);
       each_parent(a.g_list + (size_t)(t - 1) * maxn, [&](int e, int lo, int hi) {
         const float hpar = hp[q0a ^ e];
@@ -1273,9 +1275,11 @@ __device__ __forceinline__ void batch_fast_backward(const BatchArgs& a, const Ba
     }
     // 3. adjoint, ticks last..c (hp holds h_last)
     for (int t = last; t >= c; --t) {
-      if (t < last) {
-        const float* sg = a.g_seg + (size_t)(t - c) * maxn;
-        for (int i = tid; i < N; i += NT) hp[swz(i)] = sg[i];
+      if (t < last || kept) {
+        const float* sg = kept ? a.g_hist + (size_t)t * maxn : a.g_seg + (size_t)(t - c) * maxn;
+#pragma unroll
+        for (int m = 0; m < EPT; ++m)
+          if (tid + NT * m < N) hp[at(m)] = sg[tid + NT * m];
       }
       const bool inner = t < T - 1;
       const unsigned short* lst = a.g_list + (size_t)t * maxn;
@@ -1428,6 +1432,7 @@ __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_gra
   s.g_ckpt = a.g_ckpt + (size_t)blockIdx.x * nck * maxn;
   s.g_norm = a.g_norm + (size_t)blockIdx.x * a.T;
   s.g_seg = a.g_seg + (size_t)blockIdx.x * a.g_K * maxn;
+  if (a.g_hist) s.g_hist = a.g_hist + (size_t)blockIdx.x * a.T * maxn;
   for (;;) {
     if (threadIdx.x == 0) sh.next = atomicAdd(a.counter, 1);
     __syncthreads();
@@ -1537,6 +1542,8 @@ static int grad_occ_nt(int maxn) {
   });
   return per;
 }
+
+bool batch_grad_keeps(int threads, int maxn) { return batch_ept(threads, maxn) * threads == maxn; }
 
 int batch_grad_occupancy(int threads, int maxn) {
   switch (threads) {

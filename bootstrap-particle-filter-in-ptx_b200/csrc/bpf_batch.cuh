@@ -64,6 +64,7 @@ struct BatchArgs {
   float2* g_norm;             // [slots][T] {1/S, nM}: W_i = 2^(x_i - nM) / S
   float* g_seg;               // [slots][K][maxn] recomputed particles of one checkpoint segment
   const ulonglong2* g_AB;     // [T+1] PCG32 jump constants (A^t, sum_{k<t} A^k)
+  float* g_hist;              // [slots][T][maxn] every tick's particles as weighted, or null (recomputed)
   int g_K;                    // checkpoint interval
   double* grad;               // [3B] d loglik / d(mu, rho, sigma_z)
   // resumable runs (all null for a run from tick 0 that keeps nothing)
@@ -111,6 +112,8 @@ int batch_occupancy(int threads, int maxn);
 size_t batch_grad_smem_bytes(int maxn);
 cudaError_t launch_batch_grad_class(const BatchArgs& a, int threads, int maxn, int grid, cudaStream_t s);
 int batch_grad_occupancy(int threads, int maxn);
+// Whether the gradient kernel of the shape can keep every tick's particles (BatchArgs::g_hist).
+bool batch_grad_keeps(int threads, int maxn);
 // Filter j of a correlated-noise buffer takes the first `floats` floats (a multiple of 4) of the
 // area at src_off[j] into the area at dst_off[j] (16-byte aligned areas that do not overlap).
 cudaError_t launch_noise_gather(float* nz, const long long* src_off, const long long* dst_off, long long floats,

@@ -34,7 +34,7 @@ void free_batch(GpuBpfBatch* b) {
   if (b->sgraph) cudaGraphExecDestroy(b->sgraph);
   bpf_free(b->d_st); bpf_free(b->d_sth); bpf_free(b->d_stw); bpf_free(b->d_stoff); bpf_free(b->d_tick);
   bpf_free(b->d_scounters);
-  for (int c = 0; c < kClasses; ++c) bpf_free(b->g_tape[c]);
+  for (int c = 0; c < kClasses; ++c) { bpf_free(b->g_tape[c]); bpf_free(b->g_hist[c]); }
   bpf_free(b->d_AB);
   bpf_free(b->d_nzoff);
   bpf_free(b->d_filters); bpf_free(b->d_order); bpf_free(b->d_counters);
@@ -140,6 +140,25 @@ int prepare_grad(GpuBpfBatch* b, int T) {
       b->g_tape_bytes[c] = need;
     }
   }
+  // the particles of every tick, for the classes that run the unrolled kernels
+  size_t want = 0, free_b = 0, total_b = 0;
+  auto hist_bytes = [&](int c) {
+    return batch_grad_keeps(b->threads[c], kClassMaxN[c]) && b->class_cnt[c]
+               ? (size_t)b->g_grid[c] * T * kClassMaxN[c] * sizeof(float) : (size_t)0;
+  };
+  for (int c = 0; c < kClasses; ++c) if (hist_bytes(c) > b->g_hist_bytes[c]) want += hist_bytes(c);
+  if (want) {
+    BCK(cudaMemGetInfo(&free_b, &total_b));
+    for (int c = 0; c < kClasses; ++c) {
+      if (hist_bytes(c) <= b->g_hist_bytes[c]) continue;
+      bpf_free(b->g_hist[c]);
+      b->g_hist[c] = nullptr;
+      b->g_hist_bytes[c] = 0;
+      if (want > free_b / 8) continue;
+      if (bpf_malloc(&b->g_hist[c], hist_bytes(c)) == cudaSuccess) b->g_hist_bytes[c] = hist_bytes(c);
+      else { cudaGetLastError(); b->g_hist[c] = nullptr; }
+    }
+  }
   if (b->ab_T < T + 1) {
     bpf_free(b->d_AB);
     b->d_AB = nullptr;
@@ -174,6 +193,9 @@ cudaError_t enqueue_grad(GpuBpfBatch* b, const float* y, int T, double* loglik, 
     a.g_ckpt = reinterpret_cast<float*>(base + slots * L.ckpt);
     a.g_norm = reinterpret_cast<float2*>(base + slots * L.norm);
     a.g_seg = reinterpret_cast<float*>(base + slots * L.seg);
+    if (batch_grad_keeps(b->threads[c], kClassMaxN[c]) &&
+        b->g_hist_bytes[c] >= slots * T * kClassMaxN[c] * sizeof(float))
+      a.g_hist = b->g_hist[c];
     a.g_AB = b->d_AB;
     a.g_K = kGradK;
     a.grad = grad;

@@ -435,7 +435,9 @@ double*      gpu_bpf_batch_loglik_device(GpuBpfBatch* batch);
 int          gpu_bpf_batch_grad_run(GpuBpfBatch* batch, const float* y_dev, int n_ticks, double* loglik_dev,
                                     double* grad_dev);
 /* Device memory the gradient tape of gpu_bpf_batch_grad_run takes for n_ticks ticks (it is sized
- * for the CTAs in flight, not for the number of filters). */
+ * for the CTAs in flight, not for the number of filters). Where an eighth of the free device
+ * memory holds them, every tick's particles are kept too (4 bytes per particle and tick of the
+ * filters in flight); the backward pass then recomputes nothing. */
 size_t       gpu_bpf_batch_grad_tape_bytes(GpuBpfBatch* batch, int n_ticks);
 /* Correlated-noise runs: the building block of correlated pseudo-marginal MCMC (CPMMH,
  * Deligiannidis, Doucet & Pitt 2018), as the reference's CPMMH rejuvenation kernel uses it
