@@ -181,6 +181,7 @@ TickArgs make_args(GpuBpfState* s, Impl* m, float y, const float* y_ptr, BpfTick
   TickArgs a{};
   a.mu = s->mu; a.rho = s->rho; a.sigma = s->sigma_z;
   a.ess_threshold = s->ess_threshold;
+  a.ess_bound = ess_keep_bound(s->ess_threshold, m->plan.N);
   a.log_n = std::log((double)m->plan.N);
   a.obs = m->obs;
   a.obs.y = y;

@@ -1385,7 +1385,7 @@ __device__ __forceinline__ void plan_fused(const TickArgs& a, int N, FusedShared
 // the decision left in sh.tail. The two parts together write what plan_decide writes, with the
 // same arithmetic.
 template <int NCTA>
-__device__ __forceinline__ void plan_fused_decide(const TickArgs& a, int N, FusedShared& sh, int par) {
+__device__ __forceinline__ void plan_fused_decide(const TickArgs& a, FusedShared& sh, int par) {
   const int lane = threadIdx.x & 31;
   int nM;
   double tS, tQ, tH;
@@ -1406,7 +1406,7 @@ __device__ __forceinline__ void plan_fused_decide(const TickArgs& a, int N, Fuse
     }
     tS = warp_sum_d(S); tQ = warp_sum_d(Q); tH = warp_sum_d(H);
   }
-  if (lane == 0) fused_decide(a, N, nM, tS, tQ, tH, &sh.st, sh.tail);
+  if (lane == 0) fused_decide(a, nM, tS, tQ, tH, &sh.st, sh.tail);
 }
 
 // The resampling plan into the device state (on a resampling tick).
@@ -1640,7 +1640,7 @@ small_kernel(Plan p, TickArgs a, int n_ticks) {
         marks_barrier_sync<NCTA>();               // every child is written
       }
     } else {
-      if (warp == 0) plan_fused_decide<NCTA>(a, N, sh, par);
+      if (warp == 0) plan_fused_decide<NCTA>(a, sh, par);
       else if (more) fused_noise<TSTATE>(a, tile0, sh.knext[0], sh.knext[1], 32, kSmallThreads - 32, sh);
       __syncthreads();
       if (sh.st.do_resample) {

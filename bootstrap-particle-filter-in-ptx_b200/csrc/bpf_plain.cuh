@@ -11,6 +11,7 @@
 //   items[G + N/8192 + 1] int4 pass-2 work items (tile, first out, end out, flags)
 //   DevState      scalars carried from tick to tick
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "bpf_alloc.cuh"
@@ -80,6 +81,7 @@ struct TickMirror {
 struct TickArgs {
   float mu, rho, sigma;
   float ess_threshold;
+  double ess_bound;          // ess_keep_bound(ess_threshold, N): the kernels that hold a filter on the chip compare with it
   double log_n;              // ln N
   ObsModel obs;              // obs.y is used when y_ptr == nullptr
   const float* y_ptr;        // device pointer to this tick's observation, or null
@@ -100,6 +102,17 @@ struct TickArgs {
   int tail_plan;             // the last pass-1 CTA runs the plan (G <= kTailTiles; no plan launch)
   float silverman;           // Silverman jitter shrink after resampling (0 = off; needs p.jpart)
 };
+
+// The smallest double x with x / n >= thr as the plan rounds the quotient (monotone in x), so that the
+// test ess / n < thr is the comparison ess < x.
+inline double ess_keep_bound(float thr, int n) {
+  const double t = (double)thr, d = (double)n;
+  double x = t * d;
+  if (!(x > 0.0) || std::isinf(x)) return x;
+  while (x / d >= t) x = std::nextafter(x, 0.0);
+  while (x / d < t) x = std::nextafter(x, INFINITY);
+  return x;
+}
 
 // Device buffers of a plan for N particles (G, max_items set; DevState included).
 cudaError_t plan_alloc(Plan& p, int N);

@@ -130,7 +130,6 @@ struct ResidentShared {
   unsigned long long pre[NT], mass[NT], P[NT];   // own tiles: prefix within their 32 tiles, mass, global prefix
   unsigned long long base, delta, magic;  // the tick's targets
   unsigned long long ustate;              // resampling-uniform PCG32
-  double ess_bound;                       // the smallest ESS that keeps the particles
   int wn[32];                             // frame of each 32 tiles
   int c0[NT], c1[NT];                     // own tiles' first output slots and their ends
   float smax[2][kResWarps];
@@ -140,17 +139,6 @@ struct ResidentShared {
   __align__(16) DevState st;
   FusedTail tail;
 };
-
-// The smallest double x with x / n >= thr as the plan rounds it (the quotient is monotone in x), so
-// that the decision is one comparison of the ESS.
-__device__ __noinline__ double ess_keep_bound(float thr, int n) {
-  const double t = (double)thr, d = (double)n;
-  double x = t * d;
-  if (!(x > 0.0) || isinf(x)) return x;
-  while (x / d >= t) x = __longlong_as_double(__double_as_longlong(x) - 1ll);
-  while (x / d < t) x = __longlong_as_double(__double_as_longlong(x) + 1ll);
-  return x;
-}
 
 // SPLIT threads share a pass-1 thread's sixteen particles; Q tiles per group of kThreads * SPLIT
 // threads: (2, 1) for one tile a CTA, (1, 1) for two, (1, 2) for three and four.
@@ -185,7 +173,6 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
 
   if (tid < (int)(sizeof(DevState) / 8))
     reinterpret_cast<unsigned long long*>(&sh.st)[tid] = __ldcg(reinterpret_cast<const unsigned long long*>(p.st) + tid);
-  if (tid == kResThreads - 32) sh.ess_bound = ess_keep_bound(a.ess_threshold, N);
   __syncthreads();
   if (tid == 0) sh.ustate = sh.st.u_state;
   int nk[Q];                                    // the tiles' exponents (previous tick's until pass 1 sets them)
@@ -247,10 +234,10 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
     BpfTickRecord* rec = (a.rec && apf_stage != 1) ? a.rec + t : nullptr;
     const int tk = sh.st.tick;
     if (APF && apf_stage == 1) {
-      fused_decide<1>(a, N, d_nM, dS, dQ, dH, &sh.st, sh.tail);
+      fused_decide<1>(a, d_nM, dS, dQ, dH, &sh.st, sh.tail);
       fused_finish<1>(sh.tail, &sh.st, nullptr);
     } else {
-      fused_decide<0>(a, N, d_nM, dS, dQ, dH, &sh.st, sh.tail);
+      fused_decide<0>(a, d_nM, dS, dQ, dH, &sh.st, sh.tail);
       if (APF && apf_stage == 2) fused_finish<2>(sh.tail, &sh.st, rec);
       else fused_finish<0>(sh.tail, &sh.st, rec);
     }
@@ -494,14 +481,9 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       }
       dS = tS; dQ = tQ; dH = tH; d_nM = nM;
       if (lane == 0) {
-        // plan_decide's test, ESS = fl(fl(tS tS) / tQ) < ess_bound, without the division away from the
-        // bound (2^-48 covers the quotient's and the product's roundings)
         const bool degenerate = (nM == kNkEmpty) || !(tS > 0.0);
         int resample = 0;
-        if (!degenerate) {
-          const double ss = tS * tS, lim = sh.ess_bound * tQ;
-          resample = ahead || (ss < lim * (1.0 - 0x1p-48) ? true : (ss > lim * (1.0 + 0x1p-48) ? false : ss / tQ < sh.ess_bound));
-        }
+        if (!degenerate) resample = ahead || ess_below(tS * tS, tQ, a.ess_bound);
         sh.resample = resample;
         sh.degenerate = degenerate ? 1 : 0;
       }

@@ -25,27 +25,32 @@ static __device__ __noinline__ int exact_count(const float* d, int upto, unsigne
   return c >= (unsigned long long)cap ? cap : (int)c;
 }
 
+// ESS = fl(ss / q) < bound, without the division away from the bound: 2^-48 covers the roundings of the
+// quotient and of the products.
+__device__ __forceinline__ bool ess_below(double ss, double q, double bound) {
+  const double lim = bound * q;
+  if (ss < lim * (1.0 - 0x1p-48)) return true;
+  if (ss > lim * (1.0 + 0x1p-48)) return false;
+  return ss / q < bound;
+}
+
 // What the finish of a tick's plan needs from its decision (fused_decide -> fused_finish).
 struct FusedTail {
-  double tS, tH, ess, logS_prev_old;
+  double tS, tQ, tH, logS_prev_old;
   int nM, degenerate, resample, resampled_prev_old, tick_old;
 };
 
 
 // The tick's decision from its statistics, by one thread: plan_decide's operations on the device-state
 // fields that the next tick and the resampling read, in its order; the rest is left to fused_finish
-// in tl. APF as TickArgs::apf (the first stage of an auxiliary-filter tick does not advance the tick).
+// in tl. The threshold test is a.ess_bound's. APF as TickArgs::apf (the first stage of an auxiliary-filter tick does not advance the tick).
 template <int APF = 0>
-__device__ __forceinline__ void fused_decide(const TickArgs& a, int N, int nM, double tS, double tQ, double tH,
+__device__ __forceinline__ void fused_decide(const TickArgs& a, int nM, double tS, double tQ, double tH,
                                              DevState* st, FusedTail& tl) {
   const bool degenerate = (nM == kNkEmpty) || !(tS > 0.0);
-  double ess = 0.0;
   int resample = 0;
-  if (!degenerate) {
-    ess = tS * tS / tQ;
-    resample = (a.ess_threshold <= 0.0f) || (ess / (double)N < (double)a.ess_threshold);
-  }
-  tl.tS = tS; tl.tH = tH; tl.ess = ess; tl.nM = nM;
+  if (!degenerate) resample = (a.ess_threshold <= 0.0f) || ess_below(tS * tS, tQ, a.ess_bound);
+  tl.tS = tS; tl.tQ = tQ; tl.tH = tH; tl.nM = nM;
   tl.degenerate = degenerate ? 1 : 0; tl.resample = resample;
   tl.logS_prev_old = st->logS_prev; tl.resampled_prev_old = st->resampled_prev; tl.tick_old = st->tick;
   const int cur = st->cur;
@@ -84,8 +89,9 @@ __device__ __forceinline__ void fused_decide(const TickArgs& a, int N, int nM, d
 template <int APF = 0>
 __device__ __forceinline__ void fused_finish(const FusedTail& tl, DevState* st, BpfTickRecord* rec_out) {
   constexpr double kLn2d = 0.693147180559945309417232121458;
-  double dll = -INFINITY, hm = __longlong_as_double(0x7FF8000000000000LL), L = 0.0;
+  double dll = -INFINITY, hm = __longlong_as_double(0x7FF8000000000000LL), L = 0.0, ess = 0.0;
   if (!tl.degenerate) {
+    ess = tl.tS * tl.tS / tl.tQ;
     L = log(tl.tS);
     dll = __fma_rn((double)tl.nM, kLn2d, L) - tl.logS_prev_old;
     hm = tl.tH / tl.tS;
@@ -99,7 +105,7 @@ __device__ __forceinline__ void fused_finish(const FusedTail& tl, DevState* st, 
   if (rec_out) {
     BpfTickRecord r;
     r.dloglik = rec_dll; r.loglik_ref = ll_ref; r.loglik_total = st->ll_total;
-    r.h_mean = (float)hm; r.ess = (float)tl.ess; r.resampled = tl.resample; r.tick = tl.tick_old;
+    r.h_mean = (float)hm; r.ess = (float)ess; r.resampled = tl.resample; r.tick = tl.tick_old;
     *rec_out = r;
   }
   if (!tl.resample && !tl.degenerate) st->logS_prev = L;
