@@ -13,6 +13,9 @@
 // at c ^ row) so both the lane-strided and the per-thread-contiguous access
 // patterns are free of shared-memory bank conflicts.
 //
+// The classes run with their default shapes as batch_fast_filter (at most 16 particles a thread,
+// unrolled; below); this generic form serves other shapes and correlated-noise runs.
+//
 // Gradient form (batch_grad_kernel): after a filter's taped forward, the same
 // CTA runs its adjoint backward, checkpoint segment by segment from the last:
 // the segment's particles are recomputed from the checkpoint through the

@@ -146,7 +146,7 @@ cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
   cudaError_t e = launch_init(g->plan, k.mu, std_stat, k.seed, g->stream);
   const ObsModel obs = make_obs(k.nu);
   if (e == cudaSuccess && k.T > 0 && g->resident) {
-    // The whole taped run as one resident launch: N = 2^20 26 -> 13 us per tick, and three nodes to
+    // The whole taped run as one resident launch: N = 2^20 26 -> 14 us per tick, and three nodes to
     // capture anew for every theta instead of three per tick.
     TickArgs a{};
     a.mu = k.mu; a.rho = k.rho; a.sigma = k.sigma;

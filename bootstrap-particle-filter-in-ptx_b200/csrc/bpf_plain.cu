@@ -1739,14 +1739,14 @@ cudaError_t plan_alloc(Plan& p, int N) {
   al(&p.items, p.max_items * sizeof(int4));
   const size_t jbytes = (p.G * sizeof(double) + 255) & ~(size_t)255;
   al(&p.jpart, jbytes + resident_xbuf_bytes(p.G));     // one allocation for both
-  if (e == cudaSuccess) p.xbuf = reinterpret_cast<unsigned char*>(p.jpart) + jbytes;
+  if (e == cudaSuccess && resident_xbuf_bytes(p.G) > 0) p.xbuf = reinterpret_cast<unsigned char*>(p.jpart) + jbytes;
   al(&p.jticket, sizeof(unsigned));
   al(&p.pticket, sizeof(unsigned));
   al(&p.st, sizeof(DevState));
   if (e == cudaSuccess) e = cudaMemset(p.nexp, 0, p.G * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(p.jticket, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(p.pticket, 0, sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMemset(p.xbuf, 0, resident_xbuf_bytes(p.G));
+  if (e == cudaSuccess && p.xbuf) e = cudaMemset(p.xbuf, 0, resident_xbuf_bytes(p.G));
   if (e == cudaSuccess) e = cudaDeviceSynchronize();   // visible to every stream before first use
   return e;
 }

@@ -22,8 +22,8 @@
 // What bounds it: latency, three grid-wide dependencies deep at most, and the issue of about 60
 // thread-instructions per particle (16 particles a thread keep the per-thread overhead small: with
 // 1024 threads of 4 the same tick issued 144 per particle). Measured per tick: N = 300000 at
-// ESS < 0.5 N 4.4 us (16.4 with a launch per kernel), always resampling 10.4 us (20.8); N = 1000003 at
-// ESS < 0.5 N 6.1 us (12.5).
+// ESS < 0.5 N 4.0 us (16.4 with a launch per kernel), always resampling 9.1 us (20.8); N = 1000003 at
+// ESS < 0.5 N 5.7 us (12.5), always resampling 12.5; N = 2.4 M at ESS < 0.5 N 10.7.
 // Results equal the tick-per-launch path's bit for bit.
 //
 // The CTAs wait on one another, so the launch is cooperative (all resident or none start), and every
@@ -53,7 +53,7 @@ constexpr int kMail = 16;
 constexpr size_t kXHeader = 256;
 __host__ __device__ inline size_t mail_flag_bytes(int G) { return ((size_t)G * 4 + 127) & ~(size_t)127; }
 __host__ __device__ inline size_t mail_bytes(int G) { return mail_flag_bytes(G) + (((size_t)G * 64 + 127) & ~(size_t)127); }
-size_t resident_xbuf_bytes(int G) { return kXHeader + kMail * mail_bytes(G); }
+size_t resident_xbuf_bytes(int G) { return G <= kResMaxTiles ? kXHeader + kMail * mail_bytes(G) : 0; }
 
 __device__ __forceinline__ void st_relaxed_b128(void* p, unsigned long long lo, unsigned long long hi) {
   asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p), "l"(lo), "l"(hi)

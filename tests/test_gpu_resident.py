@@ -148,3 +148,46 @@ def test_resident_tape_with_and_without_kept_particles(bpf, N):
             out.append((tape.forward((MU, RHO, SIG), y, seed=seed).item(), tape.backward().cpu().numpy().tobytes()))
         tape.close()
     assert out[0:2] == out[2:4] == out[4:6]
+
+
+def test_resident_runs_on_several_streams_and_threads(bpf):
+    """Filters that together need more SMs than there are, running at the same time on their own streams
+    from two host threads, beside single ticks of another: each equals its own run alone."""
+    import threading
+    import torch
+    T, sizes = 150, (1000003, 300000, 1500000, 70000)
+    y = _series(T, 12)
+    yd = torch.tensor(y, device="cuda")
+    alone = [_device_run(bpf, n, 0.5, 0.0, 0.0, y, True, (17,))[0][:2] for n in sizes]
+    out = {}
+
+    # created beforehand: creating a filter synchronises the device, which no other thread's stream
+    # capture survives
+    fs = {n: (bpf.GpuBpf(n, RHO, SIG, MU, seed=17, ess_threshold=0.5),
+              torch.zeros(T * 40, dtype=torch.uint8, device="cuda")) for n in sizes}
+    g = bpf.GpuBpf(200000, RHO, SIG, MU, seed=1)
+    g.step(0.1)
+    torch.cuda.synchronize()
+
+    def worker(part):
+        for _ in range(3):
+            for n in part:
+                fs[n][0].reset(17)
+                fs[n][0].step_many_device(yd.data_ptr(), T, fs[n][1].data_ptr())
+        for n in part:
+            parts = bytes(fs[n][0].get_particles())   # waits for the filter's stream
+            out[n] = parts
+
+    ts = [threading.Thread(target=worker, args=(part,)) for part in (sizes[:2], sizes[2:])]
+    for t in ts:
+        t.start()
+    for v in y[:40]:
+        g.step(float(v))
+    for t in ts:
+        t.join()
+    torch.cuda.synchronize()
+    out = {n: (fs[n][1].cpu().numpy().tobytes(), p) for n, p in out.items()}
+    for f, _ in fs.values():
+        f.close()
+    g.close()
+    assert [out[n] for n in sizes] == alone
