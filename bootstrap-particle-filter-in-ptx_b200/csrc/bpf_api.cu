@@ -108,6 +108,7 @@ struct Impl {
   bool fused_small = true;
   int small_tiles = 4;                  // largest fused cluster on the filter's device (tiles)
   int res_tiles = 0;                    // largest filter of a resident run on it (tiles)
+  ResidentWaits waits;                  // of resident runs (gpu_bpf_debug_resident)
 
   // profiling
   bool profiling = false;
@@ -150,7 +151,7 @@ bool use_resident(const Impl* m, const TickArgs& a) {
 bool one_launch(const Impl* m, const TickArgs& a) { return use_small(m, a) || use_resident(m, a); }
 cudaError_t launch_run(Impl* m, const TickArgs& a, int n_ticks) {
   if (use_small(m, a)) return launch_small(m->plan, a, n_ticks, m->stream, m->pdl);
-  return launch_resident(m->plan, a, ResidentTape{}, false, n_ticks, m->res_tiles, m->stream);
+  return launch_resident(m->plan, a, ResidentTape{}, false, n_ticks, m->res_tiles, m->stream, m->waits);
 }
 
 // Filters of at most kTailTiles tiles run the plan in pass 1's last CTA instead of a plan
@@ -301,6 +302,13 @@ int wait_single_tick(Impl* m) {
   return BPF_OK;
 }
 
+// The device state's error as a read-back reports it: a degenerate tick is in its record; a kernel that
+// gave up (BPF_ERR_STATE) has left neither a state nor a result.
+int note_error(Impl* m, int error) {
+  if (error != BPF_OK) m->sticky_error = error;
+  return error == BPF_ERR_STATE ? set_err(BPF_ERR_STATE) : BPF_OK;
+}
+
 int read_back(GpuBpfState* s, Impl* m, int slot, BpfTickRecord* out) {
   if (slot == 0 && m->last_in_map) {
     const int rc = wait_single_tick(m);
@@ -311,8 +319,7 @@ int read_back(GpuBpfState* s, Impl* m, int slot, BpfTickRecord* out) {
     s->resample_count = mm.resample_count;
     s->timestep = mm.tick;
     s->last_h_est = out->h_mean;
-    if (mm.error != BPF_OK) m->sticky_error = mm.error;
-    return BPF_OK;
+    return note_error(m, mm.error);
   }
   CK(cudaMemcpyAsync(m->rec_pin + slot, m->rec_dev + slot, sizeof(BpfTickRecord), cudaMemcpyDeviceToHost, m->stream));
   CK(cudaMemcpyAsync(m->st_pin, m->plan.st, sizeof(DevState), cudaMemcpyDeviceToHost, m->stream));
@@ -322,8 +329,7 @@ int read_back(GpuBpfState* s, Impl* m, int slot, BpfTickRecord* out) {
   s->resample_count = m->st_pin->resample_count;
   s->timestep = m->st_pin->tick;
   s->last_h_est = out->h_mean;
-  if (m->st_pin->error != BPF_OK) m->sticky_error = m->st_pin->error;
-  return BPF_OK;
+  return note_error(m, m->st_pin->error);
 }
 
 BpfResult to_result(const Impl* m, const BpfTickRecord& r) {
@@ -860,6 +866,7 @@ double gpu_bpf_get_loglik_total(GpuBpfState* s) {
   if (ensure_device(m)) return NAN;
   if (cudaMemcpyAsync(m->st_pin, m->plan.st, sizeof(DevState), cudaMemcpyDeviceToHost, m->stream) != cudaSuccess ||
       cudaStreamSynchronize(m->stream) != cudaSuccess) { set_err(BPF_ERR_CUDA); return NAN; }
+  if (note_error(m, m->st_pin->error)) return NAN;
   return m->st_pin->ll_total;
 }
 
@@ -878,6 +885,8 @@ int gpu_bpf_get_particles(GpuBpfState* s, float* h_out) {
   if (rc) return rc;
   CK(cudaMemcpyAsync(m->st_pin, m->plan.st, sizeof(DevState), cudaMemcpyDeviceToHost, m->stream));
   CK(cudaStreamSynchronize(m->stream));
+  rc = note_error(m, m->st_pin->error);
+  if (rc) return rc;
   const float* src = m->st_pin->cur ? m->plan.h1 : m->plan.h0;
   CK(cudaMemcpy(h_out, src, (size_t)m->plan.N * sizeof(float), cudaMemcpyDeviceToHost));
   return BPF_OK;
@@ -982,6 +991,8 @@ int gpu_bpf_save(GpuBpfState* s, void* buf, size_t cap) {
   out += sizeof(h);
   DevState st;
   CK(cudaMemcpy(&st, m->plan.st, sizeof(DevState), cudaMemcpyDeviceToHost));
+  rc = note_error(m, st.error);
+  if (rc) return rc;
   std::memcpy(out, &st, sizeof(st));
   out += sizeof(st);
   const size_t nb = (size_t)m->plan.N * sizeof(float);
@@ -1059,6 +1070,19 @@ int gpu_bpf_set_fused_small(GpuBpfState* s, int enable) {
     if (m->t_g) { cudaGraphDestroy(m->t_g); m->t_g = nullptr; }
     m->fused_small = on;
   }
+  return BPF_OK;
+}
+
+int gpu_bpf_debug_resident(GpuBpfState* s, int fault, int cta, int exchange, double limit_ms) {
+  Impl* m = impl_of(s);
+  if (!m) return set_err(BPF_ERR_STATE);
+  ResidentWaits w;
+  if (!resident_waits_of(fault, cta, exchange, limit_ms, &w)) return set_err(BPF_ERR_ARG);
+  int rc = ensure_device(m);
+  if (rc) return rc;
+  CK(cudaStreamSynchronize(m->stream));
+  if (m->dgraph) { cudaGraphExecDestroy(m->dgraph); m->dgraph = nullptr; }   // it holds the waits
+  m->waits = w;
   return BPF_OK;
 }
 

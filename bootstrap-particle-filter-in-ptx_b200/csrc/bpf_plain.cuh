@@ -151,13 +151,31 @@ struct ResidentTape {        // gradient tape of a taped run from tick 0 (all nu
   float2* aux;                         // {1/S, nM} per tick
   float* hist;                         // every tick's particles as weighted, at hist + t * ckpt_stride, or null
 };
+// How long a wait of a resident run polls before it gives up and, in tests, one failure made on
+// purpose: CTA cta gives up in exchange xn (1-based in the run) or in the wait for the children of its
+// resampling, or does not publish its record of that exchange. No wait outlasts its limit.
+constexpr unsigned long long kResWaitNs = 2000000000ull;
+enum ResidentFault { kFaultNone = 0, kFaultExchange = 1, kFaultFlags = 2, kFaultWithhold = 3 };
+struct ResidentWaits {
+  unsigned long long limit_ns = kResWaitNs;
+  int fault = kFaultNone, cta = 0;
+  unsigned xn = 0u;
+};
+inline bool resident_waits_of(int fault, int cta, int exchange, double limit_ms, ResidentWaits* out) {
+  if (fault < kFaultNone || fault > kFaultWithhold || cta < 0 || exchange < 0 ||
+      !(limit_ms > 0.0 && limit_ms <= (double)kResWaitNs * 1e-6))
+    return false;
+  out->limit_ns = (unsigned long long)(limit_ms * 1e6);
+  out->fault = fault; out->cta = cta; out->xn = (unsigned)exchange;
+  return true;
+}
 constexpr int kResMaxTilesPerCta = 4;
 size_t resident_xbuf_bytes(int G);
 int resident_max_tiles(int device);    // 0: the device takes no resident runs
 // Whether the kernel of such a run (G tiles, observation and state noise model) is ready on the device.
 bool resident_ready(int device, int G, int max_tiles, bool tstate, bool gauss, bool apf);
 cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
-                            int max_tiles, cudaStream_t s);
+                            int max_tiles, cudaStream_t s, const ResidentWaits& waits = ResidentWaits());
 int pass2_grid_size(int device);
 // Tiles the fused tick takes on this device (16, else 8; 4 before pass2_grid_size configured it).
 int small_max_tiles(int device);

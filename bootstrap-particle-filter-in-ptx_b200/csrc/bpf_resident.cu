@@ -27,7 +27,10 @@
 // Results equal the tick-per-launch path's bit for bit.
 //
 // The CTAs wait on one another, so the launch is cooperative (all resident or none start), and every
-// wait gives up after kResWaitNs: the run then ends with BPF_ERR_STATE.
+// wait gives up after kResWaitNs. A CTA that gives up raises the abort mark and stores nothing; the
+// others tell the keeper when their last wait is over, and the keeper, which alone writes the state,
+// waits for all of them: whichever CTA gave up, the run ends with BPF_ERR_STATE, and a later run
+// does not start on such a state.
 #include "bpf_tick.cuh"
 #include <mutex>
 #include <type_traits>
@@ -36,7 +39,6 @@ namespace bpf {
 
 constexpr int kResThreads = 512;
 constexpr int kResWarps = kResThreads / 32;
-constexpr unsigned long long kResWaitNs = 2000000000ull;
 constexpr int kResMaxTiles = 1024;        // records an exchange holds at most (32 sums of 32 tiles)
 constexpr int kResHeavy = 16;             // children above which a parent's run is shared by its warp
 static_assert(kResMaxTilesPerCta == 4, "four tiles of two groups of threads");
@@ -77,11 +79,11 @@ __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
 struct Patience {
   unsigned long long t0 = 0ull;
   unsigned spins = 0u;
-  __device__ __forceinline__ bool more(const unsigned* abort_word, unsigned mark) {
+  __device__ __forceinline__ bool more(const unsigned* abort_word, unsigned mark, unsigned long long limit_ns) {
     if ((++spins & 255u) != 0u) return true;
     const unsigned long long t = global_timer_ns();
     if (t0 == 0ull) t0 = t;
-    return __all_sync(0xffffffffu, t - t0 < kResWaitNs && ld_relaxed_u32(abort_word) != mark);
+    return __all_sync(0xffffffffu, t - t0 < limit_ns && ld_relaxed_u32(abort_word) != mark);
   }
 };
 
@@ -144,7 +146,7 @@ struct ResidentShared {
 // threads: (2, 1) for one tile a CTA, (1, 1) for two, (1, 2) for three and four.
 template <bool TSTATE, bool GAUSS, bool APF, int SPLIT, int Q>
 __global__ void __launch_bounds__(kResThreads, 1)
-resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
+resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int n_ticks, int nt) {
   constexpr int NG = kResThreads / (kThreads * SPLIT);   // groups
   constexpr int NT = NG * Q;                    // tiles a CTA can hold
   constexpr int GW = 8 * SPLIT;                 // warps of a group
@@ -227,7 +229,9 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
   double dS = 0.0, dQ = 0.0, dH = 0.0;
   int d_nM = 0;
   unsigned xn = 0u;                             // exchanges so far
-  bool failed = false;                          // a wait gave up (the same in every thread of the CTA)
+  // a wait gave up (the same in every thread of the CTA), or the state is that of a run that did
+  const bool refused = sh.st.error == BPF_ERR_STATE;
+  bool failed = refused;
   bool pending = false;                         // the keeper's state is one decision behind
   int pending_rec = 0;
   auto settle = [&](int apf_stage, int t) {
@@ -248,7 +252,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
   const bool ahead = a.ess_threshold <= 0.0f;   // every tick that can resample does
   int stage = 0, prev_stage = 0;                // APF: 0 the first tick of all, else stages 1 and 2 of a tick
   int t = 0;
-  while (t < n_ticks) {
+  while (!failed && t < n_ticks) {
     if ((!APF || stage != 2) && (t & (kResThreads - 1)) == 0) {
       __syncthreads();
       if (t + tid < n_ticks) sh.ys[tid] = __ldg(a.y_ptr + t + tid);
@@ -391,7 +395,8 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
           }
           tS = warp_sum_d(tS); tQ = warp_sum_d(tQ); tH = warp_sum_d(tH);
           tE = warp_sum_u64(tE);
-          if (lane < kMail) {                          // (every lane holds the same sums)
+          const bool withheld = waits.fault == kFaultWithhold && waits.cta == (int)blockIdx.x && waits.xn == xn;
+          if (lane < kMail && !withheld) {             // (every lane holds the same sums)
             unsigned char* slot = p.xbuf + kXHeader + lane * mail_size + mail_flag_bytes(G) +
                                   ((size_t)(xn & 1u) * G + first + j) * 32;
             st_relaxed_b128(slot, (unsigned long long)__float_as_uint((float)tS) | ((unsigned long long)__float_as_uint((float)tQ) << 32),
@@ -441,7 +446,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       for (;;) {
         const bool ok = (unsigned)(a1 >> 32) == xno && (unsigned)(b1 >> 32) == xno;
         if (__all_sync(0xffffffffu, ok)) break;
-        if (!pt.more(xw + 1, epoch + 1u)) { bad = true; break; }     // the same in every lane
+        if (!pt.more(xw + 1, epoch + 1u, waits.limit_ns)) { bad = true; break; }     // the same in every lane
         ld_relaxed_b128(slot, a0, a1);
         ld_relaxed_b128(slot + 16, b0, b1);
       }
@@ -463,6 +468,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
       S = warp_sum_d(S); Qs = warp_sum_d(Qs); H = warp_sum_d(H);
       if (lane == 0) { sh.wn[pw] = nW; sh.wS[pw] = S; sh.wQ[pw] = Qs; sh.wH[pw] = H; }
     }
+    if (waits.fault == kFaultExchange && waits.cta == (int)blockIdx.x && waits.xn == xn) bad = true;
     if (__syncthreads_or(bad)) { failed = true; break; }
 
     // ---- decision (the last warp), and beside it, when every tick resamples, the masses ----
@@ -733,10 +739,11 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
           for (;;) {                              // left by a warp vote, as above
             const bool ok = !wait || (int)(ld_relaxed_u32(flag) - xno) >= 0;
             if (__all_sync(0xffffffffu, ok)) break;
-            if (!pt.more(xw + 1, epoch + 1u)) { bad = true; break; }
+            if (!pt.more(xw + 1, epoch + 1u, waits.limit_ns)) { bad = true; break; }
           }
           asm volatile("fence.acq_rel.gpu;" ::: "memory");   // acquire (a relaxed poll leaves L1 alone)
         }
+        if (waits.fault == kFaultFlags && waits.cta == (int)blockIdx.x && waits.xn == xn) bad = true;
         if (__syncthreads_or(bad)) { failed = true; break; }
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -775,7 +782,14 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
 
   if (tid == kDecider && pending && keeper && !failed) settle(prev_stage, pending_rec);
   __syncthreads();
-  if (failed && tid == 0) st_release_u32(xw + 1, epoch + 1u);   // the other CTAs stop waiting
+  // This CTA's end of the run: the abort mark, on which the other CTAs stop waiting, or, in the mailbox
+  // that the keeper polls, a number past every exchange of this run.
+  const unsigned xend = epoch + xn + 1u;
+  unsigned char* keeper_mail = p.xbuf + kXHeader + ((gridDim.x - 1u) % kMail) * mail_size;
+  if (tid == 0 && !refused) {
+    if (failed) st_release_u32(xw + 1, epoch + 1u);
+    else if (!keeper) st_release_u32(reinterpret_cast<unsigned*>(keeper_mail) + blockIdx.x, xend);
+  }
   if (!failed) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -793,6 +807,20 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
     }
   }
   if (keeper) {
+    if (!failed) {                              // every other CTA's end (one CTA a thread)
+      const bool wait = tid + 1 < (int)gridDim.x;
+      bool bad = false;
+      if (__any_sync(0xffffffffu, wait)) {
+        const unsigned* flag = reinterpret_cast<const unsigned*>(keeper_mail) + (wait ? tid : (int)blockIdx.x);
+        Patience pt;
+        for (;;) {                              // left by a warp vote, as above
+          const bool ok = !wait || (int)(ld_relaxed_u32(flag) - xend) >= 0;
+          if (__all_sync(0xffffffffu, ok)) break;
+          if (!pt.more(xw + 1, epoch + 1u, waits.limit_ns)) { bad = true; break; }
+        }
+      }
+      if (__syncthreads_or(bad)) failed = true;
+    }
     if (tid == 0) {
       if (failed) sh.st.error = BPF_ERR_STATE;
       *reinterpret_cast<volatile unsigned*>(xw) = epoch + 4u * (unsigned)n_ticks + 4u;   // past every number used
@@ -808,7 +836,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, int n_ticks, int nt) {
 // ---------------------------------------------------------------------------
 namespace {
 
-using ResidentKernel = void (*)(Plan, TickArgs, ResidentTape, int, int);
+using ResidentKernel = void (*)(Plan, TickArgs, ResidentTape, ResidentWaits, int, int);
 
 template <bool APF, int SPLIT, int Q>
 ResidentKernel pick_model(bool tstate, bool gauss, size_t* smem) {
@@ -840,7 +868,7 @@ int resident_max_tiles(int device) {
     int sms = 0, coop = 0;
     const bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
                     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop != 0 &&
-                    sms > 0 && sms * kResMaxTilesPerCta <= kResMaxTiles;
+                    sms > 0 && sms < kResThreads && sms * kResMaxTilesPerCta <= kResMaxTiles;
     if (!ok) cudaGetLastError();
     g_sms[device] = ok ? sms : -1;
   }
@@ -868,7 +896,7 @@ bool resident_ready(int device, int G, int max_tiles, bool tstate, bool gauss, b
 }
 
 cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
-                            int max_tiles, cudaStream_t s) {
+                            int max_tiles, cudaStream_t s, const ResidentWaits& waits) {
   if (!p.xbuf || p.G < 1 || p.G > max_tiles || n_ticks < 1 || !a.y_ptr) return cudaErrorInvalidValue;
   const int sms = max_tiles / kResMaxTilesPerCta;
   const int nt = (p.G + sms - 1) / sms;
@@ -884,7 +912,7 @@ cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, p, a, tape, n_ticks, nt);
+  return cudaLaunchKernelEx(&cfg, k, p, a, tape, waits, n_ticks, nt);
 }
 
 }  // namespace bpf

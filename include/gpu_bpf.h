@@ -574,6 +574,17 @@ int       gpu_bpf_debug_fail_alloc(long long k);
 long long gpu_bpf_debug_alloc_count(void);
 long long gpu_bpf_debug_live_allocs(void);
 
+/* Waits of resident runs (gpu_bpf_set_fused_small; testing aid). The CTAs of such a run wait on one
+ * another, each wait at most 2 s; a run in which one gives up ends with BPF_ERR_STATE: step_many returns
+ * it, after step_many_device the next read-back does, and later runs do not start until gpu_bpf_reset or
+ * gpu_bpf_load. This call sets the limit of this filter's waits (0 < limit_ms <= 2000) and one failure
+ * made on purpose: fault 0 none; 1 CTA cta gives up in the run's exchange number `exchange` (1-based;
+ * one per tick, two per auxiliary-filter tick after the first); 2 it gives up waiting for the children
+ * of that exchange's resampling; 3 it does not publish its record of that exchange, so every wait for
+ * it runs out. No GPU fault is involved: the kernel returns. */
+int gpu_bpf_debug_resident(GpuBpfState* state, int fault, int cta, int exchange, double limit_ms);
+int gpu_apf_debug_resident(GpuApfState* state, int fault, int cta, int exchange, double limit_ms);
+
 /* Number of kernel launches this library has issued (all filters). */
 long long gpu_bpf_launch_count(void);
 

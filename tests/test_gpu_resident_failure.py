@@ -1,0 +1,88 @@
+"""Resident runs whose CTAs give up waiting: made on purpose by gpu_bpf_debug_resident (a CTA told to
+give up, or a record never published with a limit of 20 ms on the waits), so the kernel returns its
+status and no GPU fault is involved. The run must end with BPF_ERR_STATE whichever CTA gave up and
+however late, and a reset filter must then run as a new one, bit for bit."""
+from __future__ import annotations
+
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+RHO, SIG, MU = 0.97, 0.15, -1.0
+TILE = 4096
+EXCHANGE, FLAGS, WITHHOLD = 1, 2, 3
+
+
+def _series(T, seed):
+    from gpubpf import dgp
+    return np.asarray(dgp.matched_series(T, RHO, SIG, MU, seed)[1], dtype=np.float32)
+
+
+def _arm(f, fn, fault=0, cta=0, exchange=0, limit_ms=2000.0):
+    from gpubpf import _lib
+    assert getattr(f._lib, fn)(f._s, fault, cta, exchange, limit_ms) == _lib.BPF_OK
+
+
+T = 12
+# (particles, fault, CTA, exchange): the first CTA or the keeper (the last one), the last exchange, the
+# children of the last tick, and a record that is never published, with one to four tiles a CTA
+CASES = [(70000, EXCHANGE, 0, T), (70000, EXCHANGE, 17, T), (70000, FLAGS, 0, T), (70000, FLAGS, 3, 5),
+         (70000, WITHHOLD, 2, 7), (70000, WITHHOLD, 0, T), (1000003, EXCHANGE, 1, T), (1000003, FLAGS, 1, T),
+         (592 * TILE, EXCHANGE, 0, T), (592 * TILE, FLAGS, 146, T), (592 * TILE, WITHHOLD, 147, 1)]
+
+
+@pytest.mark.parametrize("N,fault,cta,exchange", CASES)
+def test_run_with_a_wait_given_up_reports_it(bpf, N, fault, cta, exchange):
+    import torch
+    from gpubpf import _lib
+    y = _series(T, 9)
+    f = bpf.GpuBpf(N, RHO, SIG, MU, seed=3, ess_threshold=0.0)
+    want = [bytes(r) for r in f.step_many(y.tolist(), records=True)], bytes(f.get_particles())
+    yd = torch.tensor(y, device="cuda")
+    rec = torch.zeros(T * 40, dtype=torch.uint8, device="cuda")
+
+    f.reset(3)
+    _arm(f, "gpu_bpf_debug_resident", fault, cta, exchange, 20.0)
+    with pytest.raises(bpf.BpfError) as e:
+        f.step_many(y.tolist())
+    assert e.value.code == _lib.BPF_ERR_STATE
+    f.reset(3)
+    f.step_many_device(yd.data_ptr(), T, rec.data_ptr())          # reported by the read-backs
+    for read in (f.get_record, f.get_particles, f.save, f.get_result):
+        with pytest.raises(bpf.BpfError) as e:
+            read()
+        assert e.value.code == _lib.BPF_ERR_STATE
+    assert math.isnan(f.get_loglik_total())
+
+    _arm(f, "gpu_bpf_debug_resident")                             # a later run does not start on that state
+    with pytest.raises(bpf.BpfError) as e:
+        f.step_many(y.tolist())
+    assert e.value.code == _lib.BPF_ERR_STATE
+    f.reset(3)
+    assert ([bytes(r) for r in f.step_many(y.tolist(), records=True)], bytes(f.get_particles())) == want
+    f.close()
+
+
+@pytest.mark.parametrize("N", [50000, 1500000])
+@pytest.mark.parametrize("fault,cta,exchange", [(EXCHANGE, 0, 2 * T - 1), (FLAGS, 1, 2 * T - 1), (WITHHOLD, 1, 8)])
+def test_auxiliary_run_with_a_wait_given_up_reports_it(bpf, N, fault, cta, exchange):
+    from gpubpf import _lib
+    y = _series(T, 9).tolist()
+    f = bpf.GpuApf(N, RHO, SIG, MU, seed=3)
+    _arm(f, "gpu_apf_debug_resident", fault, cta, exchange, 20.0)
+    with pytest.raises(bpf.BpfError) as e:
+        f.step_many(y)
+    assert e.value.code == _lib.BPF_ERR_STATE
+    f.close()
+
+
+def test_rejects_bad_arguments(bpf):
+    from gpubpf import _lib
+    f = bpf.GpuBpf(70000, RHO, SIG, MU, seed=3)
+    for args in ((4, 0, 1, 10.0), (-1, 0, 1, 10.0), (1, -1, 1, 10.0), (1, 0, -1, 10.0), (1, 0, 1, 0.0), (1, 0, 1, 2001.0),
+                 (1, 0, 1, math.nan)):
+        assert f._lib.gpu_bpf_debug_resident(f._s, *args) == _lib.BPF_ERR_ARG
+    f.close()
