@@ -1086,6 +1086,14 @@ int gpu_bpf_debug_resident(GpuBpfState* s, int fault, int cta, int exchange, dou
   return BPF_OK;
 }
 
+int gpu_bpf_debug_wait_budget(const unsigned long long* now_ns, int n, unsigned long long limit_ns) {
+  if (!now_ns || n < 0 || limit_ns == 0ull) return -set_err(BPF_ERR_ARG);
+  WaitBudget b;
+  for (int i = 0; i < n; ++i)
+    if (b.over(now_ns[i], limit_ns)) return i;
+  return n;
+}
+
 int gpu_bpf_profile(GpuBpfState* s, int enable) {
   Impl* m = impl_of(s);
   if (!m) return set_err(BPF_ERR_STATE);

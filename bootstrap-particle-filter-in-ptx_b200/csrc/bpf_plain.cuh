@@ -155,6 +155,18 @@ struct ResidentTape {        // gradient tape of a taped run from tick 0 (all nu
 // purpose: CTA cta gives up in exchange xn (1-based in the run) or in the wait for the children of its
 // resampling, or does not publish its record of that exchange. No wait outlasts its limit.
 constexpr unsigned long long kResWaitNs = 2000000000ull;
+// Time spent polling against that limit, from the clock at one look after another. The time between two
+// looks counts as at most a sixteenth of the limit: while the GPU runs another program, or the grid is
+// held up as a whole, the clock goes on but nobody could publish what the wait is for.
+struct WaitBudget {
+  unsigned long long last = 0ull, spent = 0ull;
+  __host__ __device__ __forceinline__ bool over(unsigned long long now, unsigned long long limit) {
+    const unsigned long long step = now - last, cap = limit / 16ull + 1ull;
+    if (last != 0ull) spent += step < cap ? step : cap;
+    last = now;
+    return spent >= limit;
+  }
+};
 enum ResidentFault { kFaultNone = 0, kFaultExchange = 1, kFaultFlags = 2, kFaultWithhold = 3 };
 struct ResidentWaits {
   unsigned long long limit_ns = kResWaitNs;

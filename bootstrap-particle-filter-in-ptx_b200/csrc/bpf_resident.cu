@@ -27,7 +27,7 @@
 // Results equal the tick-per-launch path's bit for bit.
 //
 // The CTAs wait on one another, so the launch is cooperative (all resident or none start), and every
-// wait gives up after kResWaitNs. A CTA that gives up raises the abort mark and stores nothing; the
+// wait gives up after kResWaitNs of polling. A CTA that gives up raises the abort mark and stores nothing; the
 // others tell the keeper when their last wait is over, and the keeper, which alone writes the state,
 // waits for all of them: whichever CTA gave up, the run ends with BPF_ERR_STATE, and a later run
 // does not start on such a state.
@@ -74,16 +74,15 @@ __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
   return v;
 }
 
-// Whether a warp's wait goes on (the same answer in every lane): every 256 polls it looks at the time
-// and at the abort mark of this launch.
+// Whether a warp's wait goes on (the same answer in every lane): every 256 polls it looks at its budget
+// and at the abort mark of this launch. After a no the caller looks at its words once more.
 struct Patience {
-  unsigned long long t0 = 0ull;
+  WaitBudget budget;
   unsigned spins = 0u;
   __device__ __forceinline__ bool more(const unsigned* abort_word, unsigned mark, unsigned long long limit_ns) {
     if ((++spins & 255u) != 0u) return true;
-    const unsigned long long t = global_timer_ns();
-    if (t0 == 0ull) t0 = t;
-    return __all_sync(0xffffffffu, t - t0 < limit_ns && ld_relaxed_u32(abort_word) != mark);
+    const bool over = budget.over(global_timer_ns(), limit_ns);
+    return __all_sync(0xffffffffu, !over && ld_relaxed_u32(abort_word) != mark);
   }
 };
 
@@ -443,10 +442,11 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
       const unsigned char* slot = slot_of(u);
       if (u > 0) { ld_relaxed_b128(slot, a0, a1); ld_relaxed_b128(slot + 16, b0, b1); }
       Patience pt;
-      for (;;) {
+      for (bool last = false;;) {
         const bool ok = (unsigned)(a1 >> 32) == xno && (unsigned)(b1 >> 32) == xno;
         if (__all_sync(0xffffffffu, ok)) break;
-        if (!pt.more(xw + 1, epoch + 1u, waits.limit_ns)) { bad = true; break; }     // the same in every lane
+        if (last) { bad = true; break; }             // the same in every lane
+        last = !pt.more(xw + 1, epoch + 1u, waits.limit_ns);
         ld_relaxed_b128(slot, a0, a1);
         ld_relaxed_b128(slot + 16, b0, b1);
       }
@@ -736,10 +736,11 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
           if (!__any_sync(0xffffffffu, wait)) continue;
           const unsigned* flag = reinterpret_cast<const unsigned*>(mail) + (wait ? (32 * (warp + u * kResWarps) + lane) / nt : (int)blockIdx.x);
           Patience pt;
-          for (;;) {                              // left by a warp vote, as above
+          for (bool last = false;;) {             // left by a warp vote, as above
             const bool ok = !wait || (int)(ld_relaxed_u32(flag) - xno) >= 0;
             if (__all_sync(0xffffffffu, ok)) break;
-            if (!pt.more(xw + 1, epoch + 1u, waits.limit_ns)) { bad = true; break; }
+            if (last) { bad = true; break; }
+            last = !pt.more(xw + 1, epoch + 1u, waits.limit_ns);
           }
           asm volatile("fence.acq_rel.gpu;" ::: "memory");   // acquire (a relaxed poll leaves L1 alone)
         }
@@ -813,10 +814,11 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
       if (__any_sync(0xffffffffu, wait)) {
         const unsigned* flag = reinterpret_cast<const unsigned*>(keeper_mail) + (wait ? tid : (int)blockIdx.x);
         Patience pt;
-        for (;;) {                              // left by a warp vote, as above
+        for (bool last = false;;) {             // left by a warp vote, as above
           const bool ok = !wait || (int)(ld_relaxed_u32(flag) - xend) >= 0;
           if (__all_sync(0xffffffffu, ok)) break;
-          if (!pt.more(xw + 1, epoch + 1u, waits.limit_ns)) { bad = true; break; }
+          if (last) { bad = true; break; }
+          last = !pt.more(xw + 1, epoch + 1u, waits.limit_ns);
         }
       }
       if (__syncthreads_or(bad)) failed = true;

@@ -575,7 +575,7 @@ long long gpu_bpf_debug_alloc_count(void);
 long long gpu_bpf_debug_live_allocs(void);
 
 /* Waits of resident runs (gpu_bpf_set_fused_small; testing aid). The CTAs of such a run wait on one
- * another, each wait at most 2 s; a run in which one gives up ends with BPF_ERR_STATE: step_many returns
+ * another, each wait at most 2 s of polling; a run in which one gives up ends with BPF_ERR_STATE: step_many returns
  * it, after step_many_device the next read-back does, and later runs do not start until gpu_bpf_reset or
  * gpu_bpf_load. This call sets the limit of this filter's waits (0 < limit_ms <= 2000) and one failure
  * made on purpose: fault 0 none; 1 CTA cta gives up in the run's exchange number `exchange` (1-based;
@@ -584,6 +584,10 @@ long long gpu_bpf_debug_live_allocs(void);
  * it runs out. No GPU fault is involved: the kernel returns. */
 int gpu_bpf_debug_resident(GpuBpfState* state, int fault, int cta, int exchange, double limit_ms);
 int gpu_apf_debug_resident(GpuApfState* state, int fault, int cta, int exchange, double limit_ms);
+/* The look (index into now_ns, the clock at each look, nonzero) at which such a wait of limit_ns gives up,
+ * n if it does not: the time between two looks counts as at most a sixteenth of the limit, so a GPU
+ * that was taken away for a while does not end the run. On the host. */
+int gpu_bpf_debug_wait_budget(const unsigned long long* now_ns, int n, unsigned long long limit_ns);
 
 /* Number of kernel launches this library has issued (all filters). */
 long long gpu_bpf_launch_count(void);
