@@ -464,6 +464,22 @@ static cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, cudaStream_t s, 
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+__global__ void __launch_bounds__(kGradThreads) grad_close_kernel(const DevState* st, BpfTickRecord* last, int N,
+                                                                  int32_t* csr, size_t n_csr, float2* aux, int T) {
+  if (st->error != BPF_ERR_STATE) return;
+  const size_t i0 = (size_t)blockIdx.x * kGradThreads + threadIdx.x, step = (size_t)gridDim.x * kGradThreads;
+  const double nan = __longlong_as_double(0x7FF8000000000000LL);
+  if (i0 == 0) last->loglik_total = nan;
+  for (size_t i = i0; i < n_csr; i += step) csr[i] = N;
+  for (size_t i = i0; i < (size_t)T; i += step) aux[i] = make_float2((float)nan, 0.0f);
+}
+
+cudaError_t launch_grad_close(const DevState* st, BpfTickRecord* last, int N, int32_t* csr, size_t csr_stride,
+                              float2* aux, int T, cudaStream_t s) {
+  grad_close_kernel<<<148, kGradThreads, 0, s>>>(st, last, N, csr, csr_stride * (size_t)T, aux, T);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_grad_seed(int N, const float* ckpt, float* h_out, PcgTick pc, int propagate_tick, float mu,
                              float rho, float sigma, int nu_int, float nu_state, cudaStream_t s, bool pdl) {
   return launch_pdl(grad_seed_kernel, grad_ctas(N), s, pdl, N, ckpt, h_out, pc, propagate_tick, mu, rho, sigma,

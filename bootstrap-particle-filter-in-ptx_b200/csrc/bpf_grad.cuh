@@ -80,6 +80,11 @@ struct ReplayArgs {
 inline int grad_ctas(int N) { return (N + kGradTile - 1) / kGradTile; }
 inline int grad_stride(int N) { return grad_ctas(N) * kGradTile; }
 
+// After the taped forward. A run in which a kernel gave up (BPF_ERR_STATE) has a tape with holes: its last
+// record's total log-likelihood becomes NaN, no parent has a child and every normaliser is NaN, so the
+// backward stays within the arrays and its gradient is NaN. Any other tape is left as it is.
+cudaError_t launch_grad_close(const DevState* st, BpfTickRecord* last, int N, int32_t* csr, size_t csr_stride,
+                              float2* aux, int T, cudaStream_t s);
 cudaError_t launch_grad_seed(int N, const float* ckpt, float* h_out, PcgTick pc, int propagate, float mu,
                              float rho, float sigma, int nu_int, float nu_state, cudaStream_t s, bool pdl);
 cudaError_t launch_grad_recompute(int N, const int32_t* csr, const float* hp, float* hc, PcgTick pc, float mu,

@@ -84,6 +84,7 @@ struct GpuBpfGrad {
   Plan plan{};
   int pass2_grid = 0;
   int res_tiles = 0;                 // largest filter of a resident run on the device (tiles)
+  ResidentWaits waits;               // of resident runs (gpu_bpf_grad_debug_resident)
   cudaStream_t stream = nullptr;
   bool pdl = true;
 
@@ -140,6 +141,14 @@ int ensure_dev(GpuBpfGrad* g) {
   return BPF_OK;
 }
 
+// Waits for the tape's stream; BPF_ERR_STATE when a kernel of the last forward run gave up.
+int taped_state(GpuBpfGrad* g) {
+  int error = BPF_OK;
+  GCK(cudaStreamSynchronize(g->stream));
+  GCK(cudaMemcpy(&error, &g->plan.st->error, sizeof(int), cudaMemcpyDeviceToHost));
+  return error == BPF_ERR_STATE ? bpf_record_error(BPF_ERR_STATE) : BPF_OK;
+}
+
 // init + T ticks of the plain filter with the tape hooks, then loglik_total -> ll
 cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
   const float std_stat = sqrtf((k.sigma * k.sigma) / fmaxf(1.0f - k.rho * k.rho, 1e-6f));   // gpu_bpf_ptx_full.cu:430
@@ -163,7 +172,7 @@ cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
     tape.K = g->K;
     tape.aux = g->aux;
     tape.hist = g->hist;
-    e = launch_resident(g->plan, a, tape, false, k.T, g->res_tiles, g->stream);
+    e = launch_resident(g->plan, a, tape, false, k.T, g->res_tiles, g->stream, g->waits);
   }
   for (int t = 0; t < k.T && e == cudaSuccess && !g->resident; ++t) {
     TickArgs a{};
@@ -182,6 +191,8 @@ cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
     if (e == cudaSuccess) e = launch_plan(g->plan, a, g->stream, g->pdl);
     if (e == cudaSuccess) e = launch_pass2(g->plan, a, g->pass2_grid, g->stream, g->pdl);
   }
+  if (e == cudaSuccess && k.T > 0)
+    e = launch_grad_close(g->plan.st, g->rec + k.T - 1, g->N, g->csr, (size_t)g->N4, g->aux, k.T, g->stream);
   if (e == cudaSuccess && k.T > 0)
     e = cudaMemcpyAsync(k.ll, &g->rec[k.T - 1].loglik_total, sizeof(double), cudaMemcpyDeviceToDevice, g->stream);
   return e;
@@ -320,6 +331,18 @@ void* gpu_bpf_grad_stream(GpuBpfGrad* g) { return g ? (void*)g->stream : nullptr
 
 int gpu_bpf_grad_checkpoint_every(GpuBpfGrad* g) { return g ? g->K : -bpf_record_error(BPF_ERR_STATE); }
 
+int gpu_bpf_grad_debug_resident(GpuBpfGrad* g, int fault, int cta, int exchange, double limit_ms) {
+  if (!g) return bpf_record_error(BPF_ERR_STATE);
+  ResidentWaits w;
+  if (!resident_waits_of(fault, cta, exchange, limit_ms, &w)) return bpf_record_error(BPF_ERR_ARG);
+  int rc = ensure_dev(g);
+  if (rc) return rc;
+  GCK(cudaStreamSynchronize(g->stream));
+  if (g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }   // it holds the waits
+  g->waits = w;
+  return BPF_OK;
+}
+
 int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, float nu_state, float nu_obs, int seed,
                          float ess_threshold, const float* y_dev, int n_ticks, double* loglik_dev) {
   if (!g) return bpf_record_error(BPF_ERR_STATE);
@@ -351,7 +374,7 @@ int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, floa
     g->fkey = k;
   }
   GCK(cudaGraphLaunch(g->fgraph, g->stream));
-  bpf_note_launches(g->resident ? 2 : 1 + 3LL * n_ticks);
+  bpf_note_launches(g->resident ? 3 : 2 + 3LL * n_ticks);
   g->cur = k;
   g->have_fwd = true;
   g->pcs.resize(n_ticks + 1);
@@ -392,6 +415,7 @@ int gpu_bpf_grad_replay(GpuBpfGrad* g, double mu, double rho, double sigma_z, do
       !(sigma_z > 0.0))
     return bpf_record_error(BPF_ERR_ARG);
   int rc = ensure_dev(g);
+  if (!rc) rc = taped_state(g);
   if (rc) return rc;
   const size_t N4 = (size_t)g->N4;
   cudaError_t e = cudaSuccess;
@@ -437,8 +461,8 @@ int gpu_bpf_grad_get_records(GpuBpfGrad* g, BpfTickRecord* out, int n) {
   if (!g || !g->have_fwd) return bpf_record_error(BPF_ERR_STATE);
   if (!out || n < 0 || n > g->cur.T) return bpf_record_error(BPF_ERR_ARG);
   int rc = ensure_dev(g);
+  if (!rc) rc = taped_state(g);
   if (rc) return rc;
-  GCK(cudaStreamSynchronize(g->stream));
   GCK(cudaMemcpy(out, g->rec, (size_t)n * sizeof(BpfTickRecord), cudaMemcpyDeviceToHost));
   return BPF_OK;
 }
@@ -447,8 +471,8 @@ int gpu_bpf_grad_get_children(GpuBpfGrad* g, int tick, int32_t* first_child) {
   if (!g || !g->have_fwd) return bpf_record_error(BPF_ERR_STATE);
   if (!first_child || tick < 0 || tick >= g->cur.T) return bpf_record_error(BPF_ERR_ARG);
   int rc = ensure_dev(g);
+  if (!rc) rc = taped_state(g);
   if (rc) return rc;
-  GCK(cudaStreamSynchronize(g->stream));
   GCK(cudaMemcpy(first_child, g->csr + (size_t)tick * g->N4, (size_t)g->N * sizeof(int32_t),
                  cudaMemcpyDeviceToHost));
   return BPF_OK;

@@ -489,7 +489,9 @@ int         gpu_bpf_grad_checkpoint_every(GpuBpfGrad* grad);
 /* Taped forward run from a fresh start (as gpu_bpf_create + reset(seed) + n_ticks steps;
  * nu_state and nu_obs as in gpu_bpf_create):
  * y_dev[n_ticks] in, loglik_dev[0] = FP64 total log-likelihood out. Enqueued on the tape's
- * stream. ess_threshold must be 0 (BPF_ERR_UNSUPPORTED otherwise). */
+ * stream. ess_threshold must be 0 (BPF_ERR_UNSUPPORTED otherwise). Where a kernel of the run gave up
+ * waiting (gpu_bpf_debug_resident) the log-likelihood and its gradient are NaN, and replay, get_records
+ * and get_children return BPF_ERR_STATE. */
 int gpu_bpf_grad_forward(GpuBpfGrad* grad, float mu, float rho, float sigma_z, float nu_state, float nu_obs,
                          int seed, float ess_threshold, const float* y_dev, int n_ticks, double* loglik_dev);
 /* Adjoint of the last taped run: grad_dev[3] = d loglik / d(mu, rho, sigma_z), FP64. */
@@ -584,6 +586,7 @@ long long gpu_bpf_debug_live_allocs(void);
  * it runs out. No GPU fault is involved: the kernel returns. */
 int gpu_bpf_debug_resident(GpuBpfState* state, int fault, int cta, int exchange, double limit_ms);
 int gpu_apf_debug_resident(GpuApfState* state, int fault, int cta, int exchange, double limit_ms);
+int gpu_bpf_grad_debug_resident(GpuBpfGrad* grad, int fault, int cta, int exchange, double limit_ms);
 /* The look (index into now_ns, the clock at each look, nonzero) at which such a wait of limit_ns gives up,
  * n if it does not: the time between two looks counts as at most a sixteenth of the limit, so a GPU
  * that was taken away for a while does not end the run. On the host. */

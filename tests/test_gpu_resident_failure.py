@@ -86,3 +86,33 @@ def test_rejects_bad_arguments(bpf):
                  (1, 0, 1, math.nan)):
         assert f._lib.gpu_bpf_debug_resident(f._s, *args) == _lib.BPF_ERR_ARG
     f.close()
+
+
+@pytest.mark.parametrize("every", [0, 4])
+@pytest.mark.parametrize("N,fault,cta,exchange", [(70001, EXCHANGE, 0, T), (70001, FLAGS, 1, 6), (700001, FLAGS, 0, T),
+                                                  (70001, WITHHOLD, 3, 1)])
+def test_tape_with_a_wait_given_up_has_no_gradient(bpf, N, fault, cta, exchange, every):
+    """With and without the particles of every tick kept: NaN from forward and backward, an error from the
+    calls that read the tape, and a sound tape from the next forward run."""
+    import torch
+    from gpubpf import _lib
+    y = torch.tensor(_series(T, 9), device="cuda")
+    theta = (MU, RHO, SIG)
+
+    def clean(tape):
+        return tape.forward(theta, y, seed=8).item(), tape.backward().cpu().numpy().tobytes(), bytes(tape.children(T - 2))
+
+    other = bpf.GradTape(N, T, checkpoint_every=every)
+    want = clean(other)
+    other.close()
+    tape = bpf.GradTape(N, T, checkpoint_every=every)
+    assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, cta, exchange, 20.0) == _lib.BPF_OK
+    assert math.isnan(tape.forward(theta, y, seed=8).item())      # a tape that no run has filled before
+    assert np.isnan(tape.backward().cpu().numpy()).all()
+    for read in (tape.records, lambda: tape.children(0), lambda: tape.replay(theta)):
+        with pytest.raises(bpf.BpfError) as e:
+            read()
+        assert e.value.code == _lib.BPF_ERR_STATE
+    assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, 0, 0, 0, 2000.0) == _lib.BPF_OK
+    assert clean(tape) == want
+    tape.close()
