@@ -52,7 +52,7 @@ struct ApfImpl {
   int device = 0;
   Plan plan{};
   int pass2_grid = 0;
-  int res_tiles = 0;                  // largest filter of a resident run on the device (tiles)
+  int res_tiles = 0;                  // largest filter of a resident run on the device (tiles; 0 once one was refused)
   ResidentWaits waits;                // of resident runs (gpu_apf_debug_resident)
   cudaStream_t stream = nullptr;
   BpfTickRecord* rec_dev = nullptr;   // [1 + kApfRun]: slot 0 single step, 1.. a chunk's ticks
@@ -257,7 +257,9 @@ void gpu_apf_destroy(GpuApfState* s) {
 int gpu_apf_debug_resident(GpuApfState* s, int fault, int cta, int exchange, double limit_ms) {
   ApfImpl* m = impl_of(s);
   if (!m) return set_err(BPF_ERR_STATE);
-  return resident_waits_of(fault, cta, exchange, limit_ms, &m->waits) ? BPF_OK : set_err(BPF_ERR_ARG);
+  if (!resident_waits_of(fault, cta, exchange, limit_ms, &m->waits)) return set_err(BPF_ERR_ARG);
+  m->res_tiles = resident_max_tiles(m->device);
+  return BPF_OK;
 }
 
 int gpu_apf_step_many(GpuApfState* s, const float* y, int n_ticks, BpfResult* out, BpfTickRecord* rec) {
@@ -278,7 +280,12 @@ int gpu_apf_step_many(GpuApfState* s, const float* y, int n_ticks, BpfResult* ou
       ACK(cudaMemcpyAsync(m->y_dev, m->y_pin, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
       TickArgs a = make_args(s, m, 0.0f, m->y_dev);
       a.rec = m->rec_dev + 1;
-      ACK(launch_resident(m->plan, a, ResidentTape{}, true, n, m->res_tiles, m->stream, m->waits));
+      const cudaError_t e = launch_resident(m->plan, a, ResidentTape{}, true, n, m->res_tiles, m->stream, m->waits);
+      if (e != cudaSuccess) {           // refused: kernel by kernel from now on
+        cudaGetLastError();
+        m->res_tiles = 0;
+        continue;
+      }
       bpf_note_launches(1);
       ACK(cudaMemcpyAsync(m->rec_pin + 1, m->rec_dev + 1, n * sizeof(BpfTickRecord), cudaMemcpyDeviceToHost,
                           m->stream));

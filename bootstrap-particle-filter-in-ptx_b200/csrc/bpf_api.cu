@@ -98,7 +98,8 @@ struct Impl {
   BpfTickRecord* dg_rec = nullptr;
   int dg_n = 0;
   float dg_mu = NAN, dg_rho = NAN, dg_sigma = NAN, dg_thr = NAN, dg_nus = NAN, dg_silv = NAN;
-  bool dg_anc = false;
+  bool dg_anc = false, dg_resident = false;
+  long long dg_launches = 0;
 
   // programmatic dependent launch between consecutive kernels (off while profiling)
   bool pdl = true;
@@ -107,7 +108,7 @@ struct Impl {
   // fused launch (gpu_bpf_set_fused_small)
   bool fused_small = true;
   int small_tiles = 4;                  // largest fused cluster on the filter's device (tiles)
-  int res_tiles = 0;                    // largest filter of a resident run on it (tiles)
+  int res_tiles = 0;                    // largest filter of a resident run on it (tiles; 0 once one was refused)
   ResidentWaits waits;                  // of resident runs (gpu_bpf_debug_resident)
 
   // profiling
@@ -383,6 +384,8 @@ int build_device_graph(GpuBpfState* s, Impl* m, const float* y_dev, int n, BpfTi
   cudaGraph_t g = nullptr;
   const TickArgs a0 = make_args(s, m, 0.0f, y_dev, rec_dev);
   const bool one = one_launch(m, a0);                                   // (configures outside the capture)
+  m->dg_resident = one && !use_small(m, a0);
+  m->dg_launches = one ? 1 : (long long)tick_launches(m, a0) * n;
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
   if (one) {
@@ -394,10 +397,16 @@ int build_device_graph(GpuBpfState* s, Impl* m, const float* y_dev, int n, BpfTi
     }
   }
   cudaError_t e2 = cudaStreamEndCapture(m->stream, &g);
-  if (err != cudaSuccess || e2 != cudaSuccess) { if (g) cudaGraphDestroy(g); cudaGetLastError(); return set_err(BPF_ERR_CUDA); }
-  cudaError_t e3 = cudaGraphInstantiate(&m->dgraph, g, 0);
-  cudaGraphDestroy(g);
-  if (e3 != cudaSuccess) { m->dgraph = nullptr; return set_err(BPF_ERR_CUDA); }
+  if (err == cudaSuccess) err = e2;
+  if (err == cudaSuccess) err = cudaGraphInstantiate(&m->dgraph, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (err != cudaSuccess) {
+    cudaGetLastError();
+    m->dgraph = nullptr;
+    if (!m->dg_resident) return set_err(BPF_ERR_CUDA);
+    m->res_tiles = 0;                                                   // refused: tick by tick from now on
+    return build_device_graph(s, m, y_dev, n, rec_dev);
+  }
   m->dg_y = y_dev; m->dg_rec = rec_dev; m->dg_n = n;
   m->dg_mu = s->mu; m->dg_rho = s->rho; m->dg_sigma = s->sigma_z; m->dg_thr = s->ess_threshold;
   m->dg_nus = s->nu_state;
@@ -731,24 +740,31 @@ int gpu_bpf_step_many(GpuBpfState* s, const float* y, int n_ticks, BpfResult* ou
   if (rc) return rc;
   int t = 0;
   int last = 0;                                     // the last tick's place in its chunk
-  if (one_launch(m, make_args(s, m, 0.0f, m->y_dev, m->rec_dev + 1))) {
-    while (n_ticks - t > 1) {                       // (a single tick has less to load as kernels)
-      const int n = std::min(kRunChunk, n_ticks - t);
-      std::memcpy(m->y_pin, y + t, n * sizeof(float));
-      CK(cudaMemcpyAsync(m->y_dev, m->y_pin, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-      CK(launch_run(m, make_args(s, m, 0.0f, m->y_dev, m->rec_dev + 1), n));
-      CK(cudaMemcpyAsync(m->rec_pin + 1, m->rec_dev + 1, n * sizeof(BpfTickRecord), cudaMemcpyDeviceToHost, m->stream));
-      CK(cudaStreamSynchronize(m->stream));
-      g_launches += 1;
-      m->ticks_enqueued += n;
-      for (int k = 0; k < n; ++k) {
-        if (out) out[t + k] = to_result(m, m->rec_pin[1 + k]);
-        if (rec) rec[t + k] = m->rec_pin[1 + k];
-      }
-      t += n;
-      last = n - 1;
+  while (n_ticks - t > 1) {                         // (a single tick has less to load as kernels)
+    const TickArgs a = make_args(s, m, 0.0f, m->y_dev, m->rec_dev + 1);
+    if (!one_launch(m, a)) break;
+    const int n = std::min(kRunChunk, n_ticks - t);
+    std::memcpy(m->y_pin, y + t, n * sizeof(float));
+    CK(cudaMemcpyAsync(m->y_dev, m->y_pin, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    const cudaError_t e = launch_run(m, a, n);
+    if (e != cudaSuccess && !use_small(m, a)) {     // refused: tick by tick from now on
+      cudaGetLastError();
+      m->res_tiles = 0;
+      break;
     }
-  } else if (!m->profiling && !m->learn_mode) {     // learning updates need the host every K ticks
+    CK(e);
+    CK(cudaMemcpyAsync(m->rec_pin + 1, m->rec_dev + 1, n * sizeof(BpfTickRecord), cudaMemcpyDeviceToHost, m->stream));
+    CK(cudaStreamSynchronize(m->stream));
+    g_launches += 1;
+    m->ticks_enqueued += n;
+    for (int k = 0; k < n; ++k) {
+      if (out) out[t + k] = to_result(m, m->rec_pin[1 + k]);
+      if (rec) rec[t + k] = m->rec_pin[1 + k];
+    }
+    t += n;
+    last = n - 1;
+  }
+  if (!m->profiling && !m->learn_mode) {            // learning updates need the host every K ticks
     while (n_ticks - t >= kGraphChunk) {
       if (graph_stale(s, m)) { rc = build_graph(s, m); if (rc) return rc; }
       std::memcpy(m->y_pin, y + t, kGraphChunk * sizeof(float));
@@ -810,9 +826,16 @@ int gpu_bpf_step_many_device(GpuBpfState* s, const float* y_dev, int n_ticks, Bp
                        m->dg_thr != s->ess_threshold || m->dg_nus != s->nu_state ||
                        m->dg_silv != s->silverman_shrink || m->dg_anc != m->record_anc;
     if (stale) { rc = build_device_graph(s, m, y_dev, n_ticks, rec_dev); if (rc) return rc; }
-    CK(cudaGraphLaunch(m->dgraph, m->stream));
-    g_launches += one_launch(m, make_args(s, m, 0.0f, nullptr, nullptr))
-                      ? 1 : (long long)tick_launches(m, make_args(s, m, 0.0f, nullptr, nullptr)) * n_ticks;
+    cudaError_t e = cudaGraphLaunch(m->dgraph, m->stream);
+    if (e != cudaSuccess && m->dg_resident) {         // refused at the launch
+      cudaGetLastError();
+      m->res_tiles = 0;
+      rc = build_device_graph(s, m, y_dev, n_ticks, rec_dev);
+      if (rc) return rc;
+      e = cudaGraphLaunch(m->dgraph, m->stream);
+    }
+    CK(e);
+    g_launches += m->dg_launches;
     m->ticks_enqueued += n_ticks;
   } else {
     for (int t = 0; t < n_ticks; ++t) {
@@ -1083,6 +1106,7 @@ int gpu_bpf_debug_resident(GpuBpfState* s, int fault, int cta, int exchange, dou
   CK(cudaStreamSynchronize(m->stream));
   if (m->dgraph) { cudaGraphExecDestroy(m->dgraph); m->dgraph = nullptr; }   // it holds the waits
   m->waits = w;
+  m->res_tiles = resident_max_tiles(m->device);
   return BPF_OK;
 }
 

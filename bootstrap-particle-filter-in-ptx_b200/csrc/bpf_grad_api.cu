@@ -46,7 +46,8 @@ struct FwdKey {
 struct BwdKey {
   FwdKey f;
   double* grad = nullptr;
-  bool operator==(const BwdKey& o) const { return f == o.f && grad == o.grad; }
+  bool kept = false;       // the particles of every tick are on the tape
+  bool operator==(const BwdKey& o) const { return f == o.f && grad == o.grad && kept == o.kept; }
 };
 
 int nu_int_of(float nu_state) { return nu_state > 0.0f ? (int)(nu_state + 0.5f) : 0; }   // gpu_bpf_ptx_full.cu:392
@@ -83,7 +84,7 @@ struct GpuBpfGrad {
   size_t ckpt_stride = 0;
   Plan plan{};
   int pass2_grid = 0;
-  int res_tiles = 0;                 // largest filter of a resident run on the device (tiles)
+  int res_tiles = 0;                 // largest filter of a resident run on the device (tiles; 0 once one was refused)
   ResidentWaits waits;               // of resident runs (gpu_bpf_grad_debug_resident)
   cudaStream_t stream = nullptr;
   bool pdl = true;
@@ -204,7 +205,7 @@ cudaError_t enqueue_backward(GpuBpfGrad* g, const BwdKey& bk) {
   const ObsModel obs = make_obs(k.nu);
   const int nui = nu_int_of(k.nu_state);
   cudaError_t e = cudaMemsetAsync(g->acc, 0, (size_t)g->G1 * kGradAcc * sizeof(double), g->stream);
-  const bool kept = g->hist && g->resident;      // every tick's particles are on the tape
+  const bool kept = bk.kept;
   const int nseg = (T + K - 1) / K;
   for (int s = nseg - 1; s >= 0 && e == cudaSuccess; --s) {
     const int c = s * K, last = std::min(c + K, T) - 1;
@@ -340,6 +341,7 @@ int gpu_bpf_grad_debug_resident(GpuBpfGrad* g, int fault, int cta, int exchange,
   GCK(cudaStreamSynchronize(g->stream));
   if (g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }   // it holds the waits
   g->waits = w;
+  g->res_tiles = resident_max_tiles(g->device);
   return BPF_OK;
 }
 
@@ -369,11 +371,23 @@ int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, floa
     }
     if (g->hist && g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }
   }
-  if (!g->fgraph || !(g->fkey == k)) {
-    GCK(capture(g, &g->fgraph, [&]() { return enqueue_forward(g, k); }));
-    g->fkey = k;
+  auto launch = [&]() {
+    if (!g->fgraph || !(g->fkey == k)) {
+      const cudaError_t e = capture(g, &g->fgraph, [&]() { return enqueue_forward(g, k); });
+      if (e != cudaSuccess) return e;
+      g->fkey = k;
+    }
+    return cudaGraphLaunch(g->fgraph, g->stream);
+  };
+  cudaError_t e = launch();
+  if (e != cudaSuccess && g->resident) {               // refused: three kernels a tick from now on
+    cudaGetLastError();
+    g->res_tiles = 0;
+    g->resident = false;
+    if (g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }
+    e = launch();
   }
-  GCK(cudaGraphLaunch(g->fgraph, g->stream));
+  GCK(e);
   bpf_note_launches(g->resident ? 3 : 2 + 3LL * n_ticks);
   g->cur = k;
   g->have_fwd = true;
@@ -396,6 +410,7 @@ int gpu_bpf_grad_backward(GpuBpfGrad* g, double* grad_dev) {
   BwdKey bk;
   bk.f = g->cur;
   bk.grad = grad_dev;
+  bk.kept = g->hist && g->resident;
   if (!g->bgraph || !(g->bkey == bk)) {
     GCK(capture(g, &g->bgraph, [&]() { return enqueue_backward(g, bk); }));
     g->bkey = bk;

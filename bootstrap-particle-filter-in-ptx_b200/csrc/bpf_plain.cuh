@@ -143,7 +143,8 @@ cudaError_t launch_small(const Plan& p, const TickArgs& a, int n_ticks, cudaStre
 // Resident runs (bpf_resident.cu): n_ticks consecutive ticks of a filter of at most
 // resident_max_tiles(device) tiles in one cooperative launch, bit-identical to the tick-per-launch
 // path. a.y_ptr and a.rec point at the run's first tick; apf: auxiliary-filter ticks (threshold 0).
-// Not for learning, Silverman or mirrored ticks.
+// Not for learning, Silverman or mirrored ticks. The launch is refused where the whole grid does not fit
+// on what the process may use of the device; the caller then takes the ticks one by one.
 struct ResidentTape {        // gradient tape of a taped run from tick 0 (all null otherwise)
   int32_t* csr; size_t csr_stride;     // first child slots, tick t's at csr + t * csr_stride
   float* ckpt; size_t ckpt_stride;     // particles entering every K-th tick
@@ -153,7 +154,8 @@ struct ResidentTape {        // gradient tape of a taped run from tick 0 (all nu
 };
 // How long a wait of a resident run polls before it gives up and, in tests, one failure made on
 // purpose: CTA cta gives up in exchange xn (1-based in the run) or in the wait for the children of its
-// resampling, or does not publish its record of that exchange. No wait outlasts its limit.
+// resampling, or does not publish its record of that exchange; or the launch is refused on the host, as
+// one that does not fit on the device is. No wait outlasts its limit.
 constexpr unsigned long long kResWaitNs = 2000000000ull;
 // Time spent polling against that limit, from the clock at one look after another. The time between two
 // looks counts as at most a sixteenth of the limit: while the GPU runs another program, or the grid is
@@ -167,14 +169,14 @@ struct WaitBudget {
     return spent >= limit;
   }
 };
-enum ResidentFault { kFaultNone = 0, kFaultExchange = 1, kFaultFlags = 2, kFaultWithhold = 3 };
+enum ResidentFault { kFaultNone = 0, kFaultExchange = 1, kFaultFlags = 2, kFaultWithhold = 3, kFaultRefused = 4 };
 struct ResidentWaits {
   unsigned long long limit_ns = kResWaitNs;
   int fault = kFaultNone, cta = 0;
   unsigned xn = 0u;
 };
 inline bool resident_waits_of(int fault, int cta, int exchange, double limit_ms, ResidentWaits* out) {
-  if (fault < kFaultNone || fault > kFaultWithhold || cta < 0 || exchange < 0 ||
+  if (fault < kFaultNone || fault > kFaultRefused || cta < 0 || exchange < 0 ||
       !(limit_ms > 0.0 && limit_ms <= (double)kResWaitNs * 1e-6))
     return false;
   out->limit_ns = (unsigned long long)(limit_ms * 1e6);

@@ -900,6 +900,7 @@ bool resident_ready(int device, int G, int max_tiles, bool tstate, bool gauss, b
 cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
                             int max_tiles, cudaStream_t s, const ResidentWaits& waits) {
   if (!p.xbuf || p.G < 1 || p.G > max_tiles || n_ticks < 1 || !a.y_ptr) return cudaErrorInvalidValue;
+  if (waits.fault == kFaultRefused) return cudaErrorCooperativeLaunchTooLarge;
   const int sms = max_tiles / kResMaxTilesPerCta;
   const int nt = (p.G + sms - 1) / sms;
   size_t smem = 0;

@@ -583,7 +583,9 @@ long long gpu_bpf_debug_live_allocs(void);
  * made on purpose: fault 0 none; 1 CTA cta gives up in the run's exchange number `exchange` (1-based;
  * one per tick, two per auxiliary-filter tick after the first); 2 it gives up waiting for the children
  * of that exchange's resampling; 3 it does not publish its record of that exchange, so every wait for
- * it runs out. No GPU fault is involved: the kernel returns. */
+ * it runs out; 4 the launch is refused, as where the whole grid does not fit on what the process may use
+ * of the device: the ticks then run one by one, and the object makes no other attempt until the next
+ * call of this function. No GPU fault is involved: the kernel returns. */
 int gpu_bpf_debug_resident(GpuBpfState* state, int fault, int cta, int exchange, double limit_ms);
 int gpu_apf_debug_resident(GpuApfState* state, int fault, int cta, int exchange, double limit_ms);
 int gpu_bpf_grad_debug_resident(GpuBpfGrad* grad, int fault, int cta, int exchange, double limit_ms);

@@ -82,7 +82,7 @@ def test_auxiliary_run_with_a_wait_given_up_reports_it(bpf, N, fault, cta, excha
 def test_rejects_bad_arguments(bpf):
     from gpubpf import _lib
     f = bpf.GpuBpf(70000, RHO, SIG, MU, seed=3)
-    for args in ((4, 0, 1, 10.0), (-1, 0, 1, 10.0), (1, -1, 1, 10.0), (1, 0, -1, 10.0), (1, 0, 1, 0.0), (1, 0, 1, 2001.0),
+    for args in ((5, 0, 1, 10.0), (-1, 0, 1, 10.0), (1, -1, 1, 10.0), (1, 0, -1, 10.0), (1, 0, 1, 0.0), (1, 0, 1, 2001.0),
                  (1, 0, 1, math.nan)):
         assert f._lib.gpu_bpf_debug_resident(f._s, *args) == _lib.BPF_ERR_ARG
     f.close()
@@ -116,3 +116,90 @@ def test_tape_with_a_wait_given_up_has_no_gradient(bpf, N, fault, cta, exchange,
     assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, 0, 0, 0, 2000.0) == _lib.BPF_OK
     assert clean(tape) == want
     tape.close()
+
+
+REFUSED = 4
+
+
+@pytest.mark.parametrize("N,ticks", [(70000, 70), (1000003, 12)])
+def test_refused_run_goes_tick_by_tick(bpf, N, ticks):
+    """A cooperative launch that the device refuses: the same results from the kernels of a tick, from host
+    and device observations, with no error and no other attempt."""
+    import torch
+    y = _series(ticks, 5)
+    yd = torch.tensor(y, device="cuda")
+
+    def run(fault, fused):
+        rec = torch.zeros(ticks * 40, dtype=torch.uint8, device="cuda")
+        f = bpf.GpuBpf(N, RHO, SIG, MU, seed=3, ess_threshold=0.5)
+        f.set_fused_small(fused)
+        _arm(f, "gpu_bpf_debug_resident", fault)
+        n0 = f._lib.gpu_bpf_launch_count()
+        out = [bytes(r) for r in f.step_many(y.tolist(), records=True)] + [bytes(f.get_particles())]
+        n1 = f._lib.gpu_bpf_launch_count()
+        for _ in range(2):
+            f.reset(7)
+            f.step_many_device(yd.data_ptr(), ticks, rec.data_ptr())
+            out += [bytes(f.get_record()), bytes(f.get_particles()), rec.cpu().numpy().tobytes()]
+        n2 = f._lib.gpu_bpf_launch_count()
+        f.close()
+        return out, n1 - n0, n2 - n1
+
+    resident, refused, plain = run(0, True), run(REFUSED, True), run(0, False)
+    assert resident[0] == refused[0] == plain[0]
+    assert resident[1] == 1 and refused[1:] == plain[1:] and refused[1] >= 2 * ticks
+
+
+def test_refused_device_run_first(bpf):
+    """The refusal met while the device run is captured."""
+    import torch
+    y = torch.tensor(_series(T, 5), device="cuda")
+    out = []
+    for fault in (0, REFUSED):
+        rec = torch.zeros(T * 40, dtype=torch.uint8, device="cuda")
+        f = bpf.GpuBpf(300000, RHO, SIG, MU, seed=3, ess_threshold=0.0)
+        _arm(f, "gpu_bpf_debug_resident", fault)
+        f.step_many_device(y.data_ptr(), T, rec.data_ptr())
+        out.append((bytes(f.get_record()), bytes(f.get_particles()), rec.cpu().numpy().tobytes()))
+        f.close()
+    assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("N", [5000, 300000])
+def test_refused_auxiliary_run_goes_kernel_by_kernel(bpf, N):
+    """70 + 66 ticks: single ticks, then the 64-tick graph and a remainder."""
+    y = _series(136, 5).tolist()
+    out = []
+    for fault in (0, REFUSED):
+        f = bpf.GpuApf(N, RHO, SIG, MU, seed=3)
+        _arm(f, "gpu_apf_debug_resident", fault)
+        recs = f.step_many(y[:70], records=True)
+        recs += f.step_many(y[70:], records=True)
+        out.append(([bytes(r) for r in recs], bytes(f.get_particles()), f.get_loglik_total()))
+        f.close()
+    assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("every", [0, 4])
+@pytest.mark.parametrize("N,nu_state,nu_obs", [(3, 0.0, 0.0), (70001, 0.0, 5.0), (700001, 5.0, 0.0)])
+def test_refused_tape_is_taped_by_the_kernels(bpf, N, nu_state, nu_obs, every):
+    """The three kernels a tick write the tape that the resident run writes: log-likelihood, records, child
+    lists and gradient, bit for bit, whichever of the two a tape has used before."""
+    import torch
+    y = torch.tensor(_series(37, 6), device="cuda")
+
+    def read(tape, seed):
+        ll = tape.forward((MU, RHO, SIG), y, seed=seed, nu_obs=nu_obs, nu_state=nu_state).item()
+        return (ll, tape.backward().cpu().numpy().tobytes(), [bytes(r) for r in tape.records()],
+                [tape.children(t).tobytes() for t in (0, 17, 35)])
+
+    out = []
+    for faults in ((0, 0), (REFUSED, REFUSED), (0, REFUSED), (REFUSED, 0)):
+        tape = bpf.GradTape(N, 37, checkpoint_every=every)
+        got = []
+        for fault, seed in zip(faults, (3, 9)):
+            assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, 0, 0, 2000.0) == 0
+            got.append(read(tape, seed))
+        tape.close()
+        out.append(got)
+    assert out[0] == out[1] == out[2] == out[3]
