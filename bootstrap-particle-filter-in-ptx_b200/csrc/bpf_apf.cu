@@ -33,7 +33,7 @@ using namespace bpf;
 namespace {
 
 constexpr int kApfChunk = 64;   // ticks per captured graph in gpu_apf_step_many
-constexpr int kApfRun = 1024;   // ticks per resident launch there
+constexpr int kApfRun = kResRunTicks;   // ticks per resident launch there
 
 inline int set_err(int code) { return bpf_record_error(code); }
 

@@ -44,7 +44,7 @@ namespace {
 constexpr int kGraphChunk = 64;   // ticks per captured graph
 // Ticks per launch of a host run that is one launch a chunk (fused small filters, resident runs): with
 // 64 a synchronise, two copies and the particles' way in and out of the chip cost 0.2-0.9 us per tick.
-constexpr int kRunChunk = 1024;
+constexpr int kRunChunk = kResRunTicks;
 
 struct Impl {
   int device = 0;
@@ -148,7 +148,8 @@ bool use_resident(const Impl* m, const TickArgs& a) {
          !(a.silverman > 0.0f) &&
          resident_ready(m->device, m->plan.G, m->res_tiles, a.nu_int > 0, !(a.obs.nu > 0.0f), false);
 }
-// Whether a run of ticks is one launch, and that launch (a.y_ptr, a.rec: the run's first tick).
+// Whether a run of ticks is one launch (a resident run: one per kResRunTicks ticks), and that launch
+// (a.y_ptr, a.rec: the run's first tick).
 bool one_launch(const Impl* m, const TickArgs& a) { return use_small(m, a) || use_resident(m, a); }
 cudaError_t launch_run(Impl* m, const TickArgs& a, int n_ticks) {
   if (use_small(m, a)) return launch_small(m->plan, a, n_ticks, m->stream, m->pdl);
@@ -385,11 +386,11 @@ int build_device_graph(GpuBpfState* s, Impl* m, const float* y_dev, int n, BpfTi
   const TickArgs a0 = make_args(s, m, 0.0f, y_dev, rec_dev);
   const bool one = one_launch(m, a0);                                   // (configures outside the capture)
   m->dg_resident = one && !use_small(m, a0);
-  m->dg_launches = one ? 1 : (long long)tick_launches(m, a0) * n;
+  m->dg_launches = m->dg_resident ? resident_launches(n) : (one ? 1 : (long long)tick_launches(m, a0) * n);
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
   if (one) {
-    err = launch_run(m, a0, n);                                         // the whole run as one launch
+    err = launch_run(m, a0, n);                                         // the whole run
   } else {
     for (int k = 0; k < n && err == cudaSuccess; ++k) {
       TickArgs a = make_args(s, m, 0.0f, y_dev + k, rec_dev + k);

@@ -112,7 +112,7 @@ struct GpuBpfGrad {
 
   // the taped run
   bool have_fwd = false;
-  bool resident = false;             // the forward run is one resident launch
+  bool resident = false;             // the forward run is resident launches
   FwdKey cur;
   std::vector<PcgTick> pcs;          // noise constants of ticks 0..T
 
@@ -156,8 +156,8 @@ cudaError_t enqueue_forward(GpuBpfGrad* g, const FwdKey& k) {
   cudaError_t e = launch_init(g->plan, k.mu, std_stat, k.seed, g->stream);
   const ObsModel obs = make_obs(k.nu);
   if (e == cudaSuccess && k.T > 0 && g->resident) {
-    // The whole taped run as one resident launch: N = 2^20 26 -> 14 us per tick, and three nodes to
-    // capture anew for every theta instead of three per tick.
+    // The taped run as resident launches: N = 2^20 26 -> 14 us per tick, and four nodes to capture anew
+    // for every theta instead of three per tick.
     TickArgs a{};
     a.mu = k.mu; a.rho = k.rho; a.sigma = k.sigma;
     a.ess_threshold = 0.0f;
@@ -388,7 +388,7 @@ int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, floa
     e = launch();
   }
   GCK(e);
-  bpf_note_launches(g->resident ? 3 : 2 + 3LL * n_ticks);
+  bpf_note_launches(2 + (g->resident ? (long long)resident_launches(n_ticks) : 3LL * n_ticks));
   g->cur = k;
   g->have_fwd = true;
   g->pcs.resize(n_ticks + 1);

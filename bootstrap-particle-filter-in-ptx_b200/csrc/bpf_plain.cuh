@@ -141,10 +141,15 @@ cudaError_t launch_jitter(const Plan& p, const TickArgs& a, cudaStream_t s, bool
 bool small_eligible(const Plan& p, const TickArgs& a);
 cudaError_t launch_small(const Plan& p, const TickArgs& a, int n_ticks, cudaStream_t s, bool pdl);
 // Resident runs (bpf_resident.cu): n_ticks consecutive ticks of a filter of at most
-// resident_max_tiles(device) tiles in one cooperative launch, bit-identical to the tick-per-launch
-// path. a.y_ptr and a.rec point at the run's first tick; apf: auxiliary-filter ticks (threshold 0).
-// Not for learning, Silverman or mirrored ticks. The launch is refused where the whole grid does not fit
-// on what the process may use of the device; the caller then takes the ticks one by one.
+// resident_max_tiles(device) tiles, bit-identical to the tick-per-launch path, as cooperative launches of
+// at most kResRunTicks ticks: a launch holds its SMs from end to end, and this is how long other
+// streams' work may have to wait for them (4 to 25 ms; the particles' way in and out of the chip
+// between two launches costs a few us). a.y_ptr and a.rec point at the run's first tick; apf:
+// auxiliary-filter ticks (threshold 0). Not for learning, Silverman or mirrored ticks. A launch is
+// refused where the whole grid does not fit on what the process may use of the device; the caller then
+// takes the ticks one by one.
+constexpr int kResRunTicks = 1024;
+inline int resident_launches(int n_ticks) { return (n_ticks + kResRunTicks - 1) / kResRunTicks; }
 struct ResidentTape {        // gradient tape of a taped run from tick 0 (all null otherwise)
   int32_t* csr; size_t csr_stride;     // first child slots, tick t's at csr + t * csr_stride
   float* ckpt; size_t ckpt_stride;     // particles entering every K-th tick

@@ -32,6 +32,7 @@
 // waits for all of them: whichever CTA gave up, the run ends with BPF_ERR_STATE, and a later run
 // does not start on such a state.
 #include "bpf_tick.cuh"
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -915,7 +916,14 @@ cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, p, a, tape, waits, n_ticks, nt);
+  cudaError_t e = cudaSuccess;
+  for (int t = 0; t < n_ticks && e == cudaSuccess; t += kResRunTicks) {
+    TickArgs run = a;
+    run.y_ptr = a.y_ptr + t;
+    run.rec = a.rec ? a.rec + t : nullptr;
+    e = cudaLaunchKernelEx(&cfg, k, p, run, tape, waits, std::min(kResRunTicks, n_ticks - t), nt);
+  }
+  return e;
 }
 
 }  // namespace bpf

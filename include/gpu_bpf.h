@@ -242,9 +242,13 @@ int    gpu_bpf_load(GpuBpfState* state, const void* buf, size_t len);
  * run, with results bit-identical to the three-kernel tick. Filters of more than
  * 32768 particles take it where the device schedules a cluster of 16 CTAs. Runs of
  * ticks of larger filters, up to four 4096-particle tiles per SM (2.4 million
- * particles on 148 SMs), stay on the chip as one cooperative launch, bit-identical
- * too. On by default; enable = 0 selects the three-kernel tick for both. Learning filters, Silverman
- * jitter and profiled ticks always take the three-kernel path. */
+ * particles on 148 SMs), stay on the chip as cooperative launches of up to 1024
+ * ticks, bit-identical too. Such a launch takes one CTA and most of the shared
+ * memory of up to every SM (one SM per tile up to as many tiles as SMs): it starts
+ * when those SMs are free, and other streams' kernels that need them wait until it
+ * ends (4 to 25 ms for 1024 ticks). On by default; enable = 0 selects the
+ * three-kernel tick for both, which leaves the GPU between ticks. Learning filters,
+ * Silverman jitter and profiled ticks always take the three-kernel path. */
 int gpu_bpf_set_fused_small(GpuBpfState* state, int enable);
 
 /* Kernel profiling: when enabled, every tick's three kernels (pass 1, plan,
