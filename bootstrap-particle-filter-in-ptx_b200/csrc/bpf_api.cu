@@ -148,12 +148,24 @@ bool use_resident(const Impl* m, const TickArgs& a) {
          !(a.silverman > 0.0f) &&
          resident_ready(m->device, m->plan.G, m->res_tiles, a.nu_int > 0, !(a.obs.nu > 0.0f), false);
 }
-// Whether a run of ticks is one launch (a resident run: one per kResRunTicks ticks), and that launch
-// (a.y_ptr, a.rec: the run's first tick).
+// Whether a run of ticks is one launch (resident runs: one per kResRunTicks ticks, fused ones: one per
+// kSmallRunTicks), and that launch (a.y_ptr, a.rec: the run's first tick).
+constexpr int kSmallRunTicks = 16384;
 bool one_launch(const Impl* m, const TickArgs& a) { return use_small(m, a) || use_resident(m, a); }
+int run_launches(const Impl* m, const TickArgs& a, int n_ticks) {
+  return use_small(m, a) ? (n_ticks + kSmallRunTicks - 1) / kSmallRunTicks : resident_launches(n_ticks);
+}
 cudaError_t launch_run(Impl* m, const TickArgs& a, int n_ticks) {
-  if (use_small(m, a)) return launch_small(m->plan, a, n_ticks, m->stream, m->pdl);
-  return launch_resident(m->plan, a, ResidentTape{}, false, n_ticks, m->res_tiles, m->stream, m->waits);
+  if (!use_small(m, a))
+    return launch_resident(m->plan, a, ResidentTape{}, false, n_ticks, m->res_tiles, m->stream, m->waits);
+  cudaError_t e = cudaSuccess;
+  for (int t = 0; t < n_ticks && e == cudaSuccess; t += kSmallRunTicks) {
+    TickArgs run = a;
+    run.y_ptr = a.y_ptr + t;
+    run.rec = a.rec + t;
+    e = launch_small(m->plan, run, std::min(kSmallRunTicks, n_ticks - t), m->stream, m->pdl);
+  }
+  return e;
 }
 
 // Filters of at most kTailTiles tiles run the plan in pass 1's last CTA instead of a plan
@@ -378,15 +390,16 @@ int build_graph(GpuBpfState* s, Impl* m) {
   return BPF_OK;
 }
 
-constexpr int kMaxGraphTicks = 16384;   // larger device runs launch directly
+constexpr int kMaxGraphTicks = 16384;   // longer device runs of several kernels a tick launch directly
 
+// (BPF_OK without a graph: the resident form was refused)
 int build_device_graph(GpuBpfState* s, Impl* m, const float* y_dev, int n, BpfTickRecord* rec_dev) {
   if (m->dgraph) { cudaGraphExecDestroy(m->dgraph); m->dgraph = nullptr; }
   cudaGraph_t g = nullptr;
   const TickArgs a0 = make_args(s, m, 0.0f, y_dev, rec_dev);
   const bool one = one_launch(m, a0);                                   // (configures outside the capture)
   m->dg_resident = one && !use_small(m, a0);
-  m->dg_launches = m->dg_resident ? resident_launches(n) : (one ? 1 : (long long)tick_launches(m, a0) * n);
+  m->dg_launches = one ? run_launches(m, a0, n) : (long long)tick_launches(m, a0) * n;
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
   if (one) {
@@ -406,7 +419,7 @@ int build_device_graph(GpuBpfState* s, Impl* m, const float* y_dev, int n, BpfTi
     m->dgraph = nullptr;
     if (!m->dg_resident) return set_err(BPF_ERR_CUDA);
     m->res_tiles = 0;                                                   // refused: tick by tick from now on
-    return build_device_graph(s, m, y_dev, n, rec_dev);
+    return BPF_OK;
   }
   m->dg_y = y_dev; m->dg_rec = rec_dev; m->dg_n = n;
   m->dg_mu = s->mu; m->dg_rho = s->rho; m->dg_sigma = s->sigma_z; m->dg_thr = s->ess_threshold;
@@ -821,28 +834,31 @@ int gpu_bpf_step_many_device(GpuBpfState* s, const float* y_dev, int n_ticks, Bp
   if (rc) return rc;
   rc = ensure_device(m);
   if (rc) return rc;
-  if (!m->profiling && !m->learn_mode && n_ticks > 0 && n_ticks <= kMaxGraphTicks) {
+  bool launched = n_ticks == 0;
+  while (!launched && !m->profiling && !m->learn_mode &&
+         (n_ticks <= kMaxGraphTicks || one_launch(m, make_args(s, m, 0.0f, y_dev, rec_dev)))) {
     const bool stale = !m->dgraph || m->dg_y != y_dev || m->dg_rec != rec_dev || m->dg_n != n_ticks ||
                        m->dg_mu != s->mu || m->dg_rho != s->rho || m->dg_sigma != s->sigma_z ||
                        m->dg_thr != s->ess_threshold || m->dg_nus != s->nu_state ||
                        m->dg_silv != s->silverman_shrink || m->dg_anc != m->record_anc;
     if (stale) { rc = build_device_graph(s, m, y_dev, n_ticks, rec_dev); if (rc) return rc; }
-    cudaError_t e = cudaGraphLaunch(m->dgraph, m->stream);
+    if (!m->dgraph) continue;                         // refused: once more, tick by tick
+    const cudaError_t e = cudaGraphLaunch(m->dgraph, m->stream);
     if (e != cudaSuccess && m->dg_resident) {         // refused at the launch
       cudaGetLastError();
+      cudaGraphExecDestroy(m->dgraph);
+      m->dgraph = nullptr;
       m->res_tiles = 0;
-      rc = build_device_graph(s, m, y_dev, n_ticks, rec_dev);
-      if (rc) return rc;
-      e = cudaGraphLaunch(m->dgraph, m->stream);
+      continue;
     }
     CK(e);
     g_launches += m->dg_launches;
     m->ticks_enqueued += n_ticks;
-  } else {
-    for (int t = 0; t < n_ticks; ++t) {
-      rc = enqueue_tick(s, m, make_args(s, m, 0.0f, y_dev + t, rec_dev + t));
-      if (rc) return rc;
-    }
+    launched = true;
+  }
+  for (int t = 0; t < n_ticks && !launched; ++t) {
+    rc = enqueue_tick(s, m, make_args(s, m, 0.0f, y_dev + t, rec_dev + t));
+    if (rc) return rc;
   }
   if (n_ticks > 0) {
     CK(cudaMemcpyAsync(m->rec_dev, rec_dev + n_ticks - 1, sizeof(BpfTickRecord), cudaMemcpyDeviceToDevice, m->stream));

@@ -52,3 +52,29 @@ def test_tape_of_several_launches(bpf, every):
                     [tape.children(t).tobytes() for t in (0, 1023, 1024, T - 2)]))
         tape.close()
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("N,launches", [(4096, 2), (70001, 17)])
+def test_long_device_run_stays_on_the_chip(bpf, N, launches):
+    """More ticks than a graph of single ticks is built for: still the runs' launches, and where the
+    resident one is refused, tick by tick with the same results."""
+    import torch
+    T = 16385
+    y = _series(T, 5)
+    out = []
+    for fused, fault in ((True, 0), (True, 4), (False, 0)):
+        rec = torch.zeros(T * 40, dtype=torch.uint8, device="cuda")
+        f = bpf.GpuBpf(N, RHO, SIG, MU, seed=3, ess_threshold=0.5)
+        f.set_fused_small(fused)
+        assert f._lib.gpu_bpf_debug_resident(f._s, fault, 0, 0, 2000.0) == 0
+        n0 = f._lib.gpu_bpf_launch_count()
+        f.step_many_device(y.data_ptr(), T, rec.data_ptr())
+        n = f._lib.gpu_bpf_launch_count() - n0
+        if fused and (fault == 0 or N <= 65536):
+            assert n == launches
+        else:
+            assert n >= 2 * T
+        torch.cuda.synchronize()
+        out.append((rec.cpu().numpy().tobytes(), bytes(f.get_particles())))
+        f.close()
+    assert out[0] == out[1] == out[2]
