@@ -2,9 +2,11 @@
 // injected failure (see bpf_alloc.cuh). The injected failure returns
 // cudaErrorMemoryAllocation without calling the runtime, as a real out-of-memory
 // allocation would, so callers take their ordinary error path.
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <unordered_set>
+#include <vector>
 
 #include "bpf_alloc.cuh"
 #include "../../include/gpu_bpf.h"
@@ -38,11 +40,72 @@ void untrack(void* p) {
   std::lock_guard<std::mutex> lock(g_mutex);
   g_live.erase(p);
 }
+
+// Recursive: an owner's give_back frees under the lock that its caller holds.
+std::recursive_mutex g_kept_mutex;
+std::vector<KeptOwner*> g_kept;
+
+size_t kept_on(int device) {                // device < 0: on all
+  size_t n = 0;
+  for (const KeptOwner* o : g_kept) if (device < 0 || o->device == device) n += o->bytes;
+  return n;
+}
+
+// Every idle owner on the device (all devices if negative) gives its memory back; the bytes given.
+size_t kept_trim(int device) {
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  const size_t before = kept_on(device);
+  for (KeptOwner* o : g_kept)
+    if ((device < 0 || o->device == device) && o->in_use == 0 && o->bytes > 0) o->give_back();
+  return before - kept_on(device);
+}
 }  // namespace
+
+void kept_register(KeptOwner* o) {
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  g_kept.push_back(o);
+}
+void kept_unregister(KeptOwner* o) {
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  g_kept.erase(std::remove(g_kept.begin(), g_kept.end(), o), g_kept.end());
+}
+KeptUse::KeptUse(KeptOwner* o) : owner(o) {
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  ++o->in_use;
+}
+KeptUse::~KeptUse() {
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  --owner->in_use;
+}
+void kept_malloc(KeptOwner* o, void** p, size_t bytes) {
+  *p = nullptr;
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  size_t free_b = 0, total_b = 0;
+  const size_t held = kept_on(o->device);
+  const bool fits = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && held + bytes <= (free_b + held) / 8;
+  if (!fits || take_failure() || track(cudaMalloc(p, bytes), p) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    return;
+  }
+  o->bytes += bytes;
+}
+void kept_free(KeptOwner* o, void* p, size_t bytes) {
+  if (!p) return;
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  bpf_free(p);
+  o->bytes -= bytes;
+}
 
 cudaError_t bpf_malloc_raw(void** p, size_t bytes) {
   if (take_failure()) { *p = nullptr; return cudaErrorMemoryAllocation; }
-  return track(cudaMalloc(p, bytes), p);
+  cudaError_t e = cudaMalloc(p, bytes);
+  int device = 0;
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess && kept_trim(device) > 0) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return track(e, p);
 }
 cudaError_t bpf_malloc_host_raw(void** p, size_t bytes) {
   if (take_failure()) { *p = nullptr; return cudaErrorMemoryAllocation; }
@@ -78,5 +141,12 @@ long long gpu_bpf_debug_live_allocs(void) {
   std::lock_guard<std::mutex> lock(g_mutex);
   return (long long)g_live.size();
 }
+
+size_t gpu_bpf_kept_bytes(void) {
+  std::lock_guard<std::recursive_mutex> lock(g_kept_mutex);
+  return kept_on(-1);
+}
+
+size_t gpu_bpf_trim_kept(void) { return kept_trim(-1); }
 
 }  // extern "C"

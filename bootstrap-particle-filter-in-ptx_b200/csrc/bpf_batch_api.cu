@@ -17,6 +17,7 @@
 #include <string>
 #include <vector>
 
+#include "bpf_alloc.cuh"
 #include "bpf_batch.cuh"
 #include "bpf_plain.cuh"
 
@@ -27,14 +28,21 @@ using namespace bpf;
 
 namespace {
 
+void drop_hist(GpuBpfBatch* b, int c) {
+  kept_free(&b->keeper, b->g_hist[c], b->g_hist_bytes[c]);
+  b->g_hist[c] = nullptr;
+  b->g_hist_bytes[c] = 0;
+}
+
 void free_batch(GpuBpfBatch* b) {
   if (!b) return;
+  kept_unregister(&b->keeper);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   if (b->ggraph) cudaGraphExecDestroy(b->ggraph);
   if (b->sgraph) cudaGraphExecDestroy(b->sgraph);
   bpf_free(b->d_st); bpf_free(b->d_sth); bpf_free(b->d_stw); bpf_free(b->d_stoff); bpf_free(b->d_tick);
   bpf_free(b->d_scounters);
-  for (int c = 0; c < kClasses; ++c) { bpf_free(b->g_tape[c]); bpf_free(b->g_hist[c]); }
+  for (int c = 0; c < kClasses; ++c) { bpf_free(b->g_tape[c]); drop_hist(b, c); }
   bpf_free(b->d_AB);
   bpf_free(b->d_nzoff);
   bpf_free(b->d_filters); bpf_free(b->d_order); bpf_free(b->d_counters);
@@ -141,23 +149,13 @@ int prepare_grad(GpuBpfBatch* b, int T) {
     }
   }
   // the particles of every tick, for the classes that run the unrolled kernels
-  size_t want = 0, free_b = 0, total_b = 0;
-  auto hist_bytes = [&](int c) {
-    return batch_grad_keeps(b->threads[c], kClassMaxN[c]) && b->class_cnt[c]
-               ? (size_t)b->g_grid[c] * T * kClassMaxN[c] * sizeof(float) : (size_t)0;
-  };
-  for (int c = 0; c < kClasses; ++c) if (hist_bytes(c) > b->g_hist_bytes[c]) want += hist_bytes(c);
-  if (want) {
-    BCK(cudaMemGetInfo(&free_b, &total_b));
-    for (int c = 0; c < kClasses; ++c) {
-      if (hist_bytes(c) <= b->g_hist_bytes[c]) continue;
-      bpf_free(b->g_hist[c]);
-      b->g_hist[c] = nullptr;
-      b->g_hist_bytes[c] = 0;
-      if (want > free_b / 8) continue;
-      if (bpf_malloc(&b->g_hist[c], hist_bytes(c)) == cudaSuccess) b->g_hist_bytes[c] = hist_bytes(c);
-      else { cudaGetLastError(); b->g_hist[c] = nullptr; }
-    }
+  for (int c = kClasses - 1; c >= 0 && !b->hist_off; --c) {
+    if (!b->class_cnt[c] || !batch_grad_keeps(b->threads[c], kClassMaxN[c])) continue;
+    const size_t need = (size_t)b->g_grid[c] * T * kClassMaxN[c] * sizeof(float);
+    if (need <= b->g_hist_bytes[c]) continue;
+    drop_hist(b, c);
+    kept_malloc(&b->keeper, reinterpret_cast<void**>(&b->g_hist[c]), need);
+    if (b->g_hist[c]) b->g_hist_bytes[c] = need;
   }
   if (b->ab_T < T + 1) {
     bpf_free(b->d_AB);
@@ -404,6 +402,14 @@ GpuBpfBatch* gpu_bpf_batch_create(const BpfBatchFilter* filters, int n_filters, 
       cudaMemcpy(b->d_order, order.data(), n_filters * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
     return fail(BPF_ERR_CUDA);
   configure_classes(b);
+  b->keeper.device = b->device;
+  b->keeper.give_back = [b]() {
+    cudaStreamSynchronize(b->stream);
+    if (b->ggraph) { cudaGraphExecDestroy(b->ggraph); b->ggraph = nullptr; }
+    for (int c = 0; c < kClasses; ++c) drop_hist(b, c);
+    b->hist_off = true;
+  };
+  kept_register(&b->keeper);
   return b;
 }
 
@@ -468,6 +474,7 @@ int gpu_bpf_batch_grad_run(GpuBpfBatch* b, const float* y_dev, int n_ticks, doub
   if (b->ess_threshold != 0.0f) return bpf_record_error(BPF_ERR_UNSUPPORTED);   // always-resample tapes only
   int rc = ensure_device_b(b);
   if (rc) return rc;
+  KeptUse use(&b->keeper);
   GraphKey k;
   k.y = y_dev; k.T = n_ticks; k.loglik = loglik_dev;
   std::copy(b->threads, b->threads + kClasses, k.threads);

@@ -96,10 +96,12 @@ struct GpuBpfBatch {
   unsigned char* g_tape[kClasses] = {};
   size_t g_tape_bytes[kClasses] = {0, 0, 0, 0, 0};
   int g_grid[kClasses] = {1, 1, 1, 1, 1};
-  // every tick's particles of the gradient forward (per class, where an eighth of the free memory holds
-  // them): the backward then recomputes nothing (256 x 8192: 53 -> 44 us per tick forward and backward)
+  // every tick's particles of the gradient forward (kept memory, per class): the backward then recomputes
+  // nothing (256 x 8192: 53 -> 44 us per tick forward and backward). Once given back they stay away.
   float* g_hist[kClasses] = {};
   size_t g_hist_bytes[kClasses] = {0, 0, 0, 0, 0};
+  bool hist_off = false;
+  KeptOwner keeper;
   ulonglong2* d_AB = nullptr;
   int ab_T = 0;
   cudaGraphExec_t ggraph = nullptr;

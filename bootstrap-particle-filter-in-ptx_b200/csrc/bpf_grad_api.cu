@@ -96,11 +96,12 @@ struct GpuBpfGrad {
   BpfTickRecord* rec = nullptr;      // [T_max]
   float* seg = nullptr;              // [K][N4]
   // Every tick's particles of a resident forward run, [T_max][G*4096]: with them the backward is one
-  // kernel per tick and recomputes nothing (N = 2^20 16.7 -> 10.2 us per tick). Allocated by the first
-  // such run of a tape with the default checkpoint interval, where an eighth of the free memory holds
-  // them; without them the checkpoints serve.
+  // kernel per tick and recomputes nothing (N = 2^20 16.7 -> 10.2 us per tick). Kept memory, asked for by
+  // the first such run of a tape with the default checkpoint interval; without them, or once they are
+  // given back (between a forward and its backward too), the checkpoints serve.
   float* hist = nullptr;
   bool default_k = false, hist_tried = false;
+  KeptOwner keeper;
   float* lam[2] = {nullptr, nullptr};
   double* acc = nullptr;             // [G1][kGradAcc]
 
@@ -123,12 +124,26 @@ struct GpuBpfGrad {
 
 namespace {
 
+size_t hist_bytes(const GpuBpfGrad* g) { return (size_t)g->T_max * g->ckpt_stride * sizeof(float); }
+
+// The graphs that name the kept particles go with them.
+void drop_hist(GpuBpfGrad* g) {
+  if (!g->hist) return;
+  cudaStreamSynchronize(g->stream);
+  if (g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }
+  if (g->bgraph) { cudaGraphExecDestroy(g->bgraph); g->bgraph = nullptr; }
+  kept_free(&g->keeper, g->hist, hist_bytes(g));
+  g->hist = nullptr;
+}
+
 void free_grad(GpuBpfGrad* g) {
   if (!g) return;
+  kept_unregister(&g->keeper);
+  kept_free(&g->keeper, g->hist, hist_bytes(g));
   if (g->fgraph) cudaGraphExecDestroy(g->fgraph);
   if (g->bgraph) cudaGraphExecDestroy(g->bgraph);
   plan_free(g->plan);
-  bpf_free(g->csr); bpf_free(g->ckpt); bpf_free(g->aux); bpf_free(g->rec); bpf_free(g->seg); bpf_free(g->hist);
+  bpf_free(g->csr); bpf_free(g->ckpt); bpf_free(g->aux); bpf_free(g->rec); bpf_free(g->seg);
   bpf_free(g->lam[0]); bpf_free(g->lam[1]); bpf_free(g->acc);
   bpf_free(g->rs[0]); bpf_free(g->rs[1]); bpf_free(g->part); bpf_free(g->per_tick); bpf_free(g->rtotal);
   if (g->stream) cudaStreamDestroy(g->stream);
@@ -318,6 +333,9 @@ GpuBpfGrad* gpu_bpf_grad_create(int n_particles, int max_ticks, int checkpoint_e
   al(&g->lam[1], N4 * sizeof(float));
   al(&g->acc, (size_t)g->G1 * kGradAcc * sizeof(double));
   if (e != cudaSuccess) return fail(e);
+  g->keeper.device = g->device;
+  g->keeper.give_back = [g]() { drop_hist(g); };
+  kept_register(&g->keeper);
   return g;
 }
 
@@ -338,6 +356,7 @@ int gpu_bpf_grad_debug_resident(GpuBpfGrad* g, int fault, int cta, int exchange,
   if (!resident_waits_of(fault, cta, exchange, limit_ms, &w)) return bpf_record_error(BPF_ERR_ARG);
   int rc = ensure_dev(g);
   if (rc) return rc;
+  KeptUse use(&g->keeper);
   GCK(cudaStreamSynchronize(g->stream));
   if (g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }   // it holds the waits
   g->waits = w;
@@ -356,19 +375,14 @@ int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, floa
   if (ess_threshold != 0.0f) return bpf_record_error(BPF_ERR_UNSUPPORTED);   // always-resample tapes only
   int rc = ensure_dev(g);
   if (rc) return rc;
+  KeptUse use(&g->keeper);
   FwdKey k;
   k.T = n_ticks; k.seed = seed; k.mu = mu; k.rho = rho; k.sigma = sigma_z; k.nu = nu_obs; k.nu_state = nu_state;
   k.y = y_dev; k.ll = loglik_dev;
   g->resident = resident_ready(g->device, g->plan.G, g->res_tiles, nu_int_of(nu_state) > 0, !(nu_obs > 0.0f), false);
   if (g->resident && g->default_k && !g->hist_tried) {
     g->hist_tried = true;
-    const size_t bytes = (size_t)g->T_max * g->ckpt_stride * sizeof(float);
-    size_t free_b = 0, total_b = 0;
-    GCK(cudaMemGetInfo(&free_b, &total_b));
-    if (bytes <= free_b / 8 && bpf_malloc(&g->hist, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      g->hist = nullptr;
-    }
+    kept_malloc(&g->keeper, reinterpret_cast<void**>(&g->hist), hist_bytes(g));
     if (g->hist && g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }
   }
   auto launch = [&]() {
@@ -384,6 +398,7 @@ int gpu_bpf_grad_forward(GpuBpfGrad* g, float mu, float rho, float sigma_z, floa
     cudaGetLastError();
     g->res_tiles = 0;
     g->resident = false;
+    drop_hist(g);
     if (g->fgraph) { cudaGraphExecDestroy(g->fgraph); g->fgraph = nullptr; }
     e = launch();
   }
@@ -407,6 +422,7 @@ int gpu_bpf_grad_backward(GpuBpfGrad* g, double* grad_dev) {
   if (!g->have_fwd) return bpf_record_error(BPF_ERR_STATE);
   int rc = ensure_dev(g);
   if (rc) return rc;
+  KeptUse use(&g->keeper);
   BwdKey bk;
   bk.f = g->cur;
   bk.grad = grad_dev;

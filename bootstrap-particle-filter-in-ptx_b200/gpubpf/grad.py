@@ -30,6 +30,17 @@ def ancestors_from_children(first_child: np.ndarray) -> np.ndarray:
     return np.repeat(np.arange(n, dtype=np.int32), counts)
 
 
+def kept_bytes() -> int:
+    """Device memory that tapes and batches keep beyond their tape_bytes (gpu_bpf_kept_bytes)."""
+    return int(_lib.load().gpu_bpf_kept_bytes())
+
+
+def trim_kept() -> int:
+    """Give that memory back, the cached tapes' and batches' of bpf_loglik and bpf_batch_loglik included:
+    bytes freed. Their later runs recompute instead, with the same results."""
+    return int(_lib.load().gpu_bpf_trim_kept())
+
+
 class GradTape:
     """Device tape of one taped forward run: child lists, checkpoints, normalisers."""
 

@@ -439,9 +439,9 @@ double*      gpu_bpf_batch_loglik_device(GpuBpfBatch* batch);
 int          gpu_bpf_batch_grad_run(GpuBpfBatch* batch, const float* y_dev, int n_ticks, double* loglik_dev,
                                     double* grad_dev);
 /* Device memory the gradient tape of gpu_bpf_batch_grad_run takes for n_ticks ticks (it is sized
- * for the CTAs in flight, not for the number of filters). Where an eighth of the free device
- * memory holds them, every tick's particles are kept too (4 bytes per particle and tick of the
- * filters in flight); the backward pass then recomputes nothing. */
+ * for the CTAs in flight, not for the number of filters). Every tick's particles are kept besides
+ * (4 bytes per particle and tick of the filters in flight) where gpu_bpf_kept_bytes' bound allows,
+ * size class by size class; the backward pass then recomputes nothing. */
 size_t       gpu_bpf_batch_grad_tape_bytes(GpuBpfBatch* batch, int n_ticks);
 /* Correlated-noise runs: the building block of correlated pseudo-marginal MCMC (CPMMH,
  * Deligiannidis, Doucet & Pitt 2018), as the reference's CPMMH rejuvenation kernel uses it
@@ -482,8 +482,8 @@ typedef struct GpuBpfGrad GpuBpfGrad;
 
 /* Tape for up to max_ticks ticks of n_particles (checkpoint_every 0 = 16). NULL on error.
  * Device memory: gpu_bpf_grad_tape_bytes() (about 4 * n_particles * max_ticks bytes). With
- * checkpoint_every 0 the first forward run also keeps every tick's particles where an eighth of
- * the free device memory holds them (as much again; the backward pass then recomputes nothing);
+ * checkpoint_every 0 the first forward run also keeps every tick's particles where
+ * gpu_bpf_kept_bytes' bound allows (as much again; the backward pass then recomputes nothing);
  * a checkpoint interval of the caller's choice never takes more. */
 GpuBpfGrad* gpu_bpf_grad_create(int n_particles, int max_ticks, int checkpoint_every);
 void        gpu_bpf_grad_destroy(GpuBpfGrad* grad);
@@ -597,6 +597,17 @@ int gpu_bpf_grad_debug_resident(GpuBpfGrad* grad, int fault, int cta, int exchan
  * n if it does not: the time between two looks counts as at most a sixteenth of the limit, so a GPU
  * that was taken away for a while does not end the run. On the host. */
 int gpu_bpf_debug_wait_budget(const unsigned long long* now_ns, int n, unsigned long long limit_ns);
+
+/* Kept memory: device memory that gradient runs (gpu_bpf_grad_forward, gpu_bpf_batch_grad_run) take only
+ * to be faster, on top of their tape_bytes. All of a device's tapes and batches together keep at most an
+ * eighth of the device memory that is free or so kept; beyond that they recompute, with the same
+ * results. It is freed with its tape or batch, when another allocation of this library would fail
+ * for want of memory, and by gpu_bpf_trim_kept, which a program calls before it needs the memory for
+ * itself (it waits for the tapes and batches, of which those in a call of another thread keep theirs;
+ * one that gave back takes no more). gpu_bpf_kept_bytes: bytes kept now; gpu_bpf_trim_kept: bytes
+ * given back. Both count all devices. */
+size_t gpu_bpf_kept_bytes(void);
+size_t gpu_bpf_trim_kept(void);
 
 /* Number of kernel launches this library has issued (all filters). */
 long long gpu_bpf_launch_count(void);
