@@ -270,12 +270,16 @@ int ensure_device_b(GpuBpfBatch* b) {
   return BPF_OK;
 }
 
+// Which kernels the timings behind a cache entry were taken with: an entry of another generation says
+// nothing about which shape is fastest now. 2: shapes of at most 16 particles a thread run unrolled.
+constexpr int kKernelGeneration = 2;
+
 std::string gpu_key(int device) {
   cudaDeviceProp p;
   if (cudaGetDeviceProperties(&p, device) != cudaSuccess) return "unknown";
   std::string s = p.name;
   for (char& ch : s) if (ch == ' ' || ch == '"') ch = '_';
-  return s + "_sm" + std::to_string(p.multiProcessorCount);
+  return s + "_sm" + std::to_string(p.multiProcessorCount) + "_k" + std::to_string(kKernelGeneration);
 }
 
 // Autotune cache: one line per entry, "<gpu_key> <class> <threads>".

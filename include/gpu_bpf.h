@@ -396,7 +396,8 @@ int          gpu_bpf_batch_set_threads(GpuBpfBatch* batch, int size_class, int t
 int          gpu_bpf_batch_get_threads(GpuBpfBatch* batch, int size_class);
 /* Project autotuner: times every CTA shape of every non-empty class on n_ticks of y and keeps
  * the fastest; results are appended to / read from the text cache file cache_path
- * ("<gpu> <class> <threads>" lines; NULL = no cache). */
+ * ("<gpu> <class> <threads>" lines; NULL = no cache). <gpu> names the kernels' generation too: entries
+ * that an earlier build measured with other kernels are not taken. */
 int          gpu_bpf_batch_autotune(GpuBpfBatch* batch, const float* y, int n_ticks, const char* cache_path);
 /* Host buffers: y[n_ticks] in, loglik[n_filters] (FP64 total log-likelihood) and optionally the
  * last tick's filtered mean out. Synchronous. */
