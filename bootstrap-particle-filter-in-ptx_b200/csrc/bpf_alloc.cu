@@ -5,7 +5,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
-#include <unordered_set>
+#include <unordered_map>
 #include <vector>
 
 #include "bpf_alloc.cuh"
@@ -13,7 +13,7 @@
 
 namespace {
 std::mutex g_mutex;
-std::unordered_set<void*> g_live;        // live device and pinned allocations
+std::unordered_map<void*, size_t> g_live;   // live device and pinned allocations and their bytes
 long long g_fail_in = -1;                 // allocations to let through before the injected failure
 long long g_count = 0;                    // allocations attempted since load
 
@@ -27,10 +27,10 @@ bool take_failure() {
   return false;
 }
 
-cudaError_t track(cudaError_t e, void** p) {
+cudaError_t track(cudaError_t e, void** p, size_t bytes) {
   if (e == cudaSuccess && *p) {
     std::lock_guard<std::mutex> lock(g_mutex);
-    g_live.insert(*p);
+    g_live[*p] = bytes;
   }
   return e;
 }
@@ -83,7 +83,7 @@ void kept_malloc(KeptOwner* o, void** p, size_t bytes) {
   size_t free_b = 0, total_b = 0;
   const size_t held = kept_on(o->device);
   const bool fits = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && held + bytes <= (free_b + held) / 8;
-  if (!fits || take_failure() || track(cudaMalloc(p, bytes), p) != cudaSuccess) {
+  if (!fits || take_failure() || track(cudaMalloc(p, bytes), p, bytes) != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
     return;
@@ -105,15 +105,15 @@ cudaError_t bpf_malloc_raw(void** p, size_t bytes) {
     cudaGetLastError();
     e = cudaMalloc(p, bytes);
   }
-  return track(e, p);
+  return track(e, p, bytes);
 }
 cudaError_t bpf_malloc_host_raw(void** p, size_t bytes) {
   if (take_failure()) { *p = nullptr; return cudaErrorMemoryAllocation; }
-  return track(cudaMallocHost(p, bytes), p);
+  return track(cudaMallocHost(p, bytes), p, bytes);
 }
 cudaError_t bpf_host_alloc_raw(void** p, size_t bytes, unsigned flags) {
   if (take_failure()) { *p = nullptr; return cudaErrorMemoryAllocation; }
-  return track(cudaHostAlloc(p, bytes, flags), p);
+  return track(cudaHostAlloc(p, bytes, flags), p, bytes);
 }
 cudaError_t bpf_free(void* p) {
   untrack(p);
@@ -140,6 +140,13 @@ long long gpu_bpf_debug_alloc_count(void) {
 long long gpu_bpf_debug_live_allocs(void) {
   std::lock_guard<std::mutex> lock(g_mutex);
   return (long long)g_live.size();
+}
+
+size_t gpu_bpf_debug_live_bytes(void) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  size_t n = 0;
+  for (const auto& a : g_live) n += a.second;
+  return n;
 }
 
 size_t gpu_bpf_kept_bytes(void) {

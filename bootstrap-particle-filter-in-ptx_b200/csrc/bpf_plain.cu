@@ -1737,16 +1737,20 @@ cudaError_t plan_alloc(Plan& p, int N) {
   al(&p.P, p.G * sizeof(unsigned long long));
   al(&p.ofirst, (p.G + 1) * sizeof(int));
   al(&p.items, p.max_items * sizeof(int4));
+  // the exchange buffer only where the device takes resident runs of the filter, in the same allocation
+  int device = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&device);
   const size_t jbytes = (p.G * sizeof(double) + 255) & ~(size_t)255;
-  al(&p.jpart, jbytes + resident_xbuf_bytes(p.G));     // one allocation for both
-  if (e == cudaSuccess && resident_xbuf_bytes(p.G) > 0) p.xbuf = reinterpret_cast<unsigned char*>(p.jpart) + jbytes;
+  const size_t xbytes = e == cudaSuccess && p.G <= resident_max_tiles(device) ? resident_xbuf_bytes(p.G) : 0;
+  al(&p.jpart, jbytes + xbytes);
+  if (e == cudaSuccess && xbytes > 0) p.xbuf = reinterpret_cast<unsigned char*>(p.jpart) + jbytes;
   al(&p.jticket, sizeof(unsigned));
   al(&p.pticket, sizeof(unsigned));
   al(&p.st, sizeof(DevState));
   if (e == cudaSuccess) e = cudaMemset(p.nexp, 0, p.G * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(p.jticket, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(p.pticket, 0, sizeof(unsigned));
-  if (e == cudaSuccess && p.xbuf) e = cudaMemset(p.xbuf, 0, resident_xbuf_bytes(p.G));
+  if (e == cudaSuccess && p.xbuf) e = cudaMemset(p.xbuf, 0, xbytes);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();   // visible to every stream before first use
   return e;
 }

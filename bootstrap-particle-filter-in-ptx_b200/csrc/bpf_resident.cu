@@ -56,7 +56,7 @@ constexpr int kMail = 16;
 constexpr size_t kXHeader = 256;
 __host__ __device__ inline size_t mail_flag_bytes(int G) { return ((size_t)G * 4 + 127) & ~(size_t)127; }
 __host__ __device__ inline size_t mail_bytes(int G) { return mail_flag_bytes(G) + (((size_t)G * 64 + 127) & ~(size_t)127); }
-size_t resident_xbuf_bytes(int G) { return G <= kResMaxTiles ? kXHeader + kMail * mail_bytes(G) : 0; }
+size_t resident_xbuf_bytes(int G) { return kXHeader + kMail * mail_bytes(G); }
 
 __device__ __forceinline__ void st_relaxed_b128(void* p, unsigned long long lo, unsigned long long hi) {
   asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p), "l"(lo), "l"(hi)
@@ -900,7 +900,7 @@ bool resident_ready(int device, int G, int max_tiles, bool tstate, bool gauss, b
 
 cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
                             int max_tiles, cudaStream_t s, const ResidentWaits& waits) {
-  if (!p.xbuf || p.G < 1 || p.G > max_tiles || n_ticks < 1 || !a.y_ptr) return cudaErrorInvalidValue;
+  if (!p.xbuf || p.G < 1 || p.G > max_tiles || p.G > kResMaxTiles || n_ticks < 1 || !a.y_ptr) return cudaErrorInvalidValue;
   if (waits.fault == kFaultRefused) return cudaErrorCooperativeLaunchTooLarge;
   const int sms = max_tiles / kResMaxTilesPerCta;
   const int nt = (p.G + sms - 1) / sms;

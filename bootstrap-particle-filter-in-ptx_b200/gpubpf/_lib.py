@@ -142,6 +142,7 @@ SIGNATURES = {
     "gpu_bpf_debug_fail_alloc": (_i, [C.c_longlong]),
     "gpu_bpf_debug_alloc_count": (C.c_longlong, []),
     "gpu_bpf_debug_live_allocs": (C.c_longlong, []),
+    "gpu_bpf_debug_live_bytes": (C.c_size_t, []),
     "gpu_bpf_kept_bytes": (C.c_size_t, []),
     "gpu_bpf_trim_kept": (C.c_size_t, []),
     "gpu_bpf_debug_resident": (_i, [P_STATE, _i, _i, _i, _d]),

@@ -576,10 +576,12 @@ int         gpu_bpf_smc2_get_noise(GpuBpfSmc2* smc2, int j, int n_ticks, float* 
  * them fails as an out-of-memory allocation would (once; k < 0 disarms), so the
  * error path of any create function can be exercised on the host without a GPU
  * fault. gpu_bpf_debug_alloc_count: allocations attempted since the library was
- * loaded; gpu_bpf_debug_live_allocs: allocations not yet freed. */
+ * loaded; gpu_bpf_debug_live_allocs: allocations not yet freed; gpu_bpf_debug_live_bytes:
+ * their bytes. */
 int       gpu_bpf_debug_fail_alloc(long long k);
 long long gpu_bpf_debug_alloc_count(void);
 long long gpu_bpf_debug_live_allocs(void);
+size_t    gpu_bpf_debug_live_bytes(void);
 
 /* Waits of resident runs (gpu_bpf_set_fused_small; testing aid). The CTAs of such a run wait on one
  * another, each wait at most 2 s of polling; a run in which one gives up ends with BPF_ERR_STATE: step_many returns
