@@ -254,10 +254,10 @@ void gpu_apf_destroy(GpuApfState* s) {
   free(s);
 }
 
-int gpu_apf_debug_resident(GpuApfState* s, int fault, int cta, int exchange, double limit_ms) {
+int gpu_apf_debug_resident(GpuApfState* s, int fault, int mailbox, double limit_ms) {
   ApfImpl* m = impl_of(s);
   if (!m) return set_err(BPF_ERR_STATE);
-  if (!resident_waits_of(fault, cta, exchange, limit_ms, &m->waits)) return set_err(BPF_ERR_ARG);
+  if (!resident_waits_of(fault, mailbox, limit_ms, &m->waits)) return set_err(BPF_ERR_ARG);
   m->res_tiles = resident_max_tiles(m->device);
   return BPF_OK;
 }

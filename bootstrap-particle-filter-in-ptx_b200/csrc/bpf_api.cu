@@ -1113,11 +1113,11 @@ int gpu_bpf_set_fused_small(GpuBpfState* s, int enable) {
   return BPF_OK;
 }
 
-int gpu_bpf_debug_resident(GpuBpfState* s, int fault, int cta, int exchange, double limit_ms) {
+int gpu_bpf_debug_resident(GpuBpfState* s, int fault, int mailbox, double limit_ms) {
   Impl* m = impl_of(s);
   if (!m) return set_err(BPF_ERR_STATE);
   ResidentWaits w;
-  if (!resident_waits_of(fault, cta, exchange, limit_ms, &w)) return set_err(BPF_ERR_ARG);
+  if (!resident_waits_of(fault, mailbox, limit_ms, &w)) return set_err(BPF_ERR_ARG);
   int rc = ensure_device(m);
   if (rc) return rc;
   CK(cudaStreamSynchronize(m->stream));
@@ -1128,10 +1128,10 @@ int gpu_bpf_debug_resident(GpuBpfState* s, int fault, int cta, int exchange, dou
 }
 
 int gpu_bpf_debug_wait_budget(const unsigned long long* now_ns, int n, unsigned long long limit_ns) {
-  if (!now_ns || n < 0 || limit_ns == 0ull) return -set_err(BPF_ERR_ARG);
+  if (!now_ns || n < 0 || limit_ns < 1024ull || limit_ns > kResWaitNs) return -set_err(BPF_ERR_ARG);
   WaitBudget b;
   for (int i = 0; i < n; ++i)
-    if (b.over(now_ns[i], limit_ns)) return i;
+    if (b.over(WaitBudget::clock(now_ns[i]), (unsigned)(limit_ns >> 10))) return i;
   return n;
 }
 

@@ -350,10 +350,10 @@ void* gpu_bpf_grad_stream(GpuBpfGrad* g) { return g ? (void*)g->stream : nullptr
 
 int gpu_bpf_grad_checkpoint_every(GpuBpfGrad* g) { return g ? g->K : -bpf_record_error(BPF_ERR_STATE); }
 
-int gpu_bpf_grad_debug_resident(GpuBpfGrad* g, int fault, int cta, int exchange, double limit_ms) {
+int gpu_bpf_grad_debug_resident(GpuBpfGrad* g, int fault, int mailbox, double limit_ms) {
   if (!g) return bpf_record_error(BPF_ERR_STATE);
   ResidentWaits w;
-  if (!resident_waits_of(fault, cta, exchange, limit_ms, &w)) return bpf_record_error(BPF_ERR_ARG);
+  if (!resident_waits_of(fault, mailbox, limit_ms, &w)) return bpf_record_error(BPF_ERR_ARG);
   int rc = ensure_dev(g);
   if (rc) return rc;
   KeptUse use(&g->keeper);

@@ -157,35 +157,44 @@ struct ResidentTape {        // gradient tape of a taped run from tick 0 (all nu
   float2* aux;                         // {1/S, nM} per tick
   float* hist;                         // every tick's particles as weighted, at hist + t * ckpt_stride, or null
 };
-// How long a wait of a resident run polls before it gives up and, in tests, one failure made on
-// purpose: CTA cta gives up in exchange xn (1-based in the run) or in the wait for the children of its
-// resampling, or does not publish its record of that exchange; or the launch is refused on the host, as
-// one that does not fit on the device is. No wait outlasts its limit.
+// Waits of resident runs: how long one polls before it gives up and, in tests, one failure made on
+// purpose. No wait outlasts its limit.
 constexpr unsigned long long kResWaitNs = 2000000000ull;
-// Time spent polling against that limit, from the clock at one look after another. The time between two
-// looks counts as at most a sixteenth of the limit: while the GPU runs another program, or the grid is
-// held up as a whole, the clock goes on but nobody could publish what the wait is for.
+// Time spent polling against that limit, both in units of 1024 ns, from the clock at one look after
+// another. The time between two looks counts as at most a sixteenth of the limit: while the GPU runs
+// another program, or the grid is held up as a whole, the clock goes on but nobody could publish what
+// the wait is for. (32 bits: the looks are less than an hour apart, and the loops are short of registers.)
 struct WaitBudget {
-  unsigned long long last = 0ull, spent = 0ull;
-  __host__ __device__ __forceinline__ bool over(unsigned long long now, unsigned long long limit) {
-    const unsigned long long step = now - last, cap = limit / 16ull + 1ull;
-    if (last != 0ull) spent += step < cap ? step : cap;
+  unsigned last = 0u, spent = 0u;
+  static __host__ __device__ __forceinline__ unsigned clock(unsigned long long ns) { return (unsigned)(ns >> 10); }
+  __host__ __device__ __forceinline__ bool over(unsigned now, unsigned limit) {
+    const unsigned step = now - last, cap = limit / 16u + 1u;
+    if (last != 0u) spent += step < cap ? step : cap;
     last = now;
     return spent >= limit;
   }
 };
-enum ResidentFault { kFaultNone = 0, kFaultExchange = 1, kFaultFlags = 2, kFaultWithhold = 3, kFaultRefused = 4 };
+constexpr int kResMail = 16;           // mailboxes of the exchange; CTA b polls mailbox b % kResMail
+// Failures for the tests: no record, or no flag of a CTA's children, reaches one of the mailboxes, so the CTAs
+// that poll it wait until they give up; the last CTA, with its tiles' records, is absent; or the launch
+// is refused on the host, as one that does not fit on the device is.
+enum ResidentFault { kFaultNone = 0, kFaultRecords = 1, kFaultFlags = 2, kFaultAbsent = 3, kFaultRefused = 4 };
 struct ResidentWaits {
-  unsigned long long limit_ns = kResWaitNs;
-  int fault = kFaultNone, cta = 0;
-  unsigned xn = 0u;
+  unsigned limit = (unsigned)(kResWaitNs >> 10);
+  unsigned record_mail = (1u << kResMail) - 1u, flag_mail = (1u << kResMail) - 1u;   // mailboxes written to
+  bool absent = false, refused = false;
 };
-inline bool resident_waits_of(int fault, int cta, int exchange, double limit_ms, ResidentWaits* out) {
-  if (fault < kFaultNone || fault > kFaultRefused || cta < 0 || exchange < 0 ||
-      !(limit_ms > 0.0 && limit_ms <= (double)kResWaitNs * 1e-6))
+inline bool resident_waits_of(int fault, int mailbox, double limit_ms, ResidentWaits* out) {
+  if (fault < kFaultNone || fault > kFaultRefused || mailbox < 0 || mailbox >= kResMail ||
+      !(limit_ms >= 0.1 && limit_ms <= (double)kResWaitNs * 1e-6))
     return false;
-  out->limit_ns = (unsigned long long)(limit_ms * 1e6);
-  out->fault = fault; out->cta = cta; out->xn = (unsigned)exchange;
+  ResidentWaits w;
+  w.limit = (unsigned)(limit_ms * 1e6 / 1024.0);
+  if (fault == kFaultRecords) w.record_mail &= ~(1u << mailbox);
+  if (fault == kFaultFlags) w.flag_mail &= ~(1u << mailbox);
+  w.absent = fault == kFaultAbsent;
+  w.refused = fault == kFaultRefused;
+  *out = w;
   return true;
 }
 constexpr int kResMaxTilesPerCta = 4;

@@ -27,12 +27,13 @@
 // Results equal the tick-per-launch path's bit for bit.
 //
 // The CTAs wait on one another, so the launch is cooperative (all resident or none start), and every
-// wait gives up after kResWaitNs of polling. A CTA that gives up raises the abort mark and stores nothing; the
-// others tell the keeper when their last wait is over, and the keeper, which alone writes the state,
-// waits for all of them: whichever CTA gave up, the run ends with BPF_ERR_STATE, and a later run
+// wait gives up after kResWaitNs of polling. A CTA that gives up raises the abort mark, stores none of its
+// tiles and sets the state's error itself (the keeper, which writes the rest of the state, leaves that
+// word to it): whichever CTA gave up, and however late, the run ends with BPF_ERR_STATE, and a later run
 // does not start on such a state.
 #include "bpf_tick.cuh"
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 #include <type_traits>
 
@@ -52,7 +53,7 @@ static_assert(kResMaxTilesPerCta == 4, "four tiles of two groups of threads");
 // CTA b polls mailbox b % kMail: with one mailbox polled by all, the polls of a few hot lines held
 // up the records themselves.
 // ---------------------------------------------------------------------------
-constexpr int kMail = 16;
+constexpr int kMail = kResMail;
 constexpr size_t kXHeader = 256;
 __host__ __device__ inline size_t mail_flag_bytes(int G) { return ((size_t)G * 4 + 127) & ~(size_t)127; }
 __host__ __device__ inline size_t mail_bytes(int G) { return mail_flag_bytes(G) + (((size_t)G * 64 + 127) & ~(size_t)127); }
@@ -80,9 +81,9 @@ __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
 struct Patience {
   WaitBudget budget;
   unsigned spins = 0u;
-  __device__ __forceinline__ bool more(const unsigned* abort_word, unsigned mark, unsigned long long limit_ns) {
+  __device__ __forceinline__ bool more(const unsigned* abort_word, unsigned mark, unsigned limit) {
     if ((++spins & 255u) != 0u) return true;
-    const bool over = budget.over(global_timer_ns(), limit_ns);
+    const bool over = budget.over(WaitBudget::clock(global_timer_ns()), limit);
     return __all_sync(0xffffffffu, !over && ld_relaxed_u32(abort_word) != mark);
   }
 };
@@ -176,6 +177,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
   if (tid < (int)(sizeof(DevState) / 8))
     reinterpret_cast<unsigned long long*>(&sh.st)[tid] = __ldcg(reinterpret_cast<const unsigned long long*>(p.st) + tid);
   __syncthreads();
+  if (sh.st.error == BPF_ERR_STATE) n_ticks = 0;         // an earlier run gave up: nothing to go on from
   if (tid == 0) sh.ustate = sh.st.u_state;
   int nk[Q];                                    // the tiles' exponents (previous tick's until pass 1 sets them)
 #pragma unroll
@@ -229,9 +231,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
   double dS = 0.0, dQ = 0.0, dH = 0.0;
   int d_nM = 0;
   unsigned xn = 0u;                             // exchanges so far
-  // a wait gave up (the same in every thread of the CTA), or the state is that of a run that did
-  const bool refused = sh.st.error == BPF_ERR_STATE;
-  bool failed = refused;
+  bool failed = false;                          // a wait gave up (the same in every thread of the CTA)
   bool pending = false;                         // the keeper's state is one decision behind
   int pending_rec = 0;
   auto settle = [&](int apf_stage, int t) {
@@ -252,7 +252,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
   const bool ahead = a.ess_threshold <= 0.0f;   // every tick that can resample does
   int stage = 0, prev_stage = 0;                // APF: 0 the first tick of all, else stages 1 and 2 of a tick
   int t = 0;
-  while (!failed && t < n_ticks) {
+  while (t < n_ticks) {
     if ((!APF || stage != 2) && (t & (kResThreads - 1)) == 0) {
       __syncthreads();
       if (t + tid < n_ticks) sh.ys[tid] = __ldg(a.y_ptr + t + tid);
@@ -395,8 +395,7 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
           }
           tS = warp_sum_d(tS); tQ = warp_sum_d(tQ); tH = warp_sum_d(tH);
           tE = warp_sum_u64(tE);
-          const bool withheld = waits.fault == kFaultWithhold && waits.cta == (int)blockIdx.x && waits.xn == xn;
-          if (lane < kMail && !withheld) {             // (every lane holds the same sums)
+          if ((waits.record_mail >> lane) & 1u) {      // lanes 0 .. kMail - 1 (every lane holds the same sums)
             unsigned char* slot = p.xbuf + kXHeader + lane * mail_size + mail_flag_bytes(G) +
                                   ((size_t)(xn & 1u) * G + first + j) * 32;
             st_relaxed_b128(slot, (unsigned long long)__float_as_uint((float)tS) | ((unsigned long long)__float_as_uint((float)tQ) << 32),
@@ -443,11 +442,15 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
       const unsigned char* slot = slot_of(u);
       if (u > 0) { ld_relaxed_b128(slot, a0, a1); ld_relaxed_b128(slot + 16, b0, b1); }
       Patience pt;
-      for (bool last = false;;) {
+      for (;;) {
         const bool ok = (unsigned)(a1 >> 32) == xno && (unsigned)(b1 >> 32) == xno;
         if (__all_sync(0xffffffffu, ok)) break;
-        if (last) { bad = true; break; }             // the same in every lane
-        last = !pt.more(xw + 1, epoch + 1u, waits.limit_ns);
+        if (!pt.more(xw + 1, epoch + 1u, waits.limit)) {             // the same in every lane
+          ld_relaxed_b128(slot, a0, a1);
+          ld_relaxed_b128(slot + 16, b0, b1);
+          if (!__all_sync(0xffffffffu, (unsigned)(a1 >> 32) == xno && (unsigned)(b1 >> 32) == xno)) bad = true;
+          break;
+        }
         ld_relaxed_b128(slot, a0, a1);
         ld_relaxed_b128(slot + 16, b0, b1);
       }
@@ -469,7 +472,6 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
       S = warp_sum_d(S); Qs = warp_sum_d(Qs); H = warp_sum_d(H);
       if (lane == 0) { sh.wn[pw] = nW; sh.wS[pw] = S; sh.wQ[pw] = Qs; sh.wH[pw] = H; }
     }
-    if (waits.fault == kFaultExchange && waits.cta == (int)blockIdx.x && waits.xn == xn) bad = true;
     if (__syncthreads_or(bad)) { failed = true; break; }
 
     // ---- decision (the last warp), and beside it, when every tick resamples, the masses ----
@@ -716,7 +718,8 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
         }
         // every CTA whose children fall into this CTA's slots has written them before they are read
         __syncthreads();
-        if (tid < kMail) st_release_u32(reinterpret_cast<unsigned*>(p.xbuf + kXHeader + tid * mail_size) + blockIdx.x, xno);
+        if (tid < 32 && ((waits.flag_mail >> tid) & 1u))
+          st_release_u32(reinterpret_cast<unsigned*>(p.xbuf + kXHeader + tid * mail_size) + blockIdx.x, xno);
         const int slot_lo = first * kTile, slot_hi = (first + nth) * kTile;
         // which CTAs write children into this CTA's slots: bit u, tile 32 (warp + u kResWarps) + lane
         unsigned need = 0u;
@@ -737,15 +740,16 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
           if (!__any_sync(0xffffffffu, wait)) continue;
           const unsigned* flag = reinterpret_cast<const unsigned*>(mail) + (wait ? (32 * (warp + u * kResWarps) + lane) / nt : (int)blockIdx.x);
           Patience pt;
-          for (bool last = false;;) {             // left by a warp vote, as above
+          for (;;) {                              // left by a warp vote, as above
             const bool ok = !wait || (int)(ld_relaxed_u32(flag) - xno) >= 0;
             if (__all_sync(0xffffffffu, ok)) break;
-            if (last) { bad = true; break; }
-            last = !pt.more(xw + 1, epoch + 1u, waits.limit_ns);
+            if (!pt.more(xw + 1, epoch + 1u, waits.limit)) {
+              if (!__all_sync(0xffffffffu, !wait || (int)(ld_relaxed_u32(flag) - xno) >= 0)) bad = true;
+              break;
+            }
           }
           asm volatile("fence.acq_rel.gpu;" ::: "memory");   // acquire (a relaxed poll leaves L1 alone)
         }
-        if (waits.fault == kFaultFlags && waits.cta == (int)blockIdx.x && waits.xn == xn) bad = true;
         if (__syncthreads_or(bad)) { failed = true; break; }
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -784,13 +788,9 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
 
   if (tid == kDecider && pending && keeper && !failed) settle(prev_stage, pending_rec);
   __syncthreads();
-  // This CTA's end of the run: the abort mark, on which the other CTAs stop waiting, or, in the mailbox
-  // that the keeper polls, a number past every exchange of this run.
-  const unsigned xend = epoch + xn + 1u;
-  unsigned char* keeper_mail = p.xbuf + kXHeader + ((gridDim.x - 1u) % kMail) * mail_size;
-  if (tid == 0 && !refused) {
-    if (failed) st_release_u32(xw + 1, epoch + 1u);
-    else if (!keeper) st_release_u32(reinterpret_cast<unsigned*>(keeper_mail) + blockIdx.x, xend);
+  if (failed && tid == 0) {
+    st_release_u32(xw + 1, epoch + 1u);         // the other CTAs stop waiting
+    atomicExch(&p.st->error, BPF_ERR_STATE);
   }
   if (!failed) {
 #pragma unroll
@@ -809,30 +809,17 @@ resident_kernel(Plan p, TickArgs a, ResidentTape tape, ResidentWaits waits, int 
     }
   }
   if (keeper) {
-    if (!failed) {                              // every other CTA's end (one CTA a thread)
-      const bool wait = tid + 1 < (int)gridDim.x;
-      bool bad = false;
-      if (__any_sync(0xffffffffu, wait)) {
-        const unsigned* flag = reinterpret_cast<const unsigned*>(keeper_mail) + (wait ? tid : (int)blockIdx.x);
-        Patience pt;
-        for (bool last = false;;) {             // left by a warp vote, as above
-          const bool ok = !wait || (int)(ld_relaxed_u32(flag) - xend) >= 0;
-          if (__all_sync(0xffffffffu, ok)) break;
-          if (last) { bad = true; break; }
-          last = !pt.more(xw + 1, epoch + 1u, waits.limit_ns);
-        }
-      }
-      if (__syncthreads_or(bad)) failed = true;
-    }
     if (tid == 0) {
-      if (failed) sh.st.error = BPF_ERR_STATE;
       *reinterpret_cast<volatile unsigned*>(xw) = epoch + 4u * (unsigned)n_ticks + 4u;   // past every number used
+      if (sh.st.error == BPF_ERR_DEGENERATE) atomicCAS(&p.st->error, BPF_OK, BPF_ERR_DEGENERATE);
     }
-    __syncthreads();
-    if (tid < (int)(sizeof(DevState) / 8))
+    // every word but the one that holds the error
+    if (tid < (int)(sizeof(DevState) / 8) && tid != (int)(offsetof(DevState, error) / 8))
       reinterpret_cast<unsigned long long*>(p.st)[tid] = reinterpret_cast<const unsigned long long*>(&sh.st)[tid];
   }
 }
+static_assert(offsetof(DevState, error) % 8 == 0 && offsetof(DevState, seed) == offsetof(DevState, error) + 4,
+              "the error shares its word with the seed, which no run changes");
 
 // ---------------------------------------------------------------------------
 // Launcher
@@ -871,7 +858,7 @@ int resident_max_tiles(int device) {
     int sms = 0, coop = 0;
     const bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
                     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop != 0 &&
-                    sms > 0 && sms < kResThreads && sms * kResMaxTilesPerCta <= kResMaxTiles;
+                    sms > 0 && sms * kResMaxTilesPerCta <= kResMaxTiles;
     if (!ok) cudaGetLastError();
     g_sms[device] = ok ? sms : -1;
   }
@@ -901,13 +888,14 @@ bool resident_ready(int device, int G, int max_tiles, bool tstate, bool gauss, b
 cudaError_t launch_resident(const Plan& p, const TickArgs& a, const ResidentTape& tape, bool apf, int n_ticks,
                             int max_tiles, cudaStream_t s, const ResidentWaits& waits) {
   if (!p.xbuf || p.G < 1 || p.G > max_tiles || p.G > kResMaxTiles || n_ticks < 1 || !a.y_ptr) return cudaErrorInvalidValue;
-  if (waits.fault == kFaultRefused) return cudaErrorCooperativeLaunchTooLarge;
+  if (waits.refused) return cudaErrorCooperativeLaunchTooLarge;
   const int sms = max_tiles / kResMaxTilesPerCta;
   const int nt = (p.G + sms - 1) / sms;
   size_t smem = 0;
   ResidentKernel k = pick(nt, a.nu_int > 0, !(a.obs.nu > 0.0f), apf, &smem);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((p.G + nt - 1) / nt);
+  const int ctas = (p.G + nt - 1) / nt;
+  cfg.gridDim = dim3(std::max(1, ctas - (waits.absent ? 1 : 0)));
   cfg.blockDim = dim3(kResThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;

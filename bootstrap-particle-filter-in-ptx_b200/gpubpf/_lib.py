@@ -145,9 +145,9 @@ SIGNATURES = {
     "gpu_bpf_debug_live_bytes": (C.c_size_t, []),
     "gpu_bpf_kept_bytes": (C.c_size_t, []),
     "gpu_bpf_trim_kept": (C.c_size_t, []),
-    "gpu_bpf_debug_resident": (_i, [P_STATE, _i, _i, _i, _d]),
-    "gpu_apf_debug_resident": (_i, [P_APF, _i, _i, _i, _d]),
-    "gpu_bpf_grad_debug_resident": (_i, [_vp, _i, _i, _i, _d]),
+    "gpu_bpf_debug_resident": (_i, [P_STATE, _i, _i, _d]),
+    "gpu_apf_debug_resident": (_i, [P_APF, _i, _i, _d]),
+    "gpu_bpf_grad_debug_resident": (_i, [_vp, _i, _i, _d]),
     "gpu_bpf_debug_wait_budget": (_i, [C.POINTER(C.c_ulonglong), _i, C.c_ulonglong]),
     "gpu_bpf_get_learning_sums": (_i, [P_STATE, C.POINTER(_d), C.POINTER(_i)]),
     "gpu_bpf_run_static": (_i, [_i, _f, _f, _f, _f, _i, _f, _vp, _i, _vp, _vp]),

@@ -586,19 +586,20 @@ size_t    gpu_bpf_debug_live_bytes(void);
 /* Waits of resident runs (gpu_bpf_set_fused_small; testing aid). The CTAs of such a run wait on one
  * another, each wait at most 2 s of polling; a run in which one gives up ends with BPF_ERR_STATE: step_many returns
  * it, after step_many_device the next read-back does, and later runs do not start until gpu_bpf_reset or
- * gpu_bpf_load. This call sets the limit of this filter's waits (0 < limit_ms <= 2000) and one failure
- * made on purpose: fault 0 none; 1 CTA cta gives up in the run's exchange number `exchange` (1-based;
- * one per tick, two per auxiliary-filter tick after the first); 2 it gives up waiting for the children
- * of that exchange's resampling; 3 it does not publish its record of that exchange, so every wait for
- * it runs out; 4 the launch is refused, as where the whole grid does not fit on what the process may use
- * of the device: the ticks then run one by one, and the object makes no other attempt until the next
- * call of this function. No GPU fault is involved: the kernel returns. */
-int gpu_bpf_debug_resident(GpuBpfState* state, int fault, int cta, int exchange, double limit_ms);
-int gpu_apf_debug_resident(GpuApfState* state, int fault, int cta, int exchange, double limit_ms);
-int gpu_bpf_grad_debug_resident(GpuBpfGrad* grad, int fault, int cta, int exchange, double limit_ms);
-/* The look (index into now_ns, the clock at each look, nonzero) at which such a wait of limit_ns gives up,
- * n if it does not: the time between two looks counts as at most a sixteenth of the limit, so a GPU
- * that was taken away for a while does not end the run. On the host. */
+ * gpu_bpf_load. This call sets the limit of this filter's waits (0.1 <= limit_ms <= 2000) and one failure
+ * made on purpose: fault 0 none; 1 no CTA's record reaches mailbox `mailbox` (0..15), so every 16th CTA,
+ * from that one on, gives up in the run's first exchange; 2 nor does a CTA's word that its children are
+ * written, so those CTAs give up in the first resampling that needs one; 3 the last CTA does not run;
+ * 4 the launch is refused, as where the whole grid does not fit on what the process may use of the
+ * device: the ticks then run one by one, and the object makes no other attempt until the next call of
+ * this function. No GPU fault is involved: the kernel returns. */
+int gpu_bpf_debug_resident(GpuBpfState* state, int fault, int mailbox, double limit_ms);
+int gpu_apf_debug_resident(GpuApfState* state, int fault, int mailbox, double limit_ms);
+int gpu_bpf_grad_debug_resident(GpuBpfGrad* grad, int fault, int mailbox, double limit_ms);
+/* The look (index into now_ns, the clock at each look, less than an hour apart) at which such a wait of
+ * limit_ns (1024 to 2e9, counted in units of 1024 ns) gives up, n if it does not: the time between two
+ * looks counts as at most a sixteenth of the limit, so a GPU that was taken away for a while does not
+ * end the run. On the host. */
 int gpu_bpf_debug_wait_budget(const unsigned long long* now_ns, int n, unsigned long long limit_ns);
 
 /* Kept memory: device memory that gradient runs (gpu_bpf_grad_forward, gpu_bpf_batch_grad_run) take only

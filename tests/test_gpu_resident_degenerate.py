@@ -34,7 +34,7 @@ def test_auxiliary_run(bpf, N, nu_obs, value, at):
     out = []
     for fault in (0, REFUSED):
         f = bpf.GpuApf(N, RHO, SIG, MU, 0.0, nu_obs, 19)
-        assert lib.gpu_apf_debug_resident(f._s, fault, 0, 0, 2000.0) == _lib.BPF_OK
+        assert lib.gpu_apf_debug_resident(f._s, fault, 0, 2000.0) == _lib.BPF_OK
         rec = (_lib.BpfTickRecord * 40)()
         rc = lib.gpu_apf_step_many(f._s, ya, 40, None, rec)
         out.append((rc, bytes(rec), bytes(f.get_particles()), np.float64(f.get_loglik_total()).tobytes()))
@@ -55,7 +55,7 @@ def test_tape(bpf, N, value):
     out = []
     for fault in (0, REFUSED):
         tape = bpf.GradTape(N, T)
-        assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, 0, 0, 2000.0) == 0
+        assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, 0, 2000.0) == 0
         ll = tape.forward((MU, RHO, SIG), y, seed=8).cpu().numpy().tobytes()
         recs = tape.records()
         out.append((ll, [bytes(r) for r in recs], [tape.children(t).tobytes() for t in range(T - 1) if t != at]))

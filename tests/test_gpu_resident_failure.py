@@ -1,7 +1,7 @@
-"""Resident runs whose CTAs give up waiting: made on purpose by gpu_bpf_debug_resident (a CTA told to
-give up, or a record never published with a limit of 20 ms on the waits), so the kernel returns its
-status and no GPU fault is involved. The run must end with BPF_ERR_STATE whichever CTA gave up and
-however late, and a reset filter must then run as a new one, bit for bit."""
+"""Resident runs whose CTAs give up waiting: made on purpose by gpu_bpf_debug_resident (a mailbox that gets no
+records or no flags, an absent CTA, a limit of 20 ms on the waits), so the kernel returns its status and
+no GPU fault is involved. The run must end with BPF_ERR_STATE whichever CTA gave up and however late, and
+a reset filter must then run as a new one, bit for bit."""
 from __future__ import annotations
 
 import math
@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 RHO, SIG, MU = 0.97, 0.15, -1.0
 TILE = 4096
-EXCHANGE, FLAGS, WITHHOLD = 1, 2, 3
+RECORDS, FLAGS, ABSENT, REFUSED = 1, 2, 3, 4
+T = 12
 
 
 def _series(T, seed):
@@ -21,58 +22,90 @@ def _series(T, seed):
     return np.asarray(dgp.matched_series(T, RHO, SIG, MU, seed)[1], dtype=np.float32)
 
 
-def _arm(f, fn, fault=0, cta=0, exchange=0, limit_ms=2000.0):
+def _arm(f, fn, fault=0, mailbox=0, limit_ms=2000.0):
     from gpubpf import _lib
-    assert getattr(f._lib, fn)(f._s, fault, cta, exchange, limit_ms) == _lib.BPF_OK
+    assert getattr(f._lib, fn)(f._s, fault, mailbox, limit_ms) == _lib.BPF_OK
 
 
-T = 12
-# (particles, fault, CTA, exchange): the first CTA or the keeper (the last one), the last exchange, the
-# children of the last tick, and a record that is never published, with one to four tiles a CTA
-CASES = [(70000, EXCHANGE, 0, T), (70000, EXCHANGE, 17, T), (70000, FLAGS, 0, T), (70000, FLAGS, 3, 5),
-         (70000, WITHHOLD, 2, 7), (70000, WITHHOLD, 0, T), (1000003, EXCHANGE, 1, T), (1000003, FLAGS, 1, T),
-         (592 * TILE, EXCHANGE, 0, T), (592 * TILE, FLAGS, 146, T), (592 * TILE, WITHHOLD, 147, 1)]
+# The last CTA writes the state and polls mailbox (CTAs - 1) % 16: 18 CTAs of one tile, 123 of two, 148 of four.
+# With one tick and no resampling its waits are all answered while CTAs of the mailbox give up.
+CASES = [(70000, 1e-6, 1, RECORDS, 0), (70000, 1e-6, 1, RECORDS, 1), (70000, 0.0, T, FLAGS, 5),
+         (70000, 0.0, T, RECORDS, 3), (70000, 0.0, T, ABSENT, 0), (1000003, 1e-6, 1, RECORDS, 7),
+         (592 * TILE, 1e-6, 1, RECORDS, 15), (592 * TILE, 0.5, T, ABSENT, 0)]
 
 
-@pytest.mark.parametrize("N,fault,cta,exchange", CASES)
-def test_run_with_a_wait_given_up_reports_it(bpf, N, fault, cta, exchange):
+@pytest.mark.parametrize("N,thr,ticks,fault,mailbox", CASES)
+def test_run_with_a_wait_given_up_reports_it(bpf, N, thr, ticks, fault, mailbox):
     import torch
     from gpubpf import _lib
     y = _series(T, 9)
-    f = bpf.GpuBpf(N, RHO, SIG, MU, seed=3, ess_threshold=0.0)
+    f = bpf.GpuBpf(N, RHO, SIG, MU, seed=3, ess_threshold=thr)
     want = [bytes(r) for r in f.step_many(y.tolist(), records=True)], bytes(f.get_particles())
     yd = torch.tensor(y, device="cuda")
     rec = torch.zeros(T * 40, dtype=torch.uint8, device="cuda")
 
     f.reset(3)
-    _arm(f, "gpu_bpf_debug_resident", fault, cta, exchange, 20.0)
-    with pytest.raises(bpf.BpfError) as e:
-        f.step_many(y.tolist())
-    assert e.value.code == _lib.BPF_ERR_STATE
-    f.reset(3)
-    f.step_many_device(yd.data_ptr(), T, rec.data_ptr())          # reported by the read-backs
+    _arm(f, "gpu_bpf_debug_resident", fault, mailbox, 20.0)
+    f.step_many_device(yd.data_ptr(), ticks, rec.data_ptr())          # reported by the read-backs
     for read in (f.get_record, f.get_particles, f.save, f.get_result):
         with pytest.raises(bpf.BpfError) as e:
             read()
         assert e.value.code == _lib.BPF_ERR_STATE
     assert math.isnan(f.get_loglik_total())
-
-    _arm(f, "gpu_bpf_debug_resident")                             # a later run does not start on that state
+    _arm(f, "gpu_bpf_debug_resident")                                 # a later run does not start on that state
     with pytest.raises(bpf.BpfError) as e:
         f.step_many(y.tolist())
     assert e.value.code == _lib.BPF_ERR_STATE
     f.reset(3)
     assert ([bytes(r) for r in f.step_many(y.tolist(), records=True)], bytes(f.get_particles())) == want
+    if ticks > 1:                                                     # and by a host run itself
+        _arm(f, "gpu_bpf_debug_resident", fault, mailbox, 20.0)
+        f.reset(3)
+        with pytest.raises(bpf.BpfError) as e:
+            f.step_many(y.tolist())
+        assert e.value.code == _lib.BPF_ERR_STATE
+    f.close()
+
+
+@pytest.mark.parametrize("N,tiles", [(70000, 1), (1000003, 2), (592 * TILE, 4)])
+def test_last_resampling_with_a_wait_given_up_reports_it(bpf, N, tiles):
+    """One tick that resamples, its flags kept from one mailbox after another: the CTAs that poll it give up
+    if and only if children of another CTA's particles fall into their slots, which the ancestors of the
+    same tick say. The last CTA's own mailbox is left alone, so that its waits are answered."""
+    import torch
+    from gpubpf import _lib
+    y = torch.tensor(_series(T, 9), device="cuda")
+    rec = torch.zeros(40, dtype=torch.uint8, device="cuda")
+    f = bpf.GpuBpf(N, RHO, SIG, MU, seed=3, ess_threshold=0.0)
+    f.record_ancestors(True)
+    f.step_many_device(y.data_ptr(), 1, rec.data_ptr())
+    owner = np.arange(N) // (tiles * TILE)
+    waits = np.unique(owner[np.frombuffer(f.get_ancestors()[1], dtype=np.int32) // (tiles * TILE) != owner])
+    assert len(waits) > 0
+    seen = set()
+    for mailbox in sorted(set(range(16)) - {int(owner[-1]) % 16}):
+        _arm(f, "gpu_bpf_debug_resident", FLAGS, mailbox, 20.0)
+        f.reset(3)
+        f.step_many_device(y.data_ptr(), 1, rec.data_ptr())
+        gives_up = bool(np.any(waits % 16 == mailbox))
+        seen.add(gives_up)
+        if gives_up:
+            with pytest.raises(bpf.BpfError) as e:
+                f.get_particles()
+            assert e.value.code == _lib.BPF_ERR_STATE
+        else:
+            f.get_particles()
+    assert True in seen
     f.close()
 
 
 @pytest.mark.parametrize("N", [50000, 1500000])
-@pytest.mark.parametrize("fault,cta,exchange", [(EXCHANGE, 0, 2 * T - 1), (FLAGS, 1, 2 * T - 1), (WITHHOLD, 1, 8)])
-def test_auxiliary_run_with_a_wait_given_up_reports_it(bpf, N, fault, cta, exchange):
+@pytest.mark.parametrize("fault,mailbox", [(RECORDS, 0), (FLAGS, 1), (ABSENT, 0)])
+def test_auxiliary_run_with_a_wait_given_up_reports_it(bpf, N, fault, mailbox):
     from gpubpf import _lib
     y = _series(T, 9).tolist()
     f = bpf.GpuApf(N, RHO, SIG, MU, seed=3)
-    _arm(f, "gpu_apf_debug_resident", fault, cta, exchange, 20.0)
+    _arm(f, "gpu_apf_debug_resident", fault, mailbox, 20.0)
     with pytest.raises(bpf.BpfError) as e:
         f.step_many(y)
     assert e.value.code == _lib.BPF_ERR_STATE
@@ -82,43 +115,39 @@ def test_auxiliary_run_with_a_wait_given_up_reports_it(bpf, N, fault, cta, excha
 def test_rejects_bad_arguments(bpf):
     from gpubpf import _lib
     f = bpf.GpuBpf(70000, RHO, SIG, MU, seed=3)
-    for args in ((5, 0, 1, 10.0), (-1, 0, 1, 10.0), (1, -1, 1, 10.0), (1, 0, -1, 10.0), (1, 0, 1, 0.0), (1, 0, 1, 2001.0),
-                 (1, 0, 1, math.nan)):
+    for args in ((5, 0, 10.0), (-1, 0, 10.0), (1, -1, 10.0), (1, 16, 10.0), (1, 0, 0.0), (1, 0, 2001.0), (1, 0, math.nan)):
         assert f._lib.gpu_bpf_debug_resident(f._s, *args) == _lib.BPF_ERR_ARG
     f.close()
 
 
 @pytest.mark.parametrize("every", [0, 4])
-@pytest.mark.parametrize("N,fault,cta,exchange", [(70001, EXCHANGE, 0, T), (70001, FLAGS, 1, 6), (700001, FLAGS, 0, T),
-                                                  (70001, WITHHOLD, 3, 1)])
-def test_tape_with_a_wait_given_up_has_no_gradient(bpf, N, fault, cta, exchange, every):
+@pytest.mark.parametrize("N,ticks,fault,mailbox", [(70001, T, RECORDS, 0), (70001, T, FLAGS, 0), (700001, T, FLAGS, 2),
+                                                   (70001, T, ABSENT, 0)])
+def test_tape_with_a_wait_given_up_has_no_gradient(bpf, N, ticks, fault, mailbox, every):
     """With and without the particles of every tick kept: NaN from forward and backward, an error from the
     calls that read the tape, and a sound tape from the next forward run."""
     import torch
     from gpubpf import _lib
-    y = torch.tensor(_series(T, 9), device="cuda")
+    y = torch.tensor(_series(ticks, 9), device="cuda")
     theta = (MU, RHO, SIG)
 
     def clean(tape):
-        return tape.forward(theta, y, seed=8).item(), tape.backward().cpu().numpy().tobytes(), bytes(tape.children(T - 2))
+        return tape.forward(theta, y, seed=8).item(), tape.backward().cpu().numpy().tobytes(), bytes(tape.children(0))
 
     other = bpf.GradTape(N, T, checkpoint_every=every)
     want = clean(other)
     other.close()
     tape = bpf.GradTape(N, T, checkpoint_every=every)
-    assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, cta, exchange, 20.0) == _lib.BPF_OK
+    assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, mailbox, 20.0) == _lib.BPF_OK
     assert math.isnan(tape.forward(theta, y, seed=8).item())      # a tape that no run has filled before
     assert np.isnan(tape.backward().cpu().numpy()).all()
     for read in (tape.records, lambda: tape.children(0), lambda: tape.replay(theta)):
         with pytest.raises(bpf.BpfError) as e:
             read()
         assert e.value.code == _lib.BPF_ERR_STATE
-    assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, 0, 0, 0, 2000.0) == _lib.BPF_OK
+    assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, 0, 0, 2000.0) == _lib.BPF_OK
     assert clean(tape) == want
     tape.close()
-
-
-REFUSED = 4
 
 
 @pytest.mark.parametrize("N,ticks", [(70000, 70), (1000003, 12)])
@@ -198,7 +227,7 @@ def test_refused_tape_is_taped_by_the_kernels(bpf, N, nu_state, nu_obs, every):
         tape = bpf.GradTape(N, 37, checkpoint_every=every)
         got = []
         for fault, seed in zip(faults, (3, 9)):
-            assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, 0, 0, 2000.0) == 0
+            assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, 0, 2000.0) == 0
             got.append(read(tape, seed))
         tape.close()
         out.append(got)

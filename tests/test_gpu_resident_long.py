@@ -43,7 +43,7 @@ def test_tape_of_several_launches(bpf, every):
     out = []
     for fault in (0, 4):                     # 4: the resident launch is refused
         tape = bpf.GradTape(N, T, checkpoint_every=every)
-        assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, 0, 0, 2000.0) == 0
+        assert tape._lib.gpu_bpf_grad_debug_resident(tape._h, fault, 0, 2000.0) == 0
         n0 = tape._lib.gpu_bpf_launch_count()
         ll = tape.forward((MU, RHO, SIG), y, seed=4).item()
         n = tape._lib.gpu_bpf_launch_count() - n0
@@ -66,7 +66,7 @@ def test_long_device_run_stays_on_the_chip(bpf, N, launches):
         rec = torch.zeros(T * 40, dtype=torch.uint8, device="cuda")
         f = bpf.GpuBpf(N, RHO, SIG, MU, seed=3, ess_threshold=0.5)
         f.set_fused_small(fused)
-        assert f._lib.gpu_bpf_debug_resident(f._s, fault, 0, 0, 2000.0) == 0
+        assert f._lib.gpu_bpf_debug_resident(f._s, fault, 0, 2000.0) == 0
         n0 = f._lib.gpu_bpf_launch_count()
         f.step_many_device(y.data_ptr(), T, rec.data_ptr())
         n = f._lib.gpu_bpf_launch_count() - n0
