@@ -503,9 +503,9 @@ __global__ void __launch_bounds__(NT, (1024 / NT > 0 ? 1024 / NT : 1)) batch_ker
 // The same filter with at most EPT (4, 8 or 16) particles a thread, unrolled: the shapes that the
 // classes run with by default. Bit for bit the generic form's values: pass 1 keeps its strided
 // element order and reduction trees.
-// What bounded the generic form was issue: about 120 thread-instructions per particle and tick (64-bit
+// What bounded the generic form was issue: 322 thread-instructions per particle and resampling tick (64-bit
 // stream multiplies, swizzle arithmetic and bounds per element, the exact masses on every tick,
-// butterflies per sum) and 100 more where it resamples (64-bit compares per child). Here the PCG32
+// butterflies per sum, 64-bit compares per child; this form: 227). Here the PCG32
 // state is stepped, the log2-weights stay in registers between the two passes, the sums of all tiles
 // are reduced together, the exact masses are formed only on resampling ticks (from the chunk scan),
 // and the children come from pass 2's FP32 estimate with exact recounts, start marks and a vote scan.

@@ -19,8 +19,9 @@
 //             shared memory where they fall there (nearly all do: a tile's outputs drift from its
 //             slots by about sqrt(N)), else to the other particle buffer (L2), from which the owner
 //             takes them once the CTAs that write there have raised their flags.
-// What bounds it: latency, three grid-wide dependencies deep at most, and the issue of about 60
-// thread-instructions per particle (16 particles a thread keep the per-thread overhead small: with
+// What bounds it: latency, three grid-wide dependencies deep at most, and the issue of 79 thread-instructions
+// per particle and tick with two tiles a CTA (99 with one), 186 (223) where the tick resamples, by 16
+// warps an SM on 40 to 50% of the cycles (16 particles a thread keep the per-thread overhead small: with
 // 1024 threads of 4 the same tick issued 144 per particle). Measured per tick: N = 300000 at
 // ESS < 0.5 N 4.0 us (16.4 with a launch per kernel), always resampling 9.1 us (20.8); N = 1000003 at
 // ESS < 0.5 N 5.7 us (12.5), always resampling 12.5; N = 2.4 M at ESS < 0.5 N 10.7.

@@ -243,9 +243,9 @@ int    gpu_bpf_load(GpuBpfState* state, const void* buf, size_t len);
  * 32768 particles take it where the device schedules a cluster of 16 CTAs. Runs of
  * ticks of larger filters, up to four 4096-particle tiles per SM (2.4 million
  * particles on 148 SMs), stay on the chip as cooperative launches of up to 1024
- * ticks, bit-identical too. Such a launch takes one CTA and most of the shared
- * memory of up to every SM (one SM per tile up to as many tiles as SMs): it starts
- * when those SMs are free, and other streams' kernels that need them wait until it
+ * ticks, bit-identical too. Such a launch takes the registers of as many SMs as it
+ * has CTAs (one per tile up to as many tiles as SMs, then all): it starts when
+ * those SMs are free, and other streams' kernels that need them wait until it
  * ends (4 to 25 ms for 1024 ticks). On by default; enable = 0 selects the
  * three-kernel tick for both, which leaves the GPU between ticks. Learning filters,
  * Silverman jitter and profiled ticks always take the three-kernel path. */
