@@ -232,3 +232,25 @@ def test_refused_tape_is_taped_by_the_kernels(bpf, N, nu_state, nu_obs, every):
         tape.close()
         out.append(got)
     assert out[0] == out[1] == out[2] == out[3]
+
+
+@pytest.mark.parametrize("N", [5000, 300000])
+def test_recording_auxiliary_run_replays_its_graph(bpf, N):
+    """A filter that records its ancestors keeps the kernels: a single tick, the 64-tick graph, the graph again
+    and a remainder. Records and particles equal the resident run's, the last tick's ancestors those
+    of the same run ended by a single tick."""
+    y = _series(131, 5).tolist()
+    f = bpf.GpuApf(N, RHO, SIG, MU, seed=3)
+    want = [bytes(r) for r in f.step_many(y, records=True)], bytes(f.get_particles()), f.get_loglik_total()
+    f.close()
+    anc = []
+    for last in (66, 1):
+        f = bpf.GpuApf(N, RHO, SIG, MU, seed=3)
+        f.record_ancestors(True)
+        recs = f.step_many(y[:1], records=True) + f.step_many(y[1:65], records=True)
+        recs += f.step_many(y[65:131 - last], records=True) if last == 1 else []
+        recs += f.step_many(y[131 - last:], records=True)
+        assert ([bytes(r) for r in recs], bytes(f.get_particles()), f.get_loglik_total()) == want
+        anc.append([bytes(a) for a in f.get_ancestors()])
+        f.close()
+    assert anc[0] == anc[1]
